@@ -22,9 +22,10 @@
 // followed by the next Sᵀ into the same columns needs no barrier), 2..3 idle, 4..11 conversion (two groups of four: group
 // c owns query columns 64c..64c+63), 12..15 dQ read-out.  Registers are rebalanced with setmaxnreg.
 // Issue order in the steady state, after dSᵀ of tile i is in shared memory:
-//     dQ_i, dK += …_i, dV += …_{i+1}, [dQ_i read out] dPᵀ_{i+1}, Sᵀ_{i+2}
-// so that the read-out of dQ_i runs under dK/dV, the conversion of Pᵀ_{i+1} under dQ_i/dK and that of dSᵀ_{i+1} under
-// Sᵀ_{i+2}.
+//     dQ_i, dK += …_i, [dQ_i read out] dPᵀ_{i+1}, [Pᵀ_{i+1} ready] dV += …_{i+1}, Sᵀ_{i+2}
+// so that the read-out of dQ_i runs under dK, the conversion of Pᵀ_{i+1} under dQ_i / dK / dPᵀ_{i+1} and that of dSᵀ_{i+1}
+// under dV / Sᵀ_{i+2}.  (With dV before dPᵀ the chain  dSᵀ_i -> Pᵀ_{i+1} converted -> dV -> dPᵀ_{i+1} -> dSᵀ_{i+1}  was serial:
+// B8 T4096 H16 G4 D128 2.05 -> 1.87 ms, B1 T32768 H8 7.60 -> 6.82 ms, B1 T8192 H20 G10 D64 1.00 -> 0.80 ms.)
 // Masking rule as in the forward: query r sees keys lo(r) ≤ k ≤ r.
 #include "sm100.cuh"
 #include "api.h"
@@ -232,12 +233,12 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         B1_TRACE(1, it);
         if (it + 1 < n_iter) {
           if (!mbar_wait(do_full, (it + 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_FULL)) goto done;
-          if (!issue_dv(it + 1)) goto done;
-          B1_TRACE(2, it);
           // dPᵀ of the next tile goes into the columns of dQ_i: wait for the read-out
           if (!mbar_wait(dq_empty, ph, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY)) goto done;
-          B1_TRACE(3, it);
+          B1_TRACE(2, it);
           issue_dp(it + 1);
+          B1_TRACE(3, it);
+          if (!issue_dv(it + 1)) goto done;
           umma_commit(do_empty);
           if (it + 2 < n_iter && !issue_s(it + 2)) goto done;
           B1_TRACE(4, it);
@@ -262,8 +263,8 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           const int rq = q0 + col;
           const bool v = rq < p.T;
           const size_t si = (static_cast<size_t>(b) * p.H + hq) * p.T + (v ? rq : 0);
-          a_lse[col] = v ? p.lse[si] * kLog2e_b1 : 0.f;
-          a_dlt[col] = v ? p.delta[si] : 0.f;
+          a_lse[col] = v ? -p.lse[si] * kLog2e_b1 : 0.f;    // negated: the conversion adds
+          a_dlt[col] = v ? -p.delta[si] : 0.f;
           a_lo[col] = v ? (p.row_start ? max(p.row_start[static_cast<size_t>(b) * p.T + rq], p.window_left >= 0 ? rq - p.window_left : 0)
                                        : (p.window_left >= 0 ? max(rq - p.window_left, 0) : 0))
                         : 0x7fffffff;                 // invalid query rows see nothing
@@ -281,12 +282,11 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
     const uint32_t lane_off = static_cast<uint32_t>(qtr * 32) << 16;
     const int krow = qtr * 32 + lane;
     const bool plain_causal = p.row_start == nullptr && p.window_left < 0 && k0 + B1T <= p.T;
-    const int tid128 = qtr * 32 + lane;
     const float sl2 = p.scale_log2;
+    const float2 sl2x2 = make_float2(sl2, sl2);
     bool ok = true;
     for (int it = 0; it < n_iter; ++it) {
       const int st = it & 1; const uint32_t ph = it & 1;
-      const int hq = g * group + it / tiles_per_head;
       const int q0 = (i_begin + it % tiles_per_head) * B1T;
       const float* a_lse = aux + st * 3 * B1T;
       const float* a_dlt = a_lse + B1T;
@@ -309,11 +309,11 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
           const float4* l4 = reinterpret_cast<const float4*>(a_lse + cbase);
 #pragma unroll
           for (int v4 = 0; v4 < 16; ++v4) {
-            const float4 ls = l4[v4];
-            pk[2 * v4] = pack_bf16x2(exp2f(fmaf(__uint_as_float(sr[4 * v4]), sl2, -ls.x)),
-                                     exp2f(fmaf(__uint_as_float(sr[4 * v4 + 1]), sl2, -ls.y)));
-            pk[2 * v4 + 1] = pack_bf16x2(exp2f(fmaf(__uint_as_float(sr[4 * v4 + 2]), sl2, -ls.z)),
-                                         exp2f(fmaf(__uint_as_float(sr[4 * v4 + 3]), sl2, -ls.w)));
+            const float4 ls = l4[v4];                   // −lse·log2(e)
+            const float2 xa = fma_f32x2(make_float2(__uint_as_float(sr[4 * v4]), __uint_as_float(sr[4 * v4 + 1])), sl2x2, make_float2(ls.x, ls.y));
+            const float2 xb = fma_f32x2(make_float2(__uint_as_float(sr[4 * v4 + 2]), __uint_as_float(sr[4 * v4 + 3])), sl2x2, make_float2(ls.z, ls.w));
+            pk[2 * v4] = pack_bf16x2(exp2f(xa.x), exp2f(xa.y));
+            pk[2 * v4 + 1] = pack_bf16x2(exp2f(xb.x), exp2f(xb.y));
           }
         } else {
 #pragma unroll
@@ -323,7 +323,7 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
             for (int u = 0; u < 2; ++u) {
               const int col = cbase + 2 * e + u;
               const int rq = q0 + col;
-              float pr = exp2f(fmaf(__uint_as_float(sr[2 * e + u]), sl2, -a_lse[col]));
+              float pr = exp2f(fmaf(__uint_as_float(sr[2 * e + u]), sl2, a_lse[col]));
               if (!key_valid || kk > rq || kk < a_lo[col]) pr = 0.f;
               pv[u] = pr;
             }
@@ -358,10 +358,12 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 #pragma unroll
           for (int j = 0; j < 2; ++j) {
             const int v4 = v8 * 2 + j;                  // queries cbase + 4·v4 .. + 3
-            const float4 dl = d4[v4];
-            const float2 pa = unpack_bf16x2(pk[2 * v4]), pb = unpack_bf16x2(pk[2 * v4 + 1]);
-            w4[2 * j] = pack_bf16x2(pa.x * (__uint_as_float(dr[4 * v4]) - dl.x), pa.y * (__uint_as_float(dr[4 * v4 + 1]) - dl.y));
-            w4[2 * j + 1] = pack_bf16x2(pb.x * (__uint_as_float(dr[4 * v4 + 2]) - dl.z), pb.y * (__uint_as_float(dr[4 * v4 + 3]) - dl.w));
+            const float4 dl = d4[v4];                   // −δ
+            const float2 da = add_f32x2(make_float2(__uint_as_float(dr[4 * v4]), __uint_as_float(dr[4 * v4 + 1])), make_float2(dl.x, dl.y));
+            const float2 db = add_f32x2(make_float2(__uint_as_float(dr[4 * v4 + 2]), __uint_as_float(dr[4 * v4 + 3])), make_float2(dl.z, dl.w));
+            const float2 pa = mul_f32x2(unpack_bf16x2(pk[2 * v4]), da), pb = mul_f32x2(unpack_bf16x2(pk[2 * v4 + 1]), db);
+            w4[2 * j] = pack_bf16x2(pa.x, pa.y);
+            w4[2 * j + 1] = pack_bf16x2(pb.x, pb.y);
           }
           *reinterpret_cast<uint4*>(row + ((v8 ^ (krow & 7)) << 4)) = make_uint4(w4[0], w4[1], w4[2], w4[3]);
         }

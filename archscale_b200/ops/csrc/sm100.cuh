@@ -343,6 +343,34 @@ __device__ __forceinline__ float column_sum_block(const float* __restrict__ part
   return t;
 }
 
+// ------------------------------------------------------------------ two fp32 operations per instruction
+// fma / mul / add.rn.f32x2: each half is rounded like the scalar operation.
+__device__ __forceinline__ unsigned long long pack_f32x2(float2 f) {
+  unsigned long long r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(f.x), "f"(f.y));
+  return r;
+}
+__device__ __forceinline__ float2 unpack_f32x2(unsigned long long v) {
+  float2 f;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
+  return f;
+}
+__device__ __forceinline__ float2 fma_f32x2(float2 a, float2 b, float2 c) {
+  unsigned long long r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(pack_f32x2(a)), "l"(pack_f32x2(b)), "l"(pack_f32x2(c)));
+  return unpack_f32x2(r);
+}
+__device__ __forceinline__ float2 mul_f32x2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack_f32x2(a)), "l"(pack_f32x2(b)));
+  return unpack_f32x2(r);
+}
+__device__ __forceinline__ float2 add_f32x2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(pack_f32x2(a)), "l"(pack_f32x2(b)));
+  return unpack_f32x2(r);
+}
+
 // ------------------------------------------------------------------ misc
 __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
   uint32_t v;
