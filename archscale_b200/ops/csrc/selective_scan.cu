@@ -2,40 +2,80 @@
 //   dt_t = softplus(delta_t + bias),  h_t = exp(dt_t·A)·h_{t-1} + dt_t·B_t·u_t,  y_t = C_t·h_t + D·u_t  (·silu(z_t))
 // with N = 16 states per channel and an optional per-token reset flag (start of a packed document: h_{t-1} := 0).
 //
-// Work decomposition: one thread per (batch, channel, state); a warp holds 2 channels × 16 states, a CTA 16 channels.
-// Time runs sequentially inside the thread in tiles of 64 steps that the CTA stages through shared memory with
-// 32-byte row segments; sums over the 16 states use a 15-shuffle "reduce-scatter" per 16 steps (lane n ends up with
-// the total of step n), so the recurrence itself is one FMA per step and everything else has ILP across steps.
-// The forward stores the state entering every 32-step half tile (fp32, L/32 × Di × 16); the backward walks the halves
-// in reverse, recomputes the 32 states of a half into registers and runs the adjoint recurrence
+// Work decomposition: NS (2 or 4) states per thread, 16/NS threads per channel, 16 channels per CTA, time sequential inside
+// the thread.  What bounds it is one exponential per (step, channel, state) on MUFU (B4 L4096 Di3968: 1.04e9 of them, 0.23 ms):
+// everything else has to stay below that.  With one state per thread (what this file did before) every step cost four
+// shared-memory loads, fifteen sixteenths of a shuffle and its selects per state.  Several states per thread share the loads of dt and dt·u, read B and C as vectors, do two states per instruction
+// (fma.rn.f32x2) and add most of the sum over states in registers; the remaining 16/NS lanes use a reduce-scatter over 16/NS
+// steps (lane q ends up with the total of step q).  Measured, one state -> several states per thread, ms:
+//   B4 L4096 Di3968   forward 1.17 -> 0.59   backward 3.91 -> 2.82        B1 L32768 Di3968  forward 4.05 -> 2.73
+//   B8 L4096 Di4096   forward 2.06 -> 1.07   backward 7.35 -> 4.92        B1 L8192 Di5120   forward 1.13 -> 0.76   backward 3.74 -> 2.05
+//
+// The forward stages tiles of 64 steps through shared memory (the next tile's loads are in flight during the steps) and
+// stores the state entering every 32-step half tile (fp32, L/32 × Di × 16).  The backward walks 32-step tiles in reverse,
+// recomputes the 32 states from their checkpoint into registers (two states per thread: 64 registers) and runs the adjoint
 //   G_t = C_t·dy'_t + a_{t+1}·G_{t+1}
-// dB/dC (sums over channels) are reduced over the CTA's 16 channels in shared memory, written as per-CTA partial
-// sums and summed over channel blocks by a second kernel (deterministic, no atomics).
+// dB/dC (sums over channels) are reduced over the warp's 4 channels by shuffles and over the CTA's 4 warps in shared memory,
+// written as per-CTA partial sums and summed over channel blocks by a second kernel (deterministic, no atomics).
 #include "sm100.cuh"
 #include "api.h"
 
 namespace b200 {
 
-constexpr int SS_T = 64;    // steps per tile (= checkpoint interval)
+constexpr int SS_T = 64;    // steps per forward tile
+constexpr int SS_TB = 32;   // steps per backward tile (= checkpoint interval)
 constexpr int SS_C = 16;    // channels per CTA
 constexpr int SS_N = 16;    // states per channel
+constexpr int SS_YP = 24;   // row pitch of the per-step sums: 8-channel rows of neighbouring steps fall into different banks
 constexpr float SS_LOG2E = 1.4426950408889634f;
 
-template <typename T> __device__ __forceinline__ float ld1(const T* p);
-template <> __device__ __forceinline__ float ld1<float>(const float* p) { return *p; }
-template <> __device__ __forceinline__ float ld1<__nv_bfloat16>(const __nv_bfloat16* p) { return __bfloat162float(*p); }
 template <typename T> __device__ __forceinline__ void st1(T* p, float v);
 template <> __device__ __forceinline__ void st1<float>(float* p, float v) { *p = v; }
 template <> __device__ __forceinline__ void st1<__nv_bfloat16>(__nv_bfloat16* p, float v) { *p = __float2bfloat16(v); }
 
+// four neighbouring elements as they lie in memory; `vec`: the address is a multiple of their size
+template <typename T> struct Raw4;
+template <> struct Raw4<float> {
+  float4 v;
+  __device__ __forceinline__ void zero() { v = make_float4(0.f, 0.f, 0.f, 0.f); }
+  __device__ __forceinline__ void load(const float* p, bool vec) {
+    if (vec) v = *reinterpret_cast<const float4*>(p);
+    else v = make_float4(p[0], p[1], p[2], p[3]);
+  }
+  __device__ __forceinline__ float4 get() const { return v; }
+};
+template <> struct Raw4<__nv_bfloat16> {
+  uint2 v;
+  __device__ __forceinline__ void zero() { v = make_uint2(0u, 0u); }
+  __device__ __forceinline__ void load(const __nv_bfloat16* p, bool vec) {
+    if (vec) { v = *reinterpret_cast<const uint2*>(p); return; }
+    const unsigned short* s = reinterpret_cast<const unsigned short*>(p);
+    v.x = s[0] | (static_cast<uint32_t>(s[1]) << 16);
+    v.y = s[2] | (static_cast<uint32_t>(s[3]) << 16);
+  }
+  __device__ __forceinline__ float4 get() const {
+    const float2 a = unpack_bf16x2(v.x), b = unpack_bf16x2(v.y);
+    return make_float4(a.x, a.y, b.x, b.y);
+  }
+};
+__device__ __forceinline__ void put4(float* p, float4 v) { *reinterpret_cast<float4*>(p) = v; }
+__device__ __forceinline__ void put4(__nv_bfloat16* p, float4 v) {
+  *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16x2(v.x, v.y), pack_bf16x2(v.z, v.w));
+}
+// row stride and base of a [rows, 16·k] operand allow vector loads of four elements
+template <typename T> __host__ __device__ __forceinline__ bool rows_vec4(const T* p, int stride) {
+  return p == nullptr || (reinterpret_cast<uintptr_t>(p) % (4 * sizeof(T)) == 0 && stride % 4 == 0);
+}
+
 __device__ __forceinline__ float ss_softplus(float x) { return x > 20.f ? x : log1pf(__expf(x)); }
 __device__ __forceinline__ float ss_sigmoid(float x) { return 1.f / (1.f + __expf(-x)); }
 
-// v[s] (s = 0..15) summed over the 16 lanes of a half warp; lane n returns the total of step n.
-__device__ __forceinline__ float treduce16(float (&v)[16], int n) {
+// v[s] (s = 0..W-1) summed over W neighbouring lanes (lane index q inside the group); lane q returns the total of step q.
+template <int W>
+__device__ __forceinline__ float lane_scatter_sum(float (&v)[W], int q) {
 #pragma unroll
-  for (int w = 8; w >= 1; w >>= 1) {
-    const bool hi = (n & w) != 0;
+  for (int w = W / 2; w >= 1; w >>= 1) {
+    const bool hi = (q & w) != 0;
 #pragma unroll
     for (int k = 0; k < w; ++k) {
       const float send = hi ? v[k] : v[k + w];
@@ -46,201 +86,331 @@ __device__ __forceinline__ float treduce16(float (&v)[16], int n) {
   return v[0];
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256)
+template <typename T, int NS, bool RESET>
+__global__ void __launch_bounds__(SS_C * SS_N / NS)
 sscan_fwd_kernel(const T* __restrict__ u, int su, const T* __restrict__ delta, int sd, const float* __restrict__ A,
                  const T* __restrict__ Bm, int sB, const T* __restrict__ Cm, int sC, const float* __restrict__ Dp,
                  const T* __restrict__ z, int sz, const float* __restrict__ dbias, const int* __restrict__ reset,
                  T* __restrict__ y, float* __restrict__ ckpt, int L, int Di, int softplus) {
-  __shared__ float s_dt[SS_T][SS_C], s_dtu[SS_T][SS_C], s_B[SS_T][SS_N], s_C[SS_T][SS_N], s_y[SS_T][SS_C];
+  constexpr int TPC = SS_N / NS;                     // threads per channel
+  constexpr int NT = SS_C * TPC;
+  constexpr int PPT = SS_T * SS_C / 4 / NT;          // 4-element pieces of a [64, 16] tile per thread
+  __shared__ __align__(16) float2 s_d[SS_T][SS_C];   // (dt, dt·u)
+  __shared__ __align__(16) float s_B[SS_T][SS_N], s_C[SS_T][SS_N], s_y[SS_T][SS_YP];
   __shared__ int s_reset[SS_T];
-  const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int cl = 2 * w + (lane >> 4), n = lane & 15;
+  const int tid = threadIdx.x;
+  const int cl = tid / TPC, q = tid % TPC;
   const int d0 = blockIdx.x * SS_C, b = blockIdx.y, d = d0 + cl;
-  const int ci = tid >> 4, cj = tid & 15;           // cooperative mapping: rows ci + 16k, column cj
-  const float A2 = A[d * SS_N + n] * SS_LOG2E;
-  const float bias_j = dbias ? dbias[d0 + cj] : 0.f, D_j = Dp ? Dp[d0 + cj] : 0.f;
+  const int pr = tid >> 2, pc = (tid & 3) * 4;       // staging: rows pr + k·NT/4, columns pc .. pc + 3
+  const bool vu = rows_vec4(u, su), vd = rows_vec4(delta, sd), vB = rows_vec4(Bm, sB), vC = rows_vec4(Cm, sC), vz = rows_vec4(z, sz);
+  float2 A2[NS / 2], h[NS / 2];
+#pragma unroll
+  for (int j = 0; j < NS / 2; ++j) {
+    A2[j] = make_float2(A[d * SS_N + q * NS + 2 * j] * SS_LOG2E, A[d * SS_N + q * NS + 2 * j + 1] * SS_LOG2E);
+    h[j] = make_float2(0.f, 0.f);
+  }
+  float4 bias4 = make_float4(0.f, 0.f, 0.f, 0.f), D4 = bias4;
+  if (dbias) bias4 = make_float4(dbias[d0 + pc], dbias[d0 + pc + 1], dbias[d0 + pc + 2], dbias[d0 + pc + 3]);
+  if (Dp) D4 = make_float4(Dp[d0 + pc], Dp[d0 + pc + 1], Dp[d0 + pc + 2], Dp[d0 + pc + 3]);
   const int nseg = (L + SS_T - 1) / SS_T;
   const size_t row0 = static_cast<size_t>(b) * L;
-  float h = 0.f;
+  Raw4<T> ru[PPT], rd[PPT], rB[PPT], rC[PPT];
+  auto fetch = [&](int t0) {
+#pragma unroll
+    for (int k = 0; k < PPT; ++k) {
+      const int t = t0 + pr + k * (NT / 4);
+      ru[k].zero(); rd[k].zero(); rB[k].zero(); rC[k].zero();
+      if (t < L) {
+        const size_t r = row0 + t;
+        ru[k].load(u + r * su + d0 + pc, vu);
+        rd[k].load(delta + r * sd + d0 + pc, vd);
+        rB[k].load(Bm + r * sB + pc, vB);
+        rC[k].load(Cm + r * sC + pc, vC);
+      }
+    }
+  };
+  fetch(0);
   for (int seg = 0; seg < nseg; ++seg) {
     const int t0 = seg * SS_T;
-    float ur[4];
+    Raw4<T> cu[PPT], cz[PPT];
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int i = ci + 16 * k, t = t0 + i;
-      float dt = 0.f, uu = 0.f, bv = 0.f, cv = 0.f;
-      if (t < L) {
-        const size_t r = row0 + t;
-        dt = ld1(delta + r * sd + d0 + cj) + bias_j;
-        if (softplus) dt = ss_softplus(dt);
-        uu = ld1(u + r * su + d0 + cj);
-        bv = ld1(Bm + r * sB + cj);
-        cv = ld1(Cm + r * sC + cj);
+    for (int k = 0; k < PPT; ++k) {
+      const int i = pr + k * (NT / 4);
+      cu[k] = ru[k];
+      float4 dt = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (t0 + i < L) {
+        const float4 x = rd[k].get();
+        dt = make_float4(x.x + bias4.x, x.y + bias4.y, x.z + bias4.z, x.w + bias4.w);
+        if (softplus) dt = make_float4(ss_softplus(dt.x), ss_softplus(dt.y), ss_softplus(dt.z), ss_softplus(dt.w));
       }
-      ur[k] = uu;
-      s_dt[i][cj] = dt; s_dtu[i][cj] = dt * uu; s_B[i][cj] = bv; s_C[i][cj] = cv;
+      const float4 uu = ru[k].get();
+      float4* o = reinterpret_cast<float4*>(&s_d[i][pc]);
+      o[0] = make_float4(dt.x, dt.x * uu.x, dt.y, dt.y * uu.y);
+      o[1] = make_float4(dt.z, dt.z * uu.z, dt.w, dt.w * uu.w);
+      *reinterpret_cast<float4*>(&s_B[i][pc]) = rB[k].get();
+      *reinterpret_cast<float4*>(&s_C[i][pc]) = rC[k].get();
     }
-    if (tid < SS_T) s_reset[tid] = (reset && t0 + tid < L) ? reset[row0 + t0 + tid] : 0;
+    if (RESET && tid < SS_T) s_reset[tid] = t0 + tid < L ? reset[row0 + t0 + tid] : 0;
+    __syncthreads();
+    if (seg + 1 < nseg) fetch(t0 + SS_T);
+    if (z) {
+#pragma unroll
+      for (int k = 0; k < PPT; ++k) {
+        const int t = t0 + pr + k * (NT / 4);
+        cz[k].zero();
+        if (t < L) cz[k].load(z + (row0 + t) * sz + d0 + pc, vz);
+      }
+    }
+#pragma unroll 1
+    for (int sb = 0; sb < SS_T / 8; ++sb) {
+      if ((sb & 3) == 0 && ckpt) {
+        float* cp = ckpt + ((static_cast<size_t>(b) * nseg * 2 + seg * 2 + (sb >> 2)) * Di + d) * SS_N + q * NS;
+        if constexpr (NS == 4) *reinterpret_cast<float4*>(cp) = make_float4(h[0].x, h[0].y, h[1].x, h[1].y);
+        else *reinterpret_cast<float2*>(cp) = h[0];
+      }
+      float p[8];
+#pragma unroll
+      for (int s = 0; s < 8; ++s) {
+        const int i = sb * 8 + s;
+        const float2 dd = s_d[i][cl];
+        float2 Bv[NS / 2], Cv[NS / 2];
+        if constexpr (NS == 4) {
+          const float4 b4 = *reinterpret_cast<const float4*>(&s_B[i][q * 4]), c4 = *reinterpret_cast<const float4*>(&s_C[i][q * 4]);
+          Bv[0] = make_float2(b4.x, b4.y); Bv[1] = make_float2(b4.z, b4.w);
+          Cv[0] = make_float2(c4.x, c4.y); Cv[1] = make_float2(c4.z, c4.w);
+        } else {
+          Bv[0] = *reinterpret_cast<const float2*>(&s_B[i][q * 2]);
+          Cv[0] = *reinterpret_cast<const float2*>(&s_C[i][q * 2]);
+        }
+        if (RESET && s_reset[i]) {
+#pragma unroll
+          for (int j = 0; j < NS / 2; ++j) h[j] = make_float2(0.f, 0.f);
+        }
+        const float2 dt2 = make_float2(dd.x, dd.x), du2 = make_float2(dd.y, dd.y);
+        float2 acc;
+#pragma unroll
+        for (int j = 0; j < NS / 2; ++j) {
+          const float2 e = mul_f32x2(dt2, A2[j]);
+          const float2 a = make_float2(exp2f(e.x), exp2f(e.y));
+          h[j] = fma_f32x2(a, h[j], mul_f32x2(du2, Bv[j]));
+          acc = j == 0 ? mul_f32x2(h[j], Cv[j]) : fma_f32x2(h[j], Cv[j], acc);
+        }
+        p[s] = acc.x + acc.y;
+      }
+#pragma unroll
+      for (int s0 = 0; s0 < 8; s0 += TPC) {
+        float v[TPC];
+#pragma unroll
+        for (int s = 0; s < TPC; ++s) v[s] = p[s0 + s];
+        const float tot = lane_scatter_sum<TPC>(v, q);
+        s_y[sb * 8 + s0 + q][cl] = tot;
+      }
+    }
     __syncthreads();
 #pragma unroll
-    for (int sb = 0; sb < SS_T / 16; ++sb) {
-      if ((sb & 1) == 0 && ckpt) ckpt[((static_cast<size_t>(b) * nseg * 2 + seg * 2 + (sb >> 1)) * Di + d) * SS_N + n] = h;
-      float p[16];
-#pragma unroll
-      for (int s = 0; s < 16; ++s) {
-        const int i = sb * 16 + s;
-        float a = exp2f(s_dt[i][cl] * A2);
-        if (s_reset[i]) a = 0.f;
-        h = a * h + s_dtu[i][cl] * s_B[i][n];
-        p[s] = h * s_C[i][n];
-      }
-      const float tot = treduce16(p, n);
-      s_y[sb * 16 + n][cl] = tot;
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int i = ci + 16 * k, t = t0 + i;
+    for (int k = 0; k < PPT; ++k) {
+      const int i = pr + k * (NT / 4), t = t0 + i;
       if (t < L) {
-        const size_t r = row0 + t;
-        float yv = s_y[i][cj] + D_j * ur[k];
-        if (z) { const float zz = ld1(z + r * sz + d0 + cj); yv *= zz * ss_sigmoid(zz); }
-        st1(y + r * Di + d0 + cj, yv);
+        const float4 sv = *reinterpret_cast<const float4*>(&s_y[i][pc]), uu = cu[k].get();
+        float4 yv = make_float4(sv.x + D4.x * uu.x, sv.y + D4.y * uu.y, sv.z + D4.z * uu.z, sv.w + D4.w * uu.w);
+        if (z) {
+          const float4 zz = cz[k].get();
+          yv.x *= zz.x * ss_sigmoid(zz.x); yv.y *= zz.y * ss_sigmoid(zz.y);
+          yv.z *= zz.z * ss_sigmoid(zz.z); yv.w *= zz.w * ss_sigmoid(zz.w);
+        }
+        put4(y + (row0 + t) * Di + d0 + pc, yv);
       }
     }
   }
 }
 
-template <typename T>
-__global__ void __launch_bounds__(256)
+template <typename T, bool RESET, bool GATE>
+__global__ void __launch_bounds__(128, 3)
 sscan_bwd_kernel(const T* __restrict__ dy, int sdy, const T* __restrict__ u, int su, const T* __restrict__ delta, int sd,
                  const float* __restrict__ A, const T* __restrict__ Bm, int sB, const T* __restrict__ Cm, int sC,
                  const float* __restrict__ Dp, const T* __restrict__ z, int sz, const float* __restrict__ dbias,
                  const int* __restrict__ reset, const float* __restrict__ ckpt, T* __restrict__ du, T* __restrict__ ddelta,
                  T* __restrict__ dz, float* __restrict__ dA, float* __restrict__ dBf, float* __restrict__ dCf,
                  float* __restrict__ dD, float* __restrict__ ddbias, int L, int Di, int softplus) {
-  extern __shared__ float ss_dyn[];
-  typedef float (*Tile)[SS_C];
-  Tile s_dt = reinterpret_cast<Tile>(ss_dyn), s_u = s_dt + SS_T, s_dyp = s_u + SS_T, s_B = s_dyp + SS_T, s_C = s_B + SS_T;
-  Tile s_ypre = s_C + SS_T, s_ddt = s_ypre + SS_T, s_du = s_ddt + SS_T;
-  // per-warp slabs for the channel sums of dB / dC: plain stores, summed over the 8 warps in the tile epilogue
-  float (*s_dBw)[SS_T][SS_N] = reinterpret_cast<float (*)[SS_T][SS_N]>(s_du + SS_T);
-  float (*s_dCw)[SS_T][SS_N] = s_dBw + 8;
-  int* s_reset = reinterpret_cast<int*>(s_dCw + 8);
+  __shared__ __align__(16) float4 s_d[SS_TB][SS_C];                    // (dt, dt·u, dy', u)
+  __shared__ __align__(16) float s_B[SS_TB][SS_N], s_C[SS_TB][SS_N];
+  __shared__ __align__(16) float s_y[SS_TB][SS_YP], s_gb[SS_TB][SS_YP], s_da[SS_TB][SS_YP];   // Σ_n of h·C, g·B, g·a·h₋·A
+  __shared__ __align__(16) float s_bc[4][SS_TB][32];                   // per warp: dB (columns 0..15) and dC (16..31) of its 4 channels
+  __shared__ int s_reset[SS_TB];
   const int tid = threadIdx.x, lane = tid & 31, w = tid >> 5;
-  const int cl = 2 * w + (lane >> 4), n = lane & 15;
+  const int cl = tid >> 3, q = tid & 7;
   const int d0 = blockIdx.x * SS_C, b = blockIdx.y, d = d0 + cl;
-  const int ci = tid >> 4, cj = tid & 15;
-  const float Araw = A[d * SS_N + n], A2 = Araw * SS_LOG2E;
-  const float bias_j = dbias ? dbias[d0 + cj] : 0.f, D_j = Dp ? Dp[d0 + cj] : 0.f;
-  const int nseg = (L + SS_T - 1) / SS_T;
+  const int pr = tid >> 2, pc = (tid & 3) * 4;       // staging: row pr, columns pc .. pc + 3
+  const bool vu = rows_vec4(u, su), vd = rows_vec4(delta, sd), vB = rows_vec4(Bm, sB), vC = rows_vec4(Cm, sC), vz = rows_vec4(z, sz),
+             vy = rows_vec4(dy, sdy);
+  const float2 Ar = make_float2(A[d * SS_N + q * 2], A[d * SS_N + q * 2 + 1]);
+  const float2 A2 = make_float2(Ar.x * SS_LOG2E, Ar.y * SS_LOG2E);
+  float4 bias4 = make_float4(0.f, 0.f, 0.f, 0.f), D4 = bias4;
+  if (dbias) bias4 = make_float4(dbias[d0 + pc], dbias[d0 + pc + 1], dbias[d0 + pc + 2], dbias[d0 + pc + 3]);
+  if (Dp) D4 = make_float4(Dp[d0 + pc], Dp[d0 + pc + 1], Dp[d0 + pc + 2], Dp[d0 + pc + 3]);
+  const int nseg = (L + SS_TB - 1) / SS_TB, nck = 2 * ((L + SS_T - 1) / SS_T);
   const size_t row0 = static_cast<size_t>(b) * L;
-  float G = 0.f;                 // a_{t+1}·G_{t+1}: adjoint arriving from later steps
-  float dA_acc = 0.f, dD_acc = 0.f, dbias_acc = 0.f;
-  for (int seg = nseg - 1; seg >= 0; --seg) {
-    const int t0 = seg * SS_T;
-    float ur[4], sg[4], dyr[4], zr[4];
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int i = ci + 16 * k, t = t0 + i;
-      float dt = 0.f, uu = 0.f, bv = 0.f, cv = 0.f, dyv = 0.f, zz = 0.f, sig = 1.f;
-      if (t < L) {
-        const size_t r = row0 + t;
-        dt = ld1(delta + r * sd + d0 + cj) + bias_j;
-        if (softplus) { sig = ss_sigmoid(dt); dt = ss_softplus(dt); }
-        uu = ld1(u + r * su + d0 + cj);
-        bv = ld1(Bm + r * sB + cj);
-        cv = ld1(Cm + r * sC + cj);
-        dyv = ld1(dy + r * sdy + d0 + cj);
-        if (z) zz = ld1(z + r * sz + d0 + cj);
-      }
-      ur[k] = uu; sg[k] = sig; dyr[k] = dyv; zr[k] = zz;
-      s_dt[i][cj] = dt; s_u[i][cj] = uu; s_B[i][cj] = bv; s_C[i][cj] = cv;
-      s_dyp[i][cj] = z ? dyv * zz * ss_sigmoid(zz) : dyv;
+  float2 G = make_float2(0.f, 0.f);                  // a_{t+1}·G_{t+1}: adjoint arriving from later steps
+  float2 dA_acc = make_float2(0.f, 0.f);
+  float4 dD_acc = make_float4(0.f, 0.f, 0.f, 0.f), db_acc = dD_acc;
+  Raw4<T> ru, rd, ry, rz, rB, rC;
+  float2 h0;
+  auto fetch = [&](int seg) {
+    const int t = seg * SS_TB + pr;
+    ru.zero(); rd.zero(); ry.zero(); rz.zero(); rB.zero(); rC.zero();
+    if (t < L) {
+      const size_t r = row0 + t;
+      ru.load(u + r * su + d0 + pc, vu);
+      rd.load(delta + r * sd + d0 + pc, vd);
+      ry.load(dy + r * sdy + d0 + pc, vy);
+      if (GATE) rz.load(z + r * sz + d0 + pc, vz);
+      rB.load(Bm + r * sB + pc, vB);
+      rC.load(Cm + r * sC + pc, vC);
     }
-    if (tid < SS_T) s_reset[tid] = (reset && t0 + tid < L) ? reset[row0 + t0 + tid] : 0;
-    __syncthreads();
+    h0 = *reinterpret_cast<const float2*>(&ckpt[((static_cast<size_t>(b) * nck + seg) * Di + d) * SS_N + q * 2]);
+  };
+  fetch(nseg - 1);
 #pragma unroll 1
-    for (int half = 1; half >= 0; --half) {      // 32-step halves: the recomputed states of a half fit in registers
-      float h = ckpt[((static_cast<size_t>(b) * nseg * 2 + seg * 2 + half) * Di + d) * SS_N + n];
-      float hs[32];              // state before each step of the half (0 where the step resets)
-#pragma unroll
-      for (int sbl = 0; sbl < 2; ++sbl) {
-        const int sb = half * 2 + sbl;
-        float p[16];
-#pragma unroll
-        for (int s = 0; s < 16; ++s) {
-          const int i = sb * 16 + s;
-          const float dt = s_dt[i][cl];
-          float a = exp2f(dt * A2);
-          if (s_reset[i]) { a = 0.f; h = 0.f; }
-          hs[sbl * 16 + s] = h;
-          h = a * h + dt * s_u[i][cl] * s_B[i][n];
-          p[s] = h * s_C[i][n];
-        }
-        const float tot = treduce16(p, n);
-        s_ypre[sb * 16 + n][cl] = tot;
-      }
-#pragma unroll
-      for (int sbl = 1; sbl >= 0; --sbl) {
-        const int sb = half * 2 + sbl;
-        float vdt[16], vdu[16];
-#pragma unroll
-        for (int s = 15; s >= 0; --s) {
-          const int i = sb * 16 + s;
-          const float dt = s_dt[i][cl], uu = s_u[i][cl], Bv = s_B[i][n], Cv = s_C[i][n], dyp = s_dyp[i][cl];
-          float a = exp2f(dt * A2);
-          if (s_reset[i]) a = 0.f;
-          const float hprev = hs[sbl * 16 + s];
-          const float ht = a * hprev + dt * uu * Bv;
-          const float g = G + Cv * dyp;
-          float vC = dyp * ht, vB = g * dt * uu;
-          const float daa = g * hprev * a;
-          dA_acc += daa * dt;
-          vdt[s] = daa * Araw + g * Bv * uu;
-          vdu[s] = g * dt * Bv;
-          G = g * a;
-          vB += __shfl_xor_sync(0xffffffffu, vB, 16);
-          vC += __shfl_xor_sync(0xffffffffu, vC, 16);
-          if (lane < 16) { s_dBw[w][i][n] = vB; s_dCw[w][i][n] = vC; }
-        }
-        const float tdt = treduce16(vdt, n), tdu = treduce16(vdu, n);
-        s_ddt[sb * 16 + n][cl] = tdt;
-        s_du[sb * 16 + n][cl] = tdu;
-      }
-    }
-    __syncthreads();
-#pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int i = ci + 16 * k, t = t0 + i;
+  for (int seg = nseg - 1; seg >= 0; --seg) {
+    const int t = seg * SS_TB + pr;
+    const float4 uu = ru.get(), yy = ry.get(), zz = rz.get();
+    float4 dt = make_float4(0.f, 0.f, 0.f, 0.f), sg = make_float4(1.f, 1.f, 1.f, 1.f), sz4, dyp = yy;
+    {
       if (t < L) {
-        const size_t r = row0 + t;
-        const float dyp = z ? dyr[k] * zr[k] * ss_sigmoid(zr[k]) : dyr[k];
-        const float dd = s_ddt[i][cj] * sg[k];
-        st1(ddelta + r * Di + d0 + cj, dd);
-        dbias_acc += dd;
-        st1(du + r * Di + d0 + cj, s_du[i][cj] + dyp * D_j);
-        dD_acc += dyp * ur[k];
-        if (z) {
-          const float ypre = s_ypre[i][cj] + D_j * ur[k];
-          const float sgz = ss_sigmoid(zr[k]);
-          st1(dz + r * Di + d0 + cj, dyr[k] * ypre * sgz * (1.f + zr[k] * (1.f - sgz)));
+        const float4 x = rd.get();
+        dt = make_float4(x.x + bias4.x, x.y + bias4.y, x.z + bias4.z, x.w + bias4.w);
+        if (softplus) {
+          sg = make_float4(ss_sigmoid(dt.x), ss_sigmoid(dt.y), ss_sigmoid(dt.z), ss_sigmoid(dt.w));
+          dt = make_float4(ss_softplus(dt.x), ss_softplus(dt.y), ss_softplus(dt.z), ss_softplus(dt.w));
         }
-        float sb = 0.f, sc = 0.f;
+      }
+      if (GATE) {
+        sz4 = make_float4(ss_sigmoid(zz.x), ss_sigmoid(zz.y), ss_sigmoid(zz.z), ss_sigmoid(zz.w));
+        dyp = make_float4(yy.x * zz.x * sz4.x, yy.y * zz.y * sz4.y, yy.z * zz.z * sz4.z, yy.w * zz.w * sz4.w);
+      }
+      s_d[pr][pc] = make_float4(dt.x, dt.x * uu.x, dyp.x, uu.x);
+      s_d[pr][pc + 1] = make_float4(dt.y, dt.y * uu.y, dyp.y, uu.y);
+      s_d[pr][pc + 2] = make_float4(dt.z, dt.z * uu.z, dyp.z, uu.z);
+      s_d[pr][pc + 3] = make_float4(dt.w, dt.w * uu.w, dyp.w, uu.w);
+      *reinterpret_cast<float4*>(&s_B[pr][pc]) = rB.get();
+      *reinterpret_cast<float4*>(&s_C[pr][pc]) = rC.get();
+    }
+    if (RESET && tid < SS_TB) s_reset[tid] = seg * SS_TB + tid < L ? reset[row0 + seg * SS_TB + tid] : 0;
+    const float2 hin = h0;
+    __syncthreads();
+    if (seg > 0) fetch(seg - 1);
+    // ---- states after every step of the tile
+    float2 hs[SS_TB];
+    {
+      float2 h = hin;
 #pragma unroll
-        for (int ww = 0; ww < 8; ++ww) { sb += s_dBw[ww][i][cj]; sc += s_dCw[ww][i][cj]; }
-        // partial sums of this 16-channel block; summed over blocks by sscan_reduce_bc_kernel
-        const size_t po = (static_cast<size_t>(blockIdx.x) * gridDim.y * L + r) * SS_N + cj;
-        dBf[po] = sb;
-        dCf[po] = sc;
+      for (int s0 = 0; s0 < SS_TB; s0 += 8) {
+        float p[8];
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+          const int i = s0 + s;
+          const float2 dd = *reinterpret_cast<const float2*>(&s_d[i][cl]);
+          const float2 Bv = *reinterpret_cast<const float2*>(&s_B[i][q * 2]);
+          if (RESET && s_reset[i]) h = make_float2(0.f, 0.f);
+          const float2 e = mul_f32x2(make_float2(dd.x, dd.x), A2);
+          h = fma_f32x2(make_float2(exp2f(e.x), exp2f(e.y)), h, mul_f32x2(make_float2(dd.y, dd.y), Bv));
+          hs[i] = h;
+          if (GATE) {
+            const float2 c = mul_f32x2(h, *reinterpret_cast<const float2*>(&s_C[i][q * 2]));
+            p[s] = c.x + c.y;
+          }
+        }
+        if (GATE) s_y[s0 + q][cl] = lane_scatter_sum<8>(p, q);
+        __syncwarp();                                // keeps the loads of the next steps from being moved up here (registers)
       }
     }
+    // ---- adjoint, last step first
+#pragma unroll
+    for (int s0 = SS_TB - 8; s0 >= 0; s0 -= 8) {
+      float vgb[8], vda[8];
+#pragma unroll
+      for (int s = 7; s >= 0; --s) {
+        const int i = s0 + s;
+        const float4 dd = s_d[i][cl];
+        const float2 Bv = *reinterpret_cast<const float2*>(&s_B[i][q * 2]), Cv = *reinterpret_cast<const float2*>(&s_C[i][q * 2]);
+        const float2 e = mul_f32x2(make_float2(dd.x, dd.x), A2);
+        float2 a = make_float2(exp2f(e.x), exp2f(e.y));
+        float2 hp = i > 0 ? hs[i > 0 ? i - 1 : 0] : hin;
+        if (RESET && s_reset[i]) { a = make_float2(0.f, 0.f); hp = a; }
+        const float2 g = fma_f32x2(Cv, make_float2(dd.z, dd.z), G);
+        G = mul_f32x2(g, a);
+        const float2 daa = mul_f32x2(G, hp);
+        dA_acc = fma_f32x2(daa, make_float2(dd.x, dd.x), dA_acc);
+        const float2 gb = mul_f32x2(g, Bv), da = mul_f32x2(daa, Ar);
+        vgb[s] = gb.x + gb.y;
+        vda[s] = da.x + da.y;
+        const float2 vB2 = mul_f32x2(g, make_float2(dd.y, dd.y)), vC2 = mul_f32x2(hs[i], make_float2(dd.z, dd.z));
+        // four values over the warp's four channels: lane bit 4 keeps dB or dC, lane bit 3 the first or the second state
+        const bool hi = (lane & 16) != 0, odd = (lane & 8) != 0;
+        const float s0v = hi ? vB2.x : vC2.x, s1v = hi ? vB2.y : vC2.y;
+        const float k0 = (hi ? vC2.x : vB2.x) + __shfl_xor_sync(0xffffffffu, s0v, 16);
+        const float k1 = (hi ? vC2.y : vB2.y) + __shfl_xor_sync(0xffffffffu, s1v, 16);
+        const float kk = (odd ? k1 : k0) + __shfl_xor_sync(0xffffffffu, odd ? k0 : k1, 8);
+        s_bc[w][i][(hi ? 16 : 0) + 2 * q + (odd ? 1 : 0)] = kk;
+        if (s == 4) __syncwarp();
+      }
+      s_gb[s0 + q][cl] = lane_scatter_sum<8>(vgb, q);
+      s_da[s0 + q][cl] = lane_scatter_sum<8>(vda, q);
+      __syncwarp();
+    }
     __syncthreads();
+    if (t < L) {
+      const size_t r = row0 + t;
+      const float4 gb = *reinterpret_cast<const float4*>(&s_gb[pr][pc]), da = *reinterpret_cast<const float4*>(&s_da[pr][pc]);
+      const float4 dd = make_float4((da.x + gb.x * uu.x) * sg.x, (da.y + gb.y * uu.y) * sg.y, (da.z + gb.z * uu.z) * sg.z,
+                                    (da.w + gb.w * uu.w) * sg.w);
+      put4(ddelta + r * Di + d0 + pc, dd);
+      db_acc.x += dd.x; db_acc.y += dd.y; db_acc.z += dd.z; db_acc.w += dd.w;
+      put4(du + r * Di + d0 + pc, make_float4(gb.x * dt.x + dyp.x * D4.x, gb.y * dt.y + dyp.y * D4.y, gb.z * dt.z + dyp.z * D4.z,
+                                              gb.w * dt.w + dyp.w * D4.w));
+      dD_acc.x += dyp.x * uu.x; dD_acc.y += dyp.y * uu.y; dD_acc.z += dyp.z * uu.z; dD_acc.w += dyp.w * uu.w;
+      if (GATE) {
+        const float4 sv = *reinterpret_cast<const float4*>(&s_y[pr][pc]);
+        put4(dz + r * Di + d0 + pc,
+             make_float4(yy.x * (sv.x + D4.x * uu.x) * sz4.x * (1.f + zz.x * (1.f - sz4.x)),
+                         yy.y * (sv.y + D4.y * uu.y) * sz4.y * (1.f + zz.y * (1.f - sz4.y)),
+                         yy.z * (sv.z + D4.z * uu.z) * sz4.z * (1.f + zz.z * (1.f - sz4.z)),
+                         yy.w * (sv.w + D4.w * uu.w) * sz4.w * (1.f + zz.w * (1.f - sz4.w))));
+      }
+      // partial sums of this 16-channel block; summed over blocks by sscan_reduce_bc_kernel
+      const size_t po = (static_cast<size_t>(blockIdx.x) * gridDim.y * L + r) * SS_N + pc;
+#pragma unroll
+      for (int half = 0; half < 2; ++half) {
+        float4 a = *reinterpret_cast<const float4*>(&s_bc[0][pr][half * 16 + pc]);
+#pragma unroll
+        for (int ww = 1; ww < 4; ++ww) {
+          const float4 o = *reinterpret_cast<const float4*>(&s_bc[ww][pr][half * 16 + pc]);
+          a.x += o.x; a.y += o.y; a.z += o.z; a.w += o.w;
+        }
+        *reinterpret_cast<float4*>((half ? dCf : dBf) + po) = a;
+      }
+    }
+    // the next tile's staging writes s_d / s_B / s_C only (nobody reads them here any more); its sums are written after its barrier
   }
-  atomicAdd(&dA[d * SS_N + n], dA_acc);
-  if (dD) atomicAdd(&dD[d0 + cj], dD_acc);
-  if (ddbias) atomicAdd(&ddbias[d0 + cj], dbias_acc);
+  atomicAdd(&dA[d * SS_N + q * 2], dA_acc.x);
+  atomicAdd(&dA[d * SS_N + q * 2 + 1], dA_acc.y);
+#pragma unroll
+  for (int o = 4; o < 32; o <<= 1) {                 // the 8 rows of a warp
+    dD_acc.x += __shfl_xor_sync(0xffffffffu, dD_acc.x, o); dD_acc.y += __shfl_xor_sync(0xffffffffu, dD_acc.y, o);
+    dD_acc.z += __shfl_xor_sync(0xffffffffu, dD_acc.z, o); dD_acc.w += __shfl_xor_sync(0xffffffffu, dD_acc.w, o);
+    db_acc.x += __shfl_xor_sync(0xffffffffu, db_acc.x, o); db_acc.y += __shfl_xor_sync(0xffffffffu, db_acc.y, o);
+    db_acc.z += __shfl_xor_sync(0xffffffffu, db_acc.z, o); db_acc.w += __shfl_xor_sync(0xffffffffu, db_acc.w, o);
+  }
+  if (lane < 4) {
+    if (dD) {
+      atomicAdd(&dD[d0 + pc], dD_acc.x); atomicAdd(&dD[d0 + pc + 1], dD_acc.y);
+      atomicAdd(&dD[d0 + pc + 2], dD_acc.z); atomicAdd(&dD[d0 + pc + 3], dD_acc.w);
+    }
+    if (ddbias) {
+      atomicAdd(&ddbias[d0 + pc], db_acc.x); atomicAdd(&ddbias[d0 + pc + 1], db_acc.y);
+      atomicAdd(&ddbias[d0 + pc + 2], db_acc.z); atomicAdd(&ddbias[d0 + pc + 3], db_acc.w);
+    }
+  }
 }
 
 // dB / dC [rows, 16] = Σ over channel blocks of the partial sums [nblk, rows, 16] written by the backward.
@@ -256,8 +426,6 @@ __global__ void __launch_bounds__(256) sscan_reduce_bc_kernel(const float* __res
   st1(dC + i, sc);
 }
 
-constexpr int SS_BWD_SMEM = (8 * SS_T * SS_C + 16 * SS_T * SS_N) * 4 + SS_T * 4;
-
 }  // namespace b200
 
 using namespace b200;
@@ -265,6 +433,15 @@ using namespace b200;
 extern "C" int b200_selective_scan_channel_blocks(int Di) { return Di / SS_C; }
 
 extern "C" int b200_selective_scan_ckpt_segments(int L) { return 2 * ((L + SS_T - 1) / SS_T); }
+
+template <typename T, int NS>
+static void launch_sscan_fwd(const void* u, int su, const void* delta, int sd, const float* A, const void* Bm, int sB, const void* Cm,
+                             int sC, const float* D, const void* z, int sz, const float* dbias, const int* reset, void* y, float* ckpt,
+                             int B, int L, int Di, int softplus, cudaStream_t st) {
+  auto kern = reset ? sscan_fwd_kernel<T, NS, true> : sscan_fwd_kernel<T, NS, false>;
+  kern<<<dim3(Di / SS_C, B), SS_C * SS_N / NS, 0, st>>>((const T*)u, su, (const T*)delta, sd, A, (const T*)Bm, sB, (const T*)Cm, sC, D,
+                                                       (const T*)z, sz, dbias, reset, (T*)y, ckpt, L, Di, softplus);
+}
 
 // u, delta, z: rows of `su`, `sd`, `sz` elements; Bm, Cm: [B·L, 16] with row strides sB, sC; y: dense [B, L, Di].
 // reset: int32 per token (1 = h is cleared before this step) or null.  ckpt: fp32 [B, 2·ceil(L/64), Di, 16] or null.
@@ -274,19 +451,28 @@ extern "C" int b200_selective_scan_fwd(const void* u, int su, const void* delta,
                                        cudaStream_t st) {
   if (Di % SS_C) return -1;
   if (B * L == 0) return 0;
-  dim3 grid(Di / SS_C, B);
-  if (dtype == 1)
-    sscan_fwd_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)u, su, (const __nv_bfloat16*)delta, sd, A,
-        (const __nv_bfloat16*)Bm, sB, (const __nv_bfloat16*)Cm, sC, D, (const __nv_bfloat16*)z, sz, dbias, reset,
-        (__nv_bfloat16*)y, ckpt, L, Di, softplus);
-  else
-    sscan_fwd_kernel<float><<<grid, 256, 0, st>>>((const float*)u, su, (const float*)delta, sd, A, (const float*)Bm, sB,
-        (const float*)Cm, sC, D, (const float*)z, sz, dbias, reset, (float*)y, ckpt, L, Di, softplus);
+  // four states per thread need B·Di/8 warps to fill the 592 schedulers about three deep; below that two states per thread
+  const bool ns4 = static_cast<long long>(B) * Di >= 12288;
+  auto run = dtype == 1 ? (ns4 ? launch_sscan_fwd<__nv_bfloat16, 4> : launch_sscan_fwd<__nv_bfloat16, 2>)
+                        : (ns4 ? launch_sscan_fwd<float, 4> : launch_sscan_fwd<float, 2>);
+  run(u, su, delta, sd, A, Bm, sB, Cm, sC, D, z, sz, dbias, reset, y, ckpt, B, L, Di, softplus, st);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
-// dA [Di,16], dD [Di], ddbias [Di] are fp32 accumulators that must be zero on entry.  partB / partC: fp32 scratch
-// [Di/16, B·L, 16] (fully overwritten); dB / dC: [B·L, 16] in the activation dtype.
+template <typename T>
+static void launch_sscan_bwd(const void* dy, int sdy, const void* u, int su, const void* delta, int sd, const float* A, const void* Bm,
+                             int sB, const void* Cm, int sC, const float* D, const void* z, int sz, const float* dbias, const int* reset,
+                             const float* ckpt, void* du, void* ddelta, void* dz, float* dA, float* partB, float* partC, void* dB,
+                             void* dC, float* dD, float* ddbias, int B, int L, int Di, int softplus, cudaStream_t st) {
+  auto kern = reset ? (z ? sscan_bwd_kernel<T, true, true> : sscan_bwd_kernel<T, true, false>)
+                    : (z ? sscan_bwd_kernel<T, false, true> : sscan_bwd_kernel<T, false, false>);
+  kern<<<dim3(Di / SS_C, B), 128, 0, st>>>((const T*)dy, sdy, (const T*)u, su, (const T*)delta, sd, A, (const T*)Bm, sB, (const T*)Cm, sC,
+                                           D, (const T*)z, sz, dbias, reset, ckpt, (T*)du, (T*)ddelta, (T*)dz, dA, partB, partC, dD,
+                                           ddbias, L, Di, softplus);
+  const size_t n = static_cast<size_t>(B) * L * SS_N;
+  sscan_reduce_bc_kernel<T><<<static_cast<unsigned>((n + 255) / 256), 256, 0, st>>>(partB, partC, (T*)dB, (T*)dC, n, Di / SS_C);
+}
+
 extern "C" int b200_selective_scan_bwd(const void* dy, int sdy, const void* u, int su, const void* delta, int sd, const float* A,
                                        const void* Bm, int sB, const void* Cm, int sC, const float* D, const void* z, int sz,
                                        const float* dbias, const int* reset, const float* ckpt, void* du, void* ddelta, void* dz,
@@ -294,27 +480,8 @@ extern "C" int b200_selective_scan_bwd(const void* dy, int sdy, const void* u, i
                                        int dtype, int B, int L, int Di, int softplus, cudaStream_t st) {
   if (Di % SS_C) return -1;
   if (B * L == 0) return 0;
-  dim3 grid(Di / SS_C, B);
-  static bool configured = false;
-  if (!configured) {
-    if (cudaFuncSetAttribute(sscan_bwd_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, SS_BWD_SMEM) != cudaSuccess ||
-        cudaFuncSetAttribute(sscan_bwd_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, SS_BWD_SMEM) != cudaSuccess)
-      return -2;
-    configured = true;
-  }
-  const size_t n = static_cast<size_t>(B) * L * SS_N;
-  const unsigned rgrid = static_cast<unsigned>((n + 255) / 256);
-  if (dtype == 1) {
-    sscan_bwd_kernel<__nv_bfloat16><<<grid, 256, SS_BWD_SMEM, st>>>((const __nv_bfloat16*)dy, sdy, (const __nv_bfloat16*)u, su,
-        (const __nv_bfloat16*)delta, sd, A, (const __nv_bfloat16*)Bm, sB, (const __nv_bfloat16*)Cm, sC, D,
-        (const __nv_bfloat16*)z, sz, dbias, reset, ckpt, (__nv_bfloat16*)du, (__nv_bfloat16*)ddelta, (__nv_bfloat16*)dz, dA,
-        partB, partC, dD, ddbias, L, Di, softplus);
-    sscan_reduce_bc_kernel<__nv_bfloat16><<<rgrid, 256, 0, st>>>(partB, partC, (__nv_bfloat16*)dB, (__nv_bfloat16*)dC, n, Di / SS_C);
-  } else {
-    sscan_bwd_kernel<float><<<grid, 256, SS_BWD_SMEM, st>>>((const float*)dy, sdy, (const float*)u, su, (const float*)delta, sd, A,
-        (const float*)Bm, sB, (const float*)Cm, sC, D, (const float*)z, sz, dbias, reset, ckpt, (float*)du, (float*)ddelta,
-        (float*)dz, dA, partB, partC, dD, ddbias, L, Di, softplus);
-    sscan_reduce_bc_kernel<float><<<rgrid, 256, 0, st>>>(partB, partC, (float*)dB, (float*)dC, n, Di / SS_C);
-  }
+  auto run = dtype == 1 ? launch_sscan_bwd<__nv_bfloat16> : launch_sscan_bwd<float>;
+  run(dy, sdy, u, su, delta, sd, A, Bm, sB, Cm, sC, D, z, sz, dbias, reset, ckpt, du, ddelta, dz, dA, partB, partC, dB, dC, dD, ddbias, B,
+      L, Di, softplus, st);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
