@@ -256,25 +256,28 @@ __global__ void __launch_bounds__(256) add_rmsnorm_bwd_kernel(const TG* __restri
   for (int c = threadIdx.x; c < cols; c += blockDim.x) dw_partial[static_cast<size_t>(blockIdx.x) * cols + c] = dw_s[c];
 }
 
-// The same backward with every row split over a PAIR of warps (cols == NCH·256, NCH even): a lane keeps NCH/2 chunks of the
+// The same backward with every row split over a PAIR of warps (cols ≤ NCH·256, NCH even, FULL: equal): a lane keeps NCH/2 chunks of the
 // weight-gradient accumulator instead of NCH and reads the weight from shared memory, which brings the kernel under 128
 // registers and two CTAs onto an SM (the one-warp-per-row form needs 255 registers at 2048 columns).  The two partial dot products of a row meet
 // in shared memory behind a 64-thread named barrier; two buffers alternate so that one barrier per row suffices.
-template <typename TX, typename TW, int NCH, typename TG>
+// Rows that do not fill the last chunks (1984 of 2048 columns) read clamped addresses and mask the sums as above.  Against one
+// warp per row (bf16 stream, ms): 16384 x 1984 0.209 -> 0.094, 16384 x 1536 0.165 -> 0.063, 16384 x 1280 0.155 -> 0.070.
+template <typename TX, typename TW, int NCH, bool FULL, typename TG>
 __global__ void __launch_bounds__(256, 2) add_rmsnorm_bwd2_kernel(const TG* __restrict__ g_res, const __nv_bfloat16* __restrict__ g_n,
                                                                  const TX* __restrict__ x, const TW* __restrict__ w,
                                                                  const float* __restrict__ rstd, TG* __restrict__ d_res,
                                                                  __nv_bfloat16* __restrict__ d_h, float h_scale,
                                                                  float* __restrict__ dw_partial, int rows, int cols) {
-  extern __shared__ float dw_s[];                                       // [cols] weight-gradient sums, then [cols] the weight in fp32
+  extern __shared__ float dw_s[];                                       // [NCH·256] weight-gradient sums, then the weight in fp32
   __shared__ float dot_s[2][8];
   constexpr int NCL = NCH / 2;
-  float* w_s = dw_s + cols;
+  float* w_s = dw_s + NCH * 256;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int pair = warp >> 1, half = warp & 1;
   const int c0 = lane * 8 + half * NCL * 256;                           // first column of this lane
-  for (int c = threadIdx.x * 8; c < cols; c += blockDim.x * 8) {
-    float t[8]; Vec8<TW>::load(w + c, t);
+  for (int c = threadIdx.x * 8; c < NCH * 256; c += blockDim.x * 8) {
+    float t[8];
+    Vec8<TW>::load(w + (FULL ? c : min(c, cols - 8)), t);
 #pragma unroll
     for (int e = 0; e < 8; ++e) { w_s[c + e] = t[e]; dw_s[c + e] = 0.f; }
   }
@@ -286,17 +289,19 @@ __global__ void __launch_bounds__(256, 2) add_rmsnorm_bwd2_kernel(const TG* __re
     for (int e = 0; e < 8; ++e) dwacc[i][e] = 0.f;
   int it = 0;
   for (int row = blockIdx.x * 4 + pair; row < rows; row += gridDim.x * 4, ++it) {
-    const size_t base = static_cast<size_t>(row) * cols + c0;
+    const size_t base = static_cast<size_t>(row) * cols;
     const float rs = rstd[row];
     float dot = 0.f;
 #pragma unroll
     for (int i = 0; i < NCL; ++i) {
+      const int c = c0 + i * 256, cl = FULL ? c : min(c, cols - 8);
+      const bool valid = FULL || c < cols;
       float xv[8], dv[8], wv[8];
-      Vec8<TX>::load(x + base + i * 256, xv);
-      Vec8<__nv_bfloat16>::load(g_n + base + i * 256, dv);
-      Vec8<float>::load(w_s + c0 + i * 256, wv);
+      Vec8<TX>::load(x + base + cl, xv);
+      Vec8<__nv_bfloat16>::load(g_n + base + cl, dv);
+      Vec8<float>::load(w_s + c, wv);
 #pragma unroll
-      for (int e = 0; e < 8; ++e) dot += dv[e] * wv[e] * xv[e];
+      for (int e = 0; e < 8; ++e) dot += valid ? dv[e] * wv[e] * xv[e] : 0.f;
     }
     dot = warp_sum(dot);
     if (lane == 0) dot_s[it & 1][warp] = dot;
@@ -305,25 +310,29 @@ __global__ void __launch_bounds__(256, 2) add_rmsnorm_bwd2_kernel(const TG* __re
     const float c1 = dot * rs * rs * rs / cols;
 #pragma unroll
     for (int i = 0; i < NCL; ++i) {
+      const int c = c0 + i * 256, cl = FULL ? c : min(c, cols - 8);
+      const bool valid = FULL || c < cols;
       float xv[8], dv[8], wv[8], o[8];             // second read of the row: L1 / L2 hits
-      Vec8<TX>::load(x + base + i * 256, xv);
-      Vec8<__nv_bfloat16>::load(g_n + base + i * 256, dv);
-      Vec8<float>::load(w_s + c0 + i * 256, wv);
+      Vec8<TX>::load(x + base + cl, xv);
+      Vec8<__nv_bfloat16>::load(g_n + base + cl, dv);
+      Vec8<float>::load(w_s + c, wv);
 #pragma unroll
       for (int e = 0; e < 8; ++e) {
         o[e] = dv[e] * wv[e] * rs - xv[e] * c1;
-        dwacc[i][e] += dv[e] * xv[e] * rs;
+        dwacc[i][e] += dv[e] * xv[e] * rs;         // columns beyond the row are summed too, but never written
       }
       if (g_res) {
-        float gr[8]; Vec8<TG>::load(g_res + base + i * 256, gr);
+        float gr[8]; Vec8<TG>::load(g_res + base + cl, gr);
 #pragma unroll
         for (int e = 0; e < 8; ++e) o[e] += gr[e];
       }
-      if (d_res) Vec8<TG>::store(d_res + base + i * 256, o);
-      if (d_h) {
+      if (valid) {
+        if (d_res) Vec8<TG>::store(d_res + base + c, o);
+        if (d_h) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) o[e] *= h_scale;
-        Vec8<__nv_bfloat16>::store(d_h + base + i * 256, o);
+          for (int e = 0; e < 8; ++e) o[e] *= h_scale;
+          Vec8<__nv_bfloat16>::store(d_h + base + c, o);
+        }
       }
     }
   }
@@ -479,11 +488,15 @@ extern "C" int b200_add_rmsnorm_bwd(const void* g_res, const void* g_n, const vo
   else L(bf, bf, NCH, float);
   // the instantiation with the fewest 256-column chunks that covers the row (the kernel skips what lies beyond `cols`)
   if (cols % 8 || cols > 4096) return -2;
-  if (use_pair_rows() && cols == 2048) {      // wider rows spill at 128 registers; 1024-wide rows measured no faster this way
+  // wider rows spill at 128 registers; 1024-wide rows measured no faster this way
+  if (use_pair_rows() && cols > 1024 && cols <= 2048) {
 #define L2(TX, TW, NCH, TG)                                                                                            \
-  add_rmsnorm_bwd2_kernel<TX, TW, NCH, TG><<<grid, 256, 2 * smem, stream>>>(                                               \
-      static_cast<const TG*>(g_res), static_cast<const bf*>(g_n), static_cast<const TX*>(x), static_cast<const TW*>(w), rstd, \
-      static_cast<TG*>(d_res), static_cast<bf*>(d_h), h_scale, dw_partial, rows, cols)
+  do {                                                                                                                 \
+    auto kern = cols == NCH * 256 ? add_rmsnorm_bwd2_kernel<TX, TW, NCH, true, TG> : add_rmsnorm_bwd2_kernel<TX, TW, NCH, false, TG>; \
+    kern<<<grid, 256, 2 * sizeof(float) * NCH * 256, stream>>>(                                                        \
+        static_cast<const TG*>(g_res), static_cast<const bf*>(g_n), static_cast<const TX*>(x), static_cast<const TW*>(w), rstd, \
+        static_cast<TG*>(d_res), static_cast<bf*>(d_h), h_scale, dw_partial, rows, cols);                              \
+  } while (0)
 #define LN2(NCH)                                                         \
   if (g_dtype == 1 && w_dtype == 0) L2(bf, float, NCH, bf);              \
   else if (g_dtype == 1) L2(bf, bf, NCH, bf);                            \
@@ -491,7 +504,7 @@ extern "C" int b200_add_rmsnorm_bwd(const void* g_res, const void* g_n, const vo
   else if (x_dtype == 0 && w_dtype == 1) L2(float, bf, NCH, float);      \
   else if (x_dtype == 1 && w_dtype == 0) L2(bf, float, NCH, float);      \
   else L2(bf, bf, NCH, float);
-    LN2(8)
+    if (cols <= 1536) { LN2(6) } else { LN2(8) }
 #undef LN2
 #undef L2
     reduce_partials_kernel<<<(cols + 31) / 32, 1024, 0, stream>>>(dw_partial, dw, grid, cols);
