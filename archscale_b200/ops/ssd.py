@@ -70,6 +70,12 @@ class _StateScanFn(torch.autograd.Function):
         return d_add, d_keep
 
 
+def _dense16(t: torch.Tensor) -> torch.Tensor:
+    """Contiguous and on a 16-byte boundary (the kernels read four elements at a time)."""
+    t = t.contiguous()
+    return t if t.data_ptr() % 16 == 0 else t.clone()
+
+
 class _IntraChunkFn(torch.autograd.Function):
     """``y[i] = Σ_{j ≤ i, same document} (C_i·B_j) · exp(cs_i − cs_j) · dt_j · x_j`` inside every chunk, on
     ``csrc/ssd_intra.cu``: the per-head 64×64 weights never reach memory.  x (B,Lp,H,P), dt (B,Lp,H), cs (B,nC,H,64),
@@ -77,7 +83,7 @@ class _IntraChunkFn(torch.autograd.Function):
 
     @staticmethod
     def forward(ctx, x, dt, cs, cb, bc):
-        x, dt, cs, cb = x.contiguous(), dt.contiguous(), cs.contiguous(), cb.contiguous()
+        x, dt, cs, cb = _dense16(x), dt.contiguous(), cs.contiguous(), cb.contiguous()
         y = backend.require_extension().ssd_intra_fwd(x, dt, cs, cb, bc)
         backend.count_launch()
         ctx.save_for_backward(x, dt, cs, cb, bc)
@@ -86,10 +92,67 @@ class _IntraChunkFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dy):
         x, dt, cs, cb, bc = ctx.saved_tensors
-        dx, ddt, dcs, dcb = backend.require_extension().ssd_intra_bwd(x, dt, cs, cb, bc, dy.float().contiguous())
+        dx, ddt, dcs, dcb = backend.require_extension().ssd_intra_bwd(x, dt, cs, cb, bc, _dense16(dy.to(x.dtype)))
         backend.count_launch()
         Bb, Lp, H, _ = x.shape
         return dx.to(x.dtype), ddt.permute(0, 1, 3, 2).reshape(Bb, Lp, H), dcs, dcb, None
+
+
+class _ChunkScanFn(torch.autograd.Function):
+    """The one-group scan over whole chunks with every pass over [tokens, H, P] in one place: the intra-chunk kernel, the chunk
+    summaries ``xwᵀ·B``, the state recurrence, the read-out ``C·S_inᵀ`` and the element-wise passes of ``csrc/ssd_rows.cu``, which
+    read x in its own type.  x (B,Lp,H,P); dt, wl, carry (B,nC,64,H) token-major, cs (B,nC,H,64), keep (B,nC,H) fp32;
+    Bc, Cc (B·nC,64,N) fp32; D (H,) fp32 or None; bc (B,nC,64) int32 or None → out like x."""
+
+    @staticmethod
+    def forward(ctx, x, dt, cs, Bc, Cc, wl, carry, keep, D, bc):
+        ext = backend.require_extension()
+        x = _dense16(x)
+        dt, cs, Bc, Cc, wl, carry, keep = (t.contiguous() for t in (dt, cs, Bc, Cc, wl, carry, keep))
+        Bb, Lp, H, P = x.shape
+        BN, c, N = Bc.shape
+        nC = Lp // c
+        cb = torch.bmm(Cc, Bc.transpose(1, 2)).view(Bb, nC, 1, c, c)
+        y = ext.ssd_intra_fwd(x, dt.view(Bb, Lp, H), cs, cb, bc)
+        w = dt * wl
+        xw = ext.ssd_scale(x, w)
+        add = torch.bmm(xw.view(BN, c, H * P).transpose(1, 2), Bc).view(Bb, nC, H, P, N)
+        s_in = ext.ssd_state_fwd(add, keep)                                              # state entering each chunk
+        y2 = torch.bmm(Cc, s_in.view(BN, H * P, N).transpose(1, 2))
+        out = ext.ssd_combine(y, y2, carry, x, D)
+        backend.count_launch(4)
+        ctx.save_for_backward(x, dt, cs, Bc, Cc, wl, carry, keep, D, bc, cb, w, xw, s_in, y2)
+        return out
+
+    @staticmethod
+    def backward(ctx, dout):
+        ext = backend.require_extension()
+        x, dt, cs, Bc, Cc, wl, carry, keep, D, bc, cb, w, xw, s_in, y2 = ctx.saved_tensors
+        dout = _dense16(dout)
+        Bb, Lp, H, P = x.shape
+        BN, c, N = Bc.shape
+        nC = Lp // c
+        dy2, dcarry, dxD = ext.ssd_dprep(dout, y2, carry, x)
+        dy2 = dy2.view(BN, c, H * P)
+        ds_in = torch.bmm(dy2.transpose(1, 2), Cc).view(Bb, nC, H, P, N)
+        dC = torch.bmm(dy2, s_in.view(BN, H * P, N))
+        d_add, d_keep = ext.ssd_state_bwd(ds_in, s_in, keep)
+        d_add = d_add.view(BN, H * P, N)
+        dxw = torch.bmm(Bc, d_add.transpose(1, 2))
+        dB = torch.bmm(xw.view(BN, c, H * P), d_add)
+        dxi, ddt, dcs, dcb = ext.ssd_intra_bwd(x, dt.view(Bb, Lp, H), cs, cb, bc, dout)
+        dcb = dcb.view(BN, c, c)
+        dC.baddbmm_(dcb, Bc)
+        dB.baddbmm_(dcb.transpose(1, 2), Cc)
+        dx, dw = ext.ssd_dfinish(dxi, dxw, w, dout, x, D)
+        backend.count_launch(5)
+        ddt = torch.addcmul(ddt.transpose(2, 3), dw, wl)
+        return (dx, ddt, dcs, dB, dC, dw * dt, dcarry, d_keep, dxD.view(-1, H).sum(0) if D is not None else None, None)
+
+
+def _chunk_scan_ok(x: torch.Tensor, B: torch.Tensor, c: int) -> bool:
+    """One group on the kernels' types and sizes; the general form below stays for everything else."""
+    return B.shape[2] == 1 and (x.shape[3] * B.shape[3]) % 1024 == 0 and backend.has("ssd_scale") and _intra_kernel_ok(x, c)
 
 
 def _intra_kernel_ok(x: torch.Tensor, c: int) -> bool:
@@ -109,7 +172,10 @@ def ssd_scan(x, dt, A, B, C, D=None, seq_idx: Optional[torch.Tensor] = None, chu
     matmuls over all chunks at once; only the (B,H,P,N) state is carried from chunk to chunk in a short loop of
     element-wise updates.  Differentiable; equals :func:`ssd_scan_ref`."""
     dtype = x.dtype
-    x, dt, B, C = x.float(), dt.float(), B.float(), C.float()
+    fused = _chunk_scan_ok(x, B, chunk)                # x keeps its type: the kernels widen it as they read
+    dt, B, C = dt.float(), B.float(), C.float()
+    if not fused:
+        x = x.float()
     Bb, L, H, P = x.shape
     G, N = B.shape[2], B.shape[3]
     pad = (-L) % chunk
@@ -147,9 +213,12 @@ def ssd_scan(x, dt, A, B, C, D=None, seq_idx: Optional[torch.Tensor] = None, chu
     # inside a chunk: y_i = Σ_{j≤i} (C_i·B_j) · exp(cs_i − cs_j) · dt_j x_j
     Bh = B.view(Bb, nC, c, G, N)
     Ch = C.view(Bb, nC, c, G, N)
-    cb = torch.einsum("bnigk,bnjgk->bngij", Ch, Bh)                                      # (B,nC,G,c,c)
+    if not fused:
+        cb = torch.einsum("bnigk,bnjgk->bngij", Ch, Bh)                                  # (B,nC,G,c,c)
     rep = H // G
-    if _intra_kernel_ok(x, c):
+    if fused:
+        pass
+    elif _intra_kernel_ok(x, c):
         y = _IntraChunkFn.apply(x, dt, cs, cb, bc.to(torch.int32).contiguous() if brk is not None else None)
         y = y.view(Bb, nC, c, H, P)
     else:
@@ -164,6 +233,12 @@ def ssd_scan(x, dt, A, B, C, D=None, seq_idx: Optional[torch.Tensor] = None, chu
         wl = wl * last_same.unsqueeze(2)
         carry = carry * first.unsqueeze(2)
     keep = carry[..., -1]                                                                # (B,nC,H)
+    if fused:
+        BN = Bb * nC
+        y = _ChunkScanFn.apply(x, dt.view(Bb, nC, c, H), cs, Bh.reshape(BN, c, N), Ch.reshape(BN, c, N), wl.permute(0, 1, 3, 2),
+                               carry.permute(0, 1, 3, 2), keep, None if D is None else D.float().contiguous(),
+                               bc.to(torch.int32).contiguous() if brk is not None else None)
+        return y.reshape(Bb, Lp, H, P)[:, :L]
     if G == 1:
         # one group: inside a chunk the token-major layout (c, H·P) is already what a batched matmul over the chunks wants,
         # so both products run without operand permutes or per-head copies of B / C
