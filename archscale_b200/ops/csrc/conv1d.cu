@@ -2,7 +2,9 @@
 //   y[b,t,c] = act( bias[c] + Σ_j w[c,j] · x[b, t-(W-1)+j, c] ),  taps that cross a document boundary
 //   (seq_idx[b,t'] != seq_idx[b,t]) or the start of the sequence read 0.
 // A thread owns 8 consecutive channels and walks TSTEP time steps with the window in registers, so every
-// x element is loaded once (plus a W-1 halo) with 16-byte accesses.
+// x element is loaded once (plus a W-1 halo) with 16-byte accesses.  The walk is memory latency unless several steps' loads
+// are in flight: both kernels load the next group of steps (raw, as it lies in memory) before they work on the current one.
+// bf16, C 3968, B4 L4096: forward 0.138 -> 0.120 ms, backward 0.309 -> 0.223 ms; B3 L2731 C1536: 0.046 -> 0.035, 0.145 -> 0.093.
 // Backward recomputes the pre-activation, forms g = dy·act'(pre) and accumulates
 //   dx[t'] += w[c,j]·g[t] (t' = t-(W-1)+j),  dw[c,j] += g[t]·x[t'],  db[c] += g[t]
 // dx is produced gather-style (deterministic); dw/db use fp32 atomics on C·(W+1) addresses.
@@ -35,6 +37,25 @@ template <> struct V8<__nv_bfloat16> {
     uint4 u;
     u.x = pack_bf16x2(v[0], v[1]); u.y = pack_bf16x2(v[2], v[3]); u.z = pack_bf16x2(v[4], v[5]); u.w = pack_bf16x2(v[6], v[7]);
     *reinterpret_cast<uint4*>(p) = u;
+  }
+};
+
+// eight elements as they lie in memory
+template <typename T> struct Raw8;
+template <> struct Raw8<float> {
+  float4 a, b;
+  __device__ __forceinline__ void ld(const float* p) { a = reinterpret_cast<const float4*>(p)[0]; b = reinterpret_cast<const float4*>(p)[1]; }
+  __device__ __forceinline__ void get(float (&v)[8]) const {
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w; v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+  }
+};
+template <> struct Raw8<__nv_bfloat16> {
+  uint4 u;
+  __device__ __forceinline__ void ld(const __nv_bfloat16* p) { u = *reinterpret_cast<const uint4*>(p); }
+  __device__ __forceinline__ void get(float (&v)[8]) const {
+    const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+    for (int i = 0; i < 4; ++i) { const float2 f = unpack_bf16x2(w[i]); v[2 * i] = f.x; v[2 * i + 1] = f.y; }
   }
 };
 
@@ -73,8 +94,27 @@ __global__ void __launch_bounds__(128) conv1d_fwd_kernel(const T* __restrict__ x
   int sid_hist[W];
 #pragma unroll
   for (int j = 0; j < W - 1; ++j) { const int tt = t0 - (W - 1) + j; sid_hist[j] = (sb && tt >= 0) ? sb[tt] : -1; }
-  for (int t = t0; t < min(t0 + CV_TSTEP, L); ++t) {
-    V8<T>::ld(xb + static_cast<size_t>(t) * xs, win[W - 1]);
+  constexpr int U = 4;                                        // steps per group
+  const int t_end = min(t0 + CV_TSTEP, L);
+  Raw8<T> nx[U];
+#pragma unroll
+  for (int u = 0; u < U; ++u)
+    if (t0 + u < t_end) nx[u].ld(xb + static_cast<size_t>(t0 + u) * xs);
+#pragma unroll 1
+  for (int g = 0; g < CV_TSTEP / U; ++g) {
+    Raw8<T> cx[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) cx[u] = nx[u];
+    if (g + 1 < CV_TSTEP / U) {
+#pragma unroll
+      for (int u = 0; u < U; ++u)
+        if (t0 + (g + 1) * U + u < t_end) nx[u].ld(xb + static_cast<size_t>(t0 + (g + 1) * U + u) * xs);
+    }
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int t = t0 + g * U + u;
+    if (t >= t_end) return;
+    cx[u].get(win[W - 1]);
     const int sid = sb ? sb[t] : 0;
     sid_hist[W - 1] = sid;
     float acc[8];
@@ -99,6 +139,7 @@ __global__ void __launch_bounds__(128) conv1d_fwd_kernel(const T* __restrict__ x
 #pragma unroll
       for (int e = 0; e < 8; ++e) win[j][e] = win[j + 1][e];
     }
+  }
   }
 }
 
@@ -144,7 +185,27 @@ __global__ void __launch_bounds__(128) conv1d_bwd_kernel(const T* __restrict__ d
 #pragma unroll
     for (int e = 0; e < 8; ++e) gw[k][e] = 0.f;
   }
-  for (int t = t0; t < t_end + W - 1; ++t) {
+  constexpr int U = sizeof(T) == 2 ? 4 : 2;
+  Raw8<T> nx[U], nd[U];
+  auto fetch = [&](int t) {
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+      if (t + u < L && t + u < t_end + W - 1) {
+        nx[u].ld(x + (static_cast<size_t>(b) * L + t + u) * xs + c0);
+        nd[u].ld(dy + (static_cast<size_t>(b) * L + t + u) * dys + c0);
+      }
+  };
+  fetch(t0);
+#pragma unroll 1
+  for (int tg = t0; tg < t_end + W - 1; tg += U) {
+    Raw8<T> cx[U], cd[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u) { cx[u] = nx[u]; cd[u] = nd[u]; }
+    fetch(tg + U);
+#pragma unroll
+  for (int u = 0; u < U; ++u) {
+    const int t = tg + u;
+    if (t >= t_end + W - 1) break;
     // shift the windows by one step
 #pragma unroll
     for (int k = 0; k < W - 1; ++k) {
@@ -154,7 +215,7 @@ __global__ void __launch_bounds__(128) conv1d_bwd_kernel(const T* __restrict__ d
     }
     if (t < L) {
       sw[W - 1] = sb ? sb[t] : 0;
-      V8<T>::ld(x + (static_cast<size_t>(b) * L + t) * xs + c0, xw[W - 1]);
+      cx[u].get(xw[W - 1]);
       float pre[8], g[8];
 #pragma unroll
       for (int e = 0; e < 8; ++e) pre[e] = bs[e];
@@ -165,7 +226,7 @@ __global__ void __launch_bounds__(128) conv1d_bwd_kernel(const T* __restrict__ d
           for (int e = 0; e < 8; ++e) pre[e] += wk[k][e] * xw[k][e];
         }
       }
-      V8<T>::ld(dy + (static_cast<size_t>(b) * L + t) * dys + c0, g);
+      cd[u].get(g);
       if (silu) {
 #pragma unroll
         for (int e = 0; e < 8; ++e) g[e] *= dsilu_f(pre[e]);
@@ -203,6 +264,7 @@ __global__ void __launch_bounds__(128) conv1d_bwd_kernel(const T* __restrict__ d
       }
       V8<T>::st(dx + base + static_cast<size_t>(tp) * C, dxa);
     }
+  }
   }
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
