@@ -1,8 +1,13 @@
 // Gated RMSNorm with groups (Mamba-2, Gated DeltaNet, GMU with a norm):
 //   norm_before_gate:   y = (x · rstd_g · w) · silu(z)          rstd_g over the group's columns of x
 //   otherwise:          y = (x·silu(z)) · rstd_g · w            rstd_g over the group's columns of x·silu(z)
-// Forward: one warp per (row, group).  Backward: a CTA works on one group (its 8 warps stride the rows), so the weight
-// gradient of the group's columns is accumulated in shared memory and flushed with one atomic per column per CTA.
+// Groups of up to 4096 columns: a team of W = 1, 2, 4 or 8 warps (512 columns per warp) takes a (row, group), a lane owns the
+// same 16 columns of every row, keeps the row's values in registers between the sum and the outputs (one read of each
+// operand) and accumulates the weight gradient of its columns in registers.  The team's partial sums meet in shared memory
+// behind a named barrier.  Before, one warp looped over the whole row twice and the backward added every element to shared
+// memory with an atomic.  bf16, ms: 16384 x 3968 forward 0.144 -> 0.079, backward 0.353 -> 0.195 (the bytes take 0.06 and 0.10);
+// 8193 x 3072 in groups of 512 0.043 -> 0.034, 0.155 -> 0.115; 16384 x 1024 in groups of 128 0.055 -> 0.043, 0.133 -> 0.093.
+// Wider groups: the loops remain (one warp per (row, group); weight gradient in shared memory).
 #include "sm100.cuh"
 #include "api.h"
 
@@ -37,6 +42,152 @@ __device__ __forceinline__ float gn_wsum(float v) {
 __device__ __forceinline__ float gn_silu(float x) { return x / (1.f + __expf(-x)); }
 __device__ __forceinline__ float gn_dsilu(float x) { const float s = 1.f / (1.f + __expf(-x)); return s * (1.f + x * (1.f - s)); }
 
+// ---- teams of warps
+template <int W>
+__device__ __forceinline__ float gn_team_sum(float v, float* slots /* [8], this pass's buffer */, int warp, int lane) {
+  v = gn_wsum(v);
+  if (W == 1) return v;
+  if (lane == 0) slots[warp] = v;
+  asm volatile("bar.sync %0, %1;" ::"r"(1 + warp / W), "n"(W * 32) : "memory");
+  float t = 0.f;
+#pragma unroll
+  for (int k = 0; k < W; ++k) t += slots[warp / W * W + k];
+  return t;
+}
+
+template <typename T, int W>
+__global__ void __launch_bounds__(256) gated_rmsnorm_fwd_team_kernel(const T* __restrict__ x, const T* __restrict__ z, const float* __restrict__ w,
+                                                                     T* __restrict__ y, float* __restrict__ rstd, long long rows, int cols,
+                                                                     int gsize, float eps, int nbg) {
+  __shared__ float slots[8];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int ngroups = cols / gsize;
+  const long long unit = blockIdx.x * static_cast<long long>(8 / W) + warp / W;     // (row, group), the same for a team
+  if (unit >= rows * ngroups) return;
+  const long long row = unit / ngroups;
+  const int g0 = static_cast<int>(unit - row * ngroups) * gsize;
+  const size_t base = static_cast<size_t>(row) * cols + g0;
+  float v[2][8];
+  float ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int c = (warp % W * 32 + lane) * 8 + k * W * 256;
+    if (c < gsize) {
+      float xv[8], zv[8];
+      gn_ld8(x + base + c, xv);
+      if (z) gn_ld8(z + base + c, zv);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) {
+        const float s = z ? gn_silu(zv[i]) : 1.f;
+        v[k][i] = xv[i] * s;
+        const float xin = nbg ? xv[i] : v[k][i];
+        ss += xin * xin;
+      }
+    }
+  }
+  const float rs = rsqrtf(gn_team_sum<W>(ss, slots, warp, lane) / gsize + eps);
+  if (warp % W == 0 && lane == 0) rstd[unit] = rs;
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int c = (warp % W * 32 + lane) * 8 + k * W * 256;
+    if (c < gsize) {
+      float wv[8];
+      gn_ld8(w + g0 + c, wv);
+#pragma unroll
+      for (int i = 0; i < 8; ++i) v[k][i] = v[k][i] * rs * wv[i];   // same product either way; only what rstd was measured on differs
+      gn_st8(y + base + c, v[k]);
+    }
+  }
+}
+
+template <typename T, int W>
+__global__ void __launch_bounds__(256, 2) gated_rmsnorm_bwd_team_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ z,
+                                                                        const float* __restrict__ w, const float* __restrict__ rstd,
+                                                                        T* __restrict__ dx, T* __restrict__ dz, float* __restrict__ dw,
+                                                                        long long rows, int cols, int gsize, int nbg) {
+  extern __shared__ float gn_dw[];                 // [gsize]
+  __shared__ float slots[2][8];                    // alternate from row to row: one barrier per row suffices
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+  const int ngroups = cols / gsize;
+  const int grp = blockIdx.x % ngroups, g0 = grp * gsize;
+  const int ctas_per_group = gridDim.x / ngroups, cta_in_group = blockIdx.x / ngroups;
+  constexpr int TEAMS = 8 / W;
+  for (int c = threadIdx.x; c < gsize; c += blockDim.x) gn_dw[c] = 0.f;
+  float wr[2][8], dwa[2][8];
+#pragma unroll
+  for (int k = 0; k < 2; ++k) {
+    const int c = (warp % W * 32 + lane) * 8 + k * W * 256;
+#pragma unroll
+    for (int i = 0; i < 8; ++i) wr[k][i] = dwa[k][i] = 0.f;
+    if (c < gsize) gn_ld8(w + g0 + c, wr[k]);
+  }
+  int it = 0;
+  for (long long row = static_cast<long long>(cta_in_group) * TEAMS + warp / W; row < rows; row += static_cast<long long>(ctas_per_group) * TEAMS, ++it) {
+    const size_t base = static_cast<size_t>(row) * cols + g0;
+    const float rs = rstd[row * ngroups + grp];
+    float xv[2][8], dv[2][8], zv[2][8], sg[2][8];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int c = (warp % W * 32 + lane) * 8 + k * W * 256;
+      if (c < gsize) {
+        gn_ld8(x + base + c, xv[k]);
+        gn_ld8(dy + base + c, dv[k]);
+        if (z) gn_ld8(z + base + c, zv[k]);
+      }
+    }
+    float dot = 0.f;                               // Σ gw · xin  (xin = what was normalised)
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int c = (warp % W * 32 + lane) * 8 + k * W * 256;
+      if (c < gsize) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          sg[k][i] = z ? 1.f / (1.f + __expf(-zv[k][i])) : 1.f;
+          const float s = z ? zv[k][i] * sg[k][i] : 1.f;
+          dot += dv[k][i] * s * wr[k][i] * xv[k][i];   // either order of norm and gate: dy·silu(z)·w·x
+        }
+      }
+    }
+    const float c1 = gn_team_sum<W>(dot, slots[it & 1], warp, lane) * rs * rs * rs / gsize;
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int c = (warp % W * 32 + lane) * 8 + k * W * 256;
+      if (c < gsize) {
+        float ox[8], oz[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float s = z ? zv[k][i] * sg[k][i] : 1.f;
+          const float ds = z ? sg[k][i] * (1.f + zv[k][i] * (1.f - sg[k][i])) : 0.f;
+          const float xin = nbg ? xv[k][i] : xv[k][i] * s;
+          const float g = nbg ? dv[k][i] * s : dv[k][i];
+          const float dxin = g * wr[k][i] * rs - xin * c1;
+          dwa[k][i] += g * xin * rs;
+          if (nbg) { ox[i] = dxin; oz[i] = dv[k][i] * (xv[k][i] * rs * wr[k][i]) * ds; }
+          else { ox[i] = dxin * s; oz[i] = dxin * xv[k][i] * ds; }
+        }
+        gn_st8(dx + base + c, ox);
+        if (dz) gn_st8(dz + base + c, oz);
+      }
+    }
+  }
+  __syncthreads();
+  for (int turn = 0; turn < TEAMS; ++turn) {       // the teams add their sums in turn
+    if (warp / W == turn) {
+#pragma unroll
+      for (int k = 0; k < 2; ++k) {
+        const int c = (warp % W * 32 + lane) * 8 + k * W * 256;
+        if (c < gsize) {
+#pragma unroll
+          for (int i = 0; i < 8; ++i) gn_dw[c + i] += dwa[k][i];
+        }
+      }
+    }
+    __syncthreads();
+  }
+  for (int c = threadIdx.x; c < gsize; c += blockDim.x) atomicAdd(&dw[g0 + c], gn_dw[c]);
+}
+
+// ---- groups wider than 4096 columns
 template <typename T>
 __global__ void __launch_bounds__(256) gated_rmsnorm_fwd_kernel(const T* __restrict__ x, const T* __restrict__ z, const float* __restrict__ w,
                                                                 T* __restrict__ y, float* __restrict__ rstd, long long rows, int cols,
@@ -144,6 +295,16 @@ extern "C" int b200_gated_rmsnorm_fwd(const void* x, const void* z, const float*
   if (rows == 0) return 0;
   if (gsize % 8 || cols % gsize) return -1;
   const long long units = rows * (cols / gsize);
+  if (gsize <= 4096) {
+    const int W = gsize <= 512 ? 1 : gsize <= 1024 ? 2 : gsize <= 2048 ? 4 : 8;
+    const unsigned tg = static_cast<unsigned>((units * W + 7) / 8);
+#define GN_FWD(T, WW) gated_rmsnorm_fwd_team_kernel<T, WW><<<tg, 256, 0, st>>>((const T*)x, (const T*)z, w, (T*)y, rstd, rows, cols, gsize, eps, norm_before_gate)
+#define GN_FWD_W(T) do { if (W == 1) GN_FWD(T, 1); else if (W == 2) GN_FWD(T, 2); else if (W == 4) GN_FWD(T, 4); else GN_FWD(T, 8); } while (0)
+    if (dtype == 1) GN_FWD_W(__nv_bfloat16); else GN_FWD_W(float);
+#undef GN_FWD_W
+#undef GN_FWD
+    return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  }
   const unsigned grid = static_cast<unsigned>((units + 7) / 8);
   if (dtype == 1) gated_rmsnorm_fwd_kernel<__nv_bfloat16><<<grid, 256, 0, st>>>((const __nv_bfloat16*)x, (const __nv_bfloat16*)z, w, (__nv_bfloat16*)y, rstd, rows, cols, gsize, eps, norm_before_gate);
   else gated_rmsnorm_fwd_kernel<float><<<grid, 256, 0, st>>>((const float*)x, (const float*)z, w, (float*)y, rstd, rows, cols, gsize, eps, norm_before_gate);
@@ -156,6 +317,21 @@ extern "C" int b200_gated_rmsnorm_bwd(const void* dy, const void* x, const void*
   if (rows == 0) return 0;
   if (gsize % 8 || cols % gsize || gsize > 12288) return -1;
   const int ngroups = cols / gsize;
+  if (gsize <= 4096) {
+    const int W = gsize <= 512 ? 1 : gsize <= 1024 ? 2 : gsize <= 2048 ? 4 : 8, teams = 8 / W;
+    int per = (148 * 2 + ngroups - 1) / ngroups;     // two CTAs per SM
+    const long long need = (rows + teams - 1) / teams;
+    if (per > need) per = static_cast<int>(need);
+    const unsigned grid = static_cast<unsigned>(per * ngroups);
+#define GN_BWD(T, WW)                                                                                                       \
+  gated_rmsnorm_bwd_team_kernel<T, WW><<<grid, 256, sizeof(float) * gsize, st>>>((const T*)dy, (const T*)x, (const T*)z, w, rstd, \
+                                                                                 (T*)dx, (T*)dz, dw, rows, cols, gsize, norm_before_gate)
+#define GN_BWD_W(T) do { if (W == 1) GN_BWD(T, 1); else if (W == 2) GN_BWD(T, 2); else if (W == 4) GN_BWD(T, 4); else GN_BWD(T, 8); } while (0)
+    if (dtype == 1) GN_BWD_W(__nv_bfloat16); else GN_BWD_W(float);
+#undef GN_BWD_W
+#undef GN_BWD
+    return cudaGetLastError() == cudaSuccess ? 0 : -3;
+  }
   int per = (148 * 4 + ngroups - 1) / ngroups;
   const long long need = (rows + 7) / 8;
   if (per > need) per = static_cast<int>(need);
