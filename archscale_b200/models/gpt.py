@@ -363,6 +363,20 @@ class Block(nn.Module):
         return x, new_kv_cache, gmu_mems, input_embed
 
 
+def document_offsets(is_eos: torch.Tensor) -> torch.Tensor:
+    """``[0, document ends …, T, T, …]`` (int32, T + 1 entries) of a packed row whose documents end at the marked tokens.  The
+    length does not depend on the data, so the host does not wait for the tokens; the consumers (attention row tables, scan
+    resets, document ids) take the repeated ends as empty documents."""
+    T = is_eos.numel()
+    inner = is_eos.clone()
+    inner[-1:] = False                                               # an EOS at the last token ends no earlier document
+    ends = torch.arange(1, T + 1, device=is_eos.device).masked_fill_(~inner, T)
+    slot = torch.cumsum(inner, 0).masked_fill_(~inner, T)            # entry of each end; everything else writes T into the last one
+    cu = torch.full((T + 1,), T, dtype=torch.int32, device=is_eos.device)
+    cu[:1] = 0
+    return cu.scatter_(0, slot, ends.to(torch.int32))
+
+
 class GPT(nn.Module):
     def __init__(self, config: Config) -> None:
         super().__init__()
@@ -458,9 +472,12 @@ class GPT(nn.Module):
             assert idx.size(0) == 1, "packed variable-length training uses batch size 1"
             is_eos = idx.flatten() == cfg.eos_token_id
             T = idx.shape[1]
-            ends = is_eos.nonzero().flatten() + 1
-            ends = ends[ends < T]
-            cu = torch.cat([ends.new_zeros(1), ends, ends.new_full((1,), T)]).to(torch.int32)
+            if idx.is_cuda and cfg.rnn_type != "gdn":
+                cu = document_offsets(is_eos)                    # no host wait; the delta rule walks the list on the host
+            else:
+                ends = is_eos.nonzero().flatten() + 1
+                ends = ends[ends < T]
+                cu = torch.cat([ends.new_zeros(1), ends, ends.new_full((1,), T)]).to(torch.int32)
             # document id of each token: number of EOS strictly before it
             seq_idx = (torch.cumsum(is_eos.to(torch.int32), 0) - is_eos.to(torch.int32)).unsqueeze(0).to(torch.int32)
             return {"cu_seqlens": cu, "seq_idx": seq_idx}

@@ -130,9 +130,10 @@ def _scan_chunked_torch(u, delta, A, B, C, D, z, delta_bias, delta_softplus, cu_
     N = A.shape[1]
     Af = A.float()
     Bf, Cf = B.float(), C.float()
-    reset = torch.zeros(L, dtype=torch.bool, device=u.device)
+    reset = torch.zeros(L + 1, dtype=torch.bool, device=u.device)
     if cu_seqlens is not None:
-        reset[cu_seqlens[:-1].long()] = True
+        reset[cu_seqlens[:-1].long()] = True                        # a repeated end (empty document) lands on position L
+    reset = reset[:L]
     T = 64
     h = uf.new_zeros(Bb, Di, N)
     outs = []

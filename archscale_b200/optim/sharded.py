@@ -292,7 +292,7 @@ class ShardedOptimizer:
                 if self.use_muonh:
                     if not xsq_cached:
                         sq = torch.stack(torch._foreach_norm(xs)).square()
-                        x_sq.index_add_(0, torch.tensor(ks, device=dev), sq)
+                        x_sq.index_add_(0, self._hyper_index(tuple(ks), dev), sq)
                     hb_x += xs
                     hb_u += os_
                     hb_k += ks
@@ -331,8 +331,14 @@ class ShardedOptimizer:
             ratio = x_norm / u_norm
             new_sq = torch.zeros_like(x_sq)
             if hb_x:
-                kidx = torch.tensor(hb_k, device=dev)
-                coef = ratio[kidx] * torch.tensor(hb_lr, device=dev, dtype=torch.float32)
+                # nothing here may copy from pageable host memory: that waits for all queued work, and the next step's
+                # launches then start on an idle GPU
+                kidx = self._hyper_index(tuple(hb_k), dev)
+                if all(l == hb_lr[0] for l in hb_lr):
+                    coef = ratio[kidx] * hb_lr[0]
+                else:
+                    lr_t = torch.tensor(hb_lr, dtype=torch.float32)
+                    coef = ratio[kidx] * (lr_t.pin_memory().to(dev, non_blocking=True) if eng.is_cuda else lr_t)
                 upd = [u.to(x.dtype) if u.dtype != x.dtype else u for u, x in zip(hb_u, hb_x)]
                 upd = torch._foreach_mul(upd, list(coef.unbind(0)))
                 torch._foreach_sub_(hb_x, upd)
@@ -385,6 +391,13 @@ class ShardedOptimizer:
                       "kidx": torch.tensor([s[2] for s in segs], dtype=torch.int32, device=dev)}
         cache[id(g)] = tb
         return tb
+
+    def _hyper_index(self, slots: Tuple[int, ...], dev) -> torch.Tensor:
+        """Norm slots as a device index (they depend on which parameters have gradients, so a few sets at most)."""
+        cache = self.__dict__.setdefault("_hyper_idx_cache", {})
+        if slots not in cache:
+            cache[slots] = torch.tensor(slots, dtype=torch.long, device=dev)
+        return cache[slots]
 
     def _mat_norm_idx(self, dev) -> torch.Tensor:
         if getattr(self, "_mat_idx_t", None) is None:
