@@ -92,9 +92,16 @@ __global__ void __launch_bounds__(OPT_THREADS) adamw_fused_kernel(float* __restr
   }
 }
 
-// MODE 0: acc += x²; MODE 1: x -= coef·u (u bf16), acc += x²; MODE 2: x *= coef
-template <int MODE>
-__global__ void __launch_bounds__(OPT_THREADS) seg_kernel(float* __restrict__ x, const __nv_bfloat16* __restrict__ u, long long n4,
+__device__ __forceinline__ float4 seg_load4(const float* u, long long i4) { return reinterpret_cast<const float4*>(u)[i4]; }
+__device__ __forceinline__ float4 seg_load4(const __nv_bfloat16* u, long long i4) {
+  const uint2 uv = reinterpret_cast<const uint2*>(u)[i4];
+  const float2 a = unpack_bf16x2(uv.x), b = unpack_bf16x2(uv.y);
+  return make_float4(a.x, a.y, b.x, b.y);
+}
+
+// MODE 0: acc += x²; MODE 1: x -= coef·u (u bf16 or fp32), acc += x²; MODE 2: x *= coef
+template <int MODE, typename TU = __nv_bfloat16>
+__global__ void __launch_bounds__(OPT_THREADS) seg_kernel(float* __restrict__ x, const TU* __restrict__ u, long long n4,
                                                          const long long* __restrict__ bounds, const int* __restrict__ kidx,
                                                          int nseg, const float* __restrict__ coef, float* __restrict__ acc) {
   __shared__ float s_part[OPT_MAX_SEG_PER_BLOCK];
@@ -114,9 +121,8 @@ __global__ void __launch_bounds__(OPT_THREADS) seg_kernel(float* __restrict__ x,
       float4 xv = reinterpret_cast<float4*>(x)[i4];
       if (MODE == 1) {
         const float c = coef[kidx[seg]];
-        const uint2 uv = reinterpret_cast<const uint2*>(u)[i4];
-        const float2 a = unpack_bf16x2(uv.x), b = unpack_bf16x2(uv.y);
-        xv.x -= c * a.x; xv.y -= c * a.y; xv.z -= c * b.x; xv.w -= c * b.y;
+        const float4 uv = seg_load4(u, i4);
+        xv.x -= c * uv.x; xv.y -= c * uv.y; xv.z -= c * uv.z; xv.w -= c * uv.w;
         reinterpret_cast<float4*>(x)[i4] = xv;
       } else if (MODE == 2) {
         const float c = coef[kidx[seg]];
@@ -168,8 +174,8 @@ extern "C" int b200_muon_momentum(const float* g, float* m, void* u, long long n
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
-// mode 0 / 1 / 2 as described at the top; bounds: int64 [nseg + 1] on the device, bounds[0] = 0 … bounds[nseg] ≥ n
-extern "C" int b200_seg_update(int mode, float* x, const void* u, long long n, const long long* bounds, const int* kidx, int nseg,
+// mode 0 / 1 / 2 as described at the top; u_dtype 0 fp32 / 1 bf16; bounds: int64 [nseg + 1] on the device, bounds[0] = 0 … bounds[nseg] ≥ n
+extern "C" int b200_seg_update(int mode, float* x, const void* u, int u_dtype, long long n, const long long* bounds, const int* kidx, int nseg,
                                const float* coef, float* acc, cudaStream_t st) {
   if (n % 4 || nseg <= 0) return -1;
   if (n == 0) return 0;
@@ -177,6 +183,8 @@ extern "C" int b200_seg_update(int mode, float* x, const void* u, long long n, c
   const unsigned grid = static_cast<unsigned>((n4 + OPT_THREADS * OPT_VEC_PER_THREAD - 1) / (OPT_THREADS * OPT_VEC_PER_THREAD));
   const __nv_bfloat16* up = static_cast<const __nv_bfloat16*>(u);
   if (mode == 0) seg_kernel<0><<<grid, OPT_THREADS, 0, st>>>(x, up, n4, bounds, kidx, nseg, coef, acc);
+  else if (mode == 1 && u_dtype == 0)
+    seg_kernel<1, float><<<grid, OPT_THREADS, 0, st>>>(x, static_cast<const float*>(u), n4, bounds, kidx, nseg, coef, acc);
   else if (mode == 1) seg_kernel<1><<<grid, OPT_THREADS, 0, st>>>(x, up, n4, bounds, kidx, nseg, coef, acc);
   else if (mode == 2) seg_kernel<2><<<grid, OPT_THREADS, 0, st>>>(x, up, n4, bounds, kidx, nseg, coef, acc);
   else return -1;

@@ -252,6 +252,11 @@ class ShardedOptimizer:
             self.nadam_mu_product *= scalar_opts.nadam_mu(self.betas[0], self.step_count)
 
         # ---- matrices: momentum on local slices, orthogonalise on owners, scatter back
+        # Adam directions of embeddings and heads: one segment each on the segment kernels (two passes over the master instead of
+        # the four of the foreach form, whose per-tensor device factors also take PyTorch's unvectorised broadcast kernels)
+        hyper_seg = [t for t in pending_hyper if self._hyper_seg_ok(t[0], t[1])]
+        if hyper_seg:
+            pending_hyper = [t for t in pending_hyper if not self._hyper_seg_ok(t[0], t[1])]
         hb_x: List[torch.Tensor] = [t[0] for t in pending_hyper]
         hb_u: List[torch.Tensor] = [t[1] for t in pending_hyper]
         hb_k: List[int] = [t[2] for t in pending_hyper]
@@ -313,7 +318,7 @@ class ShardedOptimizer:
                 ops.backend.count_launch(len(seg_groups))
 
         # ---- hyperball: global norms (2 all-reduces for the whole model), update, renormalise
-        if hb_x or seg_groups:
+        if hb_x or seg_groups or hyper_seg:
             if eng.mesh.fsdp > 1:
                 packed = torch.stack((x_sq, u_sq))
                 keep = packed[:, self.local_norm_idx].clone() if self.local_norm_idx is not None else None
@@ -343,6 +348,12 @@ class ShardedOptimizer:
                 upd = torch._foreach_mul(upd, list(coef.unbind(0)))
                 torch._foreach_sub_(hb_x, upd)
                 new_sq.index_add_(0, kidx, torch.stack(torch._foreach_norm(hb_x)).square())
+            if hyper_seg:
+                ext = ops.backend.require_extension()
+                coef_h = {l: ratio * l for l in {t[3] for t in hyper_seg}}
+                for x, u, k, l in hyper_seg:
+                    ext.seg_update_(1, x, u, *self._hyper_bounds(x.numel(), k), coef_h[l], new_sq)
+                ops.backend.count_launch(len(hyper_seg))
             if seg_groups:
                 ext = ops.backend.require_extension()
                 coef_m = (ratio * lr_m).contiguous()
@@ -357,6 +368,9 @@ class ShardedOptimizer:
             scale_v = (x_norm / new_sq.sqrt().clamp_min(self.ns_epsilon)).contiguous()
             if hb_x:
                 torch._foreach_mul_(hb_x, list(scale_v[kidx].unbind(0)))
+            for x, _, k, _ in hyper_seg:
+                ext.seg_update_(2, x, None, *self._hyper_bounds(x.numel(), k), scale_v, None)
+                ops.backend.count_launch()
             if seg_groups:
                 for x, _, tb in seg_groups:
                     ext.seg_update_(2, x, None, tb["bounds"], tb["kidx"], scale_v, None)
@@ -391,6 +405,19 @@ class ShardedOptimizer:
                       "kidx": torch.tensor([s[2] for s in segs], dtype=torch.int32, device=dev)}
         cache[id(g)] = tb
         return tb
+
+    def _hyper_seg_ok(self, x: torch.Tensor, u: torch.Tensor) -> bool:
+        return (self.engine.is_cuda and ops.backend.has("seg_update_") and x.dtype == torch.float32 and u.dtype == torch.float32
+                and x.is_contiguous() and u.is_contiguous() and x.numel() % 4 == 0 and x.numel() > 0
+                and x.data_ptr() % 16 == 0 and u.data_ptr() % 16 == 0)
+
+    def _hyper_bounds(self, n: int, slot: int) -> Tuple[torch.Tensor, torch.Tensor]:
+        """One-segment tables (element bounds, norm slot) on the device."""
+        cache = self.__dict__.setdefault("_hyper_bounds_cache", {})
+        if (n, slot) not in cache:
+            dev = self.engine.device
+            cache[(n, slot)] = (torch.tensor([0, n], dtype=torch.int64, device=dev), torch.tensor([slot], dtype=torch.int32, device=dev))
+        return cache[(n, slot)]
 
     def _hyper_index(self, slots: Tuple[int, ...], dev) -> torch.Tensor:
         """Norm slots as a device index (they depend on which parameters have gradients, so a few sets at most)."""
