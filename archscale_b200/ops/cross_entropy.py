@@ -77,11 +77,12 @@ def _ce_chunk_fwd_bwd(logits: torch.Tensor, target: torch.Tensor, ignore_index: 
 
 class _FLCEFn(torch.autograd.Function):
     @staticmethod
-    def forward(ctx, x, weight, target, ignore_index, label_smoothing, lse_square_scale, chunk_rows):
+    def forward(ctx, x, weight, target, ignore_index, label_smoothing, lse_square_scale, chunk_rows, grad_mode):
         N, H = x.shape
         V = weight.shape[0]
-        need_dx = x.requires_grad
-        need_dw = weight.requires_grad
+        # grad_mode: the caller's; in here it is always off, and a parameter requires gradients under no_grad too
+        need_dx = grad_mode and x.requires_grad
+        need_dw = grad_mode and weight.requires_grad
         dx = torch.empty_like(x) if need_dx else None
         dw = torch.zeros(V, H, device=x.device, dtype=torch.float32) if need_dw else None
         total = torch.zeros((), device=x.device, dtype=torch.float32)
@@ -109,7 +110,7 @@ class _FLCEFn(torch.autograd.Function):
         s = gout * inv
         gx = (dx * s.to(dx.dtype)) if dx is not None else None
         gw = (dw * s).to(ctx.wdtype) if dw is not None else None
-        return gx, gw, None, None, None, None, None
+        return gx, gw, None, None, None, None, None, None
 
 
 def default_chunk_rows(N: int, H: int, V: int, on_gpu: bool = False) -> int:
@@ -141,7 +142,7 @@ def fused_linear_cross_entropy(x: torch.Tensor, weight: torch.Tensor, target: to
     t = target.reshape(-1)
     if chunk_rows is None:
         chunk_rows = default_chunk_rows(x2.shape[0], x2.shape[1], weight.shape[0], on_gpu=x2.is_cuda)
-    return _FLCEFn.apply(x2, weight, t, ignore_index, label_smoothing, lse_square_scale, chunk_rows)
+    return _FLCEFn.apply(x2, weight, t, ignore_index, label_smoothing, lse_square_scale, chunk_rows, torch.is_grad_enabled())
 
 
 def fused_linear_cross_entropy_ref(x, weight, target, ignore_index: int = -100, label_smoothing: float = 0.0,

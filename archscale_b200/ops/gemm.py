@@ -127,12 +127,12 @@ class _LinearFn(torch.autograd.Function):
 
 class _LinearSwiGLUFn(torch.autograd.Function):
     """``silu(x·W_gateᵀ) ∘ (x·W_upᵀ)`` with the activation computed in the GEMM epilogue (``W = [gate rows | up rows]``).
-    The pre-activation is still written (the backward needs it) but not read back in the forward pass."""
+    The pre-activation is written only when a backward pass will read it; the forward pass never reads it back."""
 
     @staticmethod
-    def forward(ctx, x, weight):
+    def forward(ctx, x, weight, keep_h):
         x2 = x.reshape(-1, x.shape[-1])
-        h, act = backend.require_extension().gemm_swiglu(x2, weight, True)
+        h, act = backend.require_extension().gemm_swiglu(x2, weight, keep_h)
         backend.count_launch()
         ctx.save_for_backward(x, weight, h)
         ctx.weight_ref = weight
@@ -156,7 +156,7 @@ class _LinearSwiGLUFn(torch.autograd.Function):
                 matmul_tn_acc_(main_grad, dh, x2)
             else:
                 dw = matmul_tn(dh, x2)
-        return dx, dw
+        return dx, dw, None
 
 
 def fused_swiglu_enabled() -> bool:
@@ -179,7 +179,7 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor) -> Optional[torch.Tenso
         return None                                     # this GEMM carries the unit's fused all-gather: keep that path
     if not x.is_contiguous():
         x = x.contiguous()
-    return _LinearSwiGLUFn.apply(x, weight)
+    return _LinearSwiGLUFn.apply(x, weight, torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad))
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
