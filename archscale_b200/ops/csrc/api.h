@@ -152,7 +152,10 @@ int b200_conv1d_bwd(const void* dy, const void* x, int dtype, const float* w, co
 int b200_selective_scan_ckpt_segments(int L);
 int b200_selective_scan_fwd(const void* u, int su, const void* delta, int sd, const float* A, const void* Bm, int sB,
                             const void* Cm, int sC, const float* D, const void* z, int sz, const float* dbias, const int* reset,
-                            void* y, float* ckpt, int dtype, int B, int L, int Di, int softplus, cudaStream_t st);
+                            void* y, float* ckpt, int dtype, int B, int L, int Di, int softplus, int parts, float* scratch,
+                            cudaStream_t st);
+int b200_selective_scan_parts(int B, int L, int Di);                      // parts of the time axis the forward runs side by side
+long long b200_selective_scan_scratch(int B, int Di, int parts);          // floats of scratch for them
 int b200_selective_scan_bwd(const void* dy, int sdy, const void* u, int su, const void* delta, int sd, const float* A,
                             const void* Bm, int sB, const void* Cm, int sC, const float* D, const void* z, int sz,
                             const float* dbias, const int* reset, const float* ckpt, void* du, void* ddelta, void* dz, float* dA,

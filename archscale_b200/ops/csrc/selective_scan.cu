@@ -8,8 +8,9 @@
 // shared-memory loads, fifteen sixteenths of a shuffle and its selects per state.  Several states per thread share the loads of dt and dt·u, read B and C as vectors, do two states per instruction
 // (fma.rn.f32x2) and add most of the sum over states in registers; the remaining 16/NS lanes use a reduce-scatter over 16/NS
 // steps (lane q ends up with the total of step q).  Measured, one state -> several states per thread, ms:
-//   B4 L4096 Di3968   forward 1.17 -> 0.59   backward 3.91 -> 2.82        B1 L32768 Di3968  forward 4.05 -> 2.73
-//   B8 L4096 Di4096   forward 2.06 -> 1.07   backward 7.35 -> 4.92        B1 L8192 Di5120   forward 1.13 -> 0.76   backward 3.74 -> 2.05
+//   B4 L4096 Di3968   forward 1.17 -> 0.59   backward 3.91 -> 2.82        B1 L32768 Di3968  forward 4.05 -> 1.70
+//   B8 L4096 Di4096   forward 2.06 -> 1.07   backward 7.35 -> 4.92        B1 L8192 Di5120   forward 1.13 -> 0.56   backward 3.74 -> 2.05
+// (the B1 figures with the time axis split, see b200_selective_scan_parts).
 //
 // The forward stages tiles of 64 steps through shared memory (the next tile's loads are in flight during the steps) and
 // stores the state entering every 32-step half tile (fp32, L/32 × Di × 16).  The backward walks 32-step tiles in reverse,
@@ -86,12 +87,16 @@ __device__ __forceinline__ float lane_scatter_sum(float (&v)[W], int q) {
   return v[0];
 }
 
-template <typename T, int NS, bool RESET>
+// Time may be split into gridDim.z parts of `part` steps (a multiple of 64): a first launch (END) runs every part from h = 0 and
+// leaves its final states, the sum of its dt and whether it holds a reset; the second folds the parts before its own into its
+// initial state (their decay is exp(A·Σdt)) and computes the outputs.
+template <typename T, int NS, bool RESET, bool END>
 __global__ void __launch_bounds__(SS_C * SS_N / NS)
 sscan_fwd_kernel(const T* __restrict__ u, int su, const T* __restrict__ delta, int sd, const float* __restrict__ A,
                  const T* __restrict__ Bm, int sB, const T* __restrict__ Cm, int sC, const float* __restrict__ Dp,
                  const T* __restrict__ z, int sz, const float* __restrict__ dbias, const int* __restrict__ reset,
-                 T* __restrict__ y, float* __restrict__ ckpt, int L, int Di, int softplus) {
+                 T* __restrict__ y, float* __restrict__ ckpt, int L, int Di, int softplus, int part, float* __restrict__ p_h,
+                 float* __restrict__ p_dt, int* __restrict__ p_reset) {
   constexpr int TPC = SS_N / NS;                     // threads per channel
   constexpr int NT = SS_C * TPC;
   constexpr int PPT = SS_T * SS_C / 4 / NT;          // 4-element pieces of a [64, 16] tile per thread
@@ -114,6 +119,23 @@ sscan_fwd_kernel(const T* __restrict__ u, int su, const T* __restrict__ delta, i
   if (Dp) D4 = make_float4(Dp[d0 + pc], Dp[d0 + pc + 1], Dp[d0 + pc + 2], Dp[d0 + pc + 3]);
   const int nseg = (L + SS_T - 1) / SS_T;
   const size_t row0 = static_cast<size_t>(b) * L;
+  const int z0 = blockIdx.z, parts = gridDim.z;
+  const int seg_lo = z0 * (part / SS_T), seg_hi = min(nseg, seg_lo + part / SS_T);
+  float sum_dt = 0.f;
+  int any_reset = 0;
+  if (!END) {
+    for (int k = 0; k < z0; ++k) {
+      const size_t pi = (static_cast<size_t>(b) * parts + k) * Di + d;
+      const bool cut = RESET && p_reset[b * parts + k] != 0;
+      const float sdt = p_dt[pi];
+#pragma unroll
+      for (int j = 0; j < NS / 2; ++j) {
+        const float2 e = *reinterpret_cast<const float2*>(&p_h[pi * SS_N + q * NS + 2 * j]);
+        const float2 a = cut ? make_float2(0.f, 0.f) : make_float2(exp2f(sdt * A2[j].x), exp2f(sdt * A2[j].y));
+        h[j] = fma_f32x2(a, h[j], e);
+      }
+    }
+  }
   Raw4<T> ru[PPT], rd[PPT], rB[PPT], rC[PPT];
   auto fetch = [&](int t0) {
 #pragma unroll
@@ -125,12 +147,12 @@ sscan_fwd_kernel(const T* __restrict__ u, int su, const T* __restrict__ delta, i
         ru[k].load(u + r * su + d0 + pc, vu);
         rd[k].load(delta + r * sd + d0 + pc, vd);
         rB[k].load(Bm + r * sB + pc, vB);
-        rC[k].load(Cm + r * sC + pc, vC);
+        if (!END) rC[k].load(Cm + r * sC + pc, vC);
       }
     }
   };
-  fetch(0);
-  for (int seg = 0; seg < nseg; ++seg) {
+  fetch(seg_lo * SS_T);
+  for (int seg = seg_lo; seg < seg_hi; ++seg) {
     const int t0 = seg * SS_T;
     Raw4<T> cu[PPT], cz[PPT];
 #pragma unroll
@@ -148,12 +170,12 @@ sscan_fwd_kernel(const T* __restrict__ u, int su, const T* __restrict__ delta, i
       o[0] = make_float4(dt.x, dt.x * uu.x, dt.y, dt.y * uu.y);
       o[1] = make_float4(dt.z, dt.z * uu.z, dt.w, dt.w * uu.w);
       *reinterpret_cast<float4*>(&s_B[i][pc]) = rB[k].get();
-      *reinterpret_cast<float4*>(&s_C[i][pc]) = rC[k].get();
+      if (!END) *reinterpret_cast<float4*>(&s_C[i][pc]) = rC[k].get();
     }
     if (RESET && tid < SS_T) s_reset[tid] = t0 + tid < L ? reset[row0 + t0 + tid] : 0;
     __syncthreads();
-    if (seg + 1 < nseg) fetch(t0 + SS_T);
-    if (z) {
+    if (seg + 1 < seg_hi) fetch(t0 + SS_T);
+    if (!END && z) {
 #pragma unroll
       for (int k = 0; k < PPT; ++k) {
         const int t = t0 + pr + k * (NT / 4);
@@ -163,7 +185,7 @@ sscan_fwd_kernel(const T* __restrict__ u, int su, const T* __restrict__ delta, i
     }
 #pragma unroll 1
     for (int sb = 0; sb < SS_T / 8; ++sb) {
-      if ((sb & 3) == 0 && ckpt) {
+      if (!END && (sb & 3) == 0 && ckpt) {
         float* cp = ckpt + ((static_cast<size_t>(b) * nseg * 2 + seg * 2 + (sb >> 2)) * Di + d) * SS_N + q * NS;
         if constexpr (NS == 4) *reinterpret_cast<float4*>(cp) = make_float4(h[0].x, h[0].y, h[1].x, h[1].y);
         else *reinterpret_cast<float2*>(cp) = h[0];
@@ -175,17 +197,22 @@ sscan_fwd_kernel(const T* __restrict__ u, int su, const T* __restrict__ delta, i
         const float2 dd = s_d[i][cl];
         float2 Bv[NS / 2], Cv[NS / 2];
         if constexpr (NS == 4) {
-          const float4 b4 = *reinterpret_cast<const float4*>(&s_B[i][q * 4]), c4 = *reinterpret_cast<const float4*>(&s_C[i][q * 4]);
+          const float4 b4 = *reinterpret_cast<const float4*>(&s_B[i][q * 4]);
           Bv[0] = make_float2(b4.x, b4.y); Bv[1] = make_float2(b4.z, b4.w);
-          Cv[0] = make_float2(c4.x, c4.y); Cv[1] = make_float2(c4.z, c4.w);
+          if (!END) {
+            const float4 c4 = *reinterpret_cast<const float4*>(&s_C[i][q * 4]);
+            Cv[0] = make_float2(c4.x, c4.y); Cv[1] = make_float2(c4.z, c4.w);
+          }
         } else {
           Bv[0] = *reinterpret_cast<const float2*>(&s_B[i][q * 2]);
-          Cv[0] = *reinterpret_cast<const float2*>(&s_C[i][q * 2]);
+          if (!END) Cv[0] = *reinterpret_cast<const float2*>(&s_C[i][q * 2]);
         }
         if (RESET && s_reset[i]) {
+          any_reset = 1;
 #pragma unroll
           for (int j = 0; j < NS / 2; ++j) h[j] = make_float2(0.f, 0.f);
         }
+        if (END) sum_dt += dd.x;
         const float2 dt2 = make_float2(dd.x, dd.x), du2 = make_float2(dd.y, dd.y);
         float2 acc;
 #pragma unroll
@@ -193,10 +220,11 @@ sscan_fwd_kernel(const T* __restrict__ u, int su, const T* __restrict__ delta, i
           const float2 e = mul_f32x2(dt2, A2[j]);
           const float2 a = make_float2(exp2f(e.x), exp2f(e.y));
           h[j] = fma_f32x2(a, h[j], mul_f32x2(du2, Bv[j]));
-          acc = j == 0 ? mul_f32x2(h[j], Cv[j]) : fma_f32x2(h[j], Cv[j], acc);
+          if (!END) acc = j == 0 ? mul_f32x2(h[j], Cv[j]) : fma_f32x2(h[j], Cv[j], acc);
         }
-        p[s] = acc.x + acc.y;
+        if (!END) p[s] = acc.x + acc.y;
       }
+      if (END) continue;
 #pragma unroll
       for (int s0 = 0; s0 < 8; s0 += TPC) {
         float v[TPC];
@@ -207,6 +235,7 @@ sscan_fwd_kernel(const T* __restrict__ u, int su, const T* __restrict__ delta, i
       }
     }
     __syncthreads();
+    if (END) continue;
 #pragma unroll
     for (int k = 0; k < PPT; ++k) {
       const int i = pr + k * (NT / 4), t = t0 + i;
@@ -221,6 +250,13 @@ sscan_fwd_kernel(const T* __restrict__ u, int su, const T* __restrict__ delta, i
         put4(y + (row0 + t) * Di + d0 + pc, yv);
       }
     }
+  }
+  if (END) {
+    const size_t pi = (static_cast<size_t>(b) * parts + z0) * Di + d;
+#pragma unroll
+    for (int j = 0; j < NS / 2; ++j) *reinterpret_cast<float2*>(&p_h[pi * SS_N + q * NS + 2 * j]) = h[j];
+    if (q == 0) p_dt[pi] = sum_dt;
+    if (RESET && blockIdx.x == 0 && tid == 0) p_reset[b * parts + z0] = any_reset;
   }
 }
 
@@ -437,25 +473,54 @@ extern "C" int b200_selective_scan_ckpt_segments(int L) { return 2 * ((L + SS_T 
 template <typename T, int NS>
 static void launch_sscan_fwd(const void* u, int su, const void* delta, int sd, const float* A, const void* Bm, int sB, const void* Cm,
                              int sC, const float* D, const void* z, int sz, const float* dbias, const int* reset, void* y, float* ckpt,
-                             int B, int L, int Di, int softplus, cudaStream_t st) {
-  auto kern = reset ? sscan_fwd_kernel<T, NS, true> : sscan_fwd_kernel<T, NS, false>;
-  kern<<<dim3(Di / SS_C, B), SS_C * SS_N / NS, 0, st>>>((const T*)u, su, (const T*)delta, sd, A, (const T*)Bm, sB, (const T*)Cm, sC, D,
-                                                       (const T*)z, sz, dbias, reset, (T*)y, ckpt, L, Di, softplus);
+                             int B, int L, int Di, int softplus, int parts, float* scratch, cudaStream_t st) {
+  const int part = ((L + parts - 1) / parts + SS_T - 1) / SS_T * SS_T;
+  parts = (L + part - 1) / part;                       // no empty part
+  float* p_h = scratch;
+  float* p_dt = scratch + static_cast<size_t>(B) * parts * Di * SS_N;
+  int* p_reset = reinterpret_cast<int*>(p_dt + static_cast<size_t>(B) * parts * Di);
+  auto run = [&](auto kern, int nz) {
+    kern<<<dim3(Di / SS_C, B, nz), SS_C * SS_N / NS, 0, st>>>((const T*)u, su, (const T*)delta, sd, A, (const T*)Bm, sB, (const T*)Cm, sC, D,
+                                                             (const T*)z, sz, dbias, reset, (T*)y, ckpt, L, Di, softplus, part, p_h, p_dt,
+                                                             p_reset);
+  };
+  if (parts > 1) {
+    if constexpr (NS == 4) {
+      if (reset) run(sscan_fwd_kernel<T, 4, true, true>, parts); else run(sscan_fwd_kernel<T, 4, false, true>, parts);
+    }
+  }
+  if (reset) run(sscan_fwd_kernel<T, NS, true, false>, parts); else run(sscan_fwd_kernel<T, NS, false, false>, parts);
+}
+
+// Parts of the sequence that the forward scan runs side by side.  With few channels the steps cost their latency: splitting the
+// time costs a second pass over the exponentials but multiplies the warps.  Parts are kept at 512 steps or more.  Whole -> split,
+// ms: B1 L32768 Di3968 2.73 -> 1.70, B1 L8192 Di5120 0.76 -> 0.56, but B2 L4096 Di4096 0.432 -> 0.462: the line lies at B·Di = 8192.
+extern "C" int b200_selective_scan_parts(int B, int L, int Di) {
+  const long long width = static_cast<long long>(B) * Di;
+  if (width <= 0 || width >= 8192) return 1;
+  int parts = static_cast<int>((49152 + width - 1) / width);
+  if (parts > L / 512) parts = L / 512;
+  return parts > 2 ? parts : 1;                        // two parts would only pay back the second pass
+}
+// floats of scratch for that many parts
+extern "C" long long b200_selective_scan_scratch(int B, int Di, int parts) {
+  return parts > 1 ? static_cast<long long>(B) * parts * (Di * (SS_N + 1LL) + 1) : 0;
 }
 
 // u, delta, z: rows of `su`, `sd`, `sz` elements; Bm, Cm: [B·L, 16] with row strides sB, sC; y: dense [B, L, Di].
 // reset: int32 per token (1 = h is cleared before this step) or null.  ckpt: fp32 [B, 2·ceil(L/64), Di, 16] or null.
+// parts, scratch: see b200_selective_scan_parts / _scratch (1, null: one pass).
 extern "C" int b200_selective_scan_fwd(const void* u, int su, const void* delta, int sd, const float* A, const void* Bm, int sB,
                                        const void* Cm, int sC, const float* D, const void* z, int sz, const float* dbias,
-                                       const int* reset, void* y, float* ckpt, int dtype, int B, int L, int Di, int softplus,
-                                       cudaStream_t st) {
-  if (Di % SS_C) return -1;
+                                       const int* reset, void* y, float* ckpt, int dtype, int B, int L, int Di, int softplus, int parts,
+                                       float* scratch, cudaStream_t st) {
+  if (Di % SS_C || parts < 1 || (parts > 1 && !scratch)) return -1;
   if (B * L == 0) return 0;
   // four states per thread need B·Di/8 warps to fill the 592 schedulers about three deep; below that two states per thread
-  const bool ns4 = static_cast<long long>(B) * Di >= 12288;
+  const bool ns4 = parts > 1 || static_cast<long long>(B) * Di >= 12288;
   auto run = dtype == 1 ? (ns4 ? launch_sscan_fwd<__nv_bfloat16, 4> : launch_sscan_fwd<__nv_bfloat16, 2>)
                         : (ns4 ? launch_sscan_fwd<float, 4> : launch_sscan_fwd<float, 2>);
-  run(u, su, delta, sd, A, Bm, sB, Cm, sC, D, z, sz, dbias, reset, y, ckpt, B, L, Di, softplus, st);
+  run(u, su, delta, sd, A, Bm, sB, Cm, sC, D, z, sz, dbias, reset, y, ckpt, B, L, Di, softplus, parts, scratch, st);
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 

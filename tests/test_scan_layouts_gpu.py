@@ -27,6 +27,9 @@ def _scan_case(B, L, Di, dtype, packed, gate, shift):
     (1, 129, 12288, torch.float32, True, True, 0),      # four states per thread with documents, breaks on and beside tile edges
     (1, 100, 64, torch.float32, True, False, 2),
     (1, 1, 16, torch.float32, False, True, 0),
+    (1, 1536, 48, torch.float32, False, True, 0),       # time in three parts
+    (1, 1601, 32, torch.float32, True, True, 0),        # parts of 576 steps, the last one shorter; breaks in the first part only
+    (2, 2049, 32, torch.bfloat16, False, False, 1),     # one step into the last 64-step tile
 ])
 def test_selective_scan_branches(B, L, Di, dtype, packed, gate, shift):
     from archscale_b200.ops.selective_scan import selective_scan, selective_scan_ref
