@@ -5,9 +5,10 @@ Behavioural reference: `lit_gpt/selective_scan_interface.py:102-168` (``selectiv
 ``Δ = softplus(Δ + bias)``; packed sequences reset ``h`` at every ``cu_seqlens`` boundary
 (the varlen fork used at `lit_gpt/mamba_simple.py:84-88`).
 
-CUDA path: ``csrc/selective_scan.cu`` — one thread per (batch, channel, state), 64-step tiles staged
-through shared memory, state sums by warp shuffles; the backward recomputes each tile's states from
-the per-tile checkpoints saved by the forward and runs the adjoint recurrence in reverse.
+CUDA path: ``csrc/selective_scan.cu`` — two or four states per thread, tiles of steps staged through
+shared memory, state sums in registers and by short lane reductions (small batches also split the
+time axis); the backward recomputes each tile's states from the checkpoints saved by the forward
+and runs the adjoint recurrence in reverse.
 """
 from __future__ import annotations
 
