@@ -8,8 +8,8 @@
 // shared-memory loads, fifteen sixteenths of a shuffle and its selects per state.  Several states per thread share the loads of dt and dt·u, read B and C as vectors, do two states per instruction
 // (fma.rn.f32x2) and add most of the sum over states in registers; the remaining 16/NS lanes use a reduce-scatter over 16/NS
 // steps (lane q ends up with the total of step q).  Measured, one state -> several states per thread, ms:
-//   B4 L4096 Di3968   forward 1.17 -> 0.59   backward 3.91 -> 2.82        B1 L32768 Di3968  forward 4.05 -> 1.70
-//   B8 L4096 Di4096   forward 2.06 -> 1.07   backward 7.35 -> 4.92        B1 L8192 Di5120   forward 1.13 -> 0.56   backward 3.74 -> 2.05
+//   B4 L4096 Di3968   forward 1.17 -> 0.59   backward 3.91 -> 2.34        B1 L32768 Di3968  forward 4.05 -> 1.70
+//   B8 L4096 Di4096   forward 2.06 -> 1.07   backward 7.35 -> 4.67        B1 L8192 Di5120   forward 1.13 -> 0.56   backward 3.74 -> 2.15
 // (the B1 figures with the time axis split, see b200_selective_scan_parts).
 //
 // The forward stages tiles of 64 steps through shared memory (the next tile's loads are in flight during the steps) and
@@ -260,8 +260,12 @@ sscan_fwd_kernel(const T* __restrict__ u, int su, const T* __restrict__ delta, i
   }
 }
 
-template <typename T, bool RESET, bool GATE>
-__global__ void __launch_bounds__(128, 3)
+// MINB: resident CTAs per SM the registers are limited for.  2 (255 registers, hardly any spill) where the grid leaves no more
+// to an SM anyway, else 4 (128 registers).  ms with 2 / 3 / 4: B4 L4096 Di3968 (992 CTAs) 2.91 / 2.84 / 2.34, B8 L4096 Di4096
+// 5.09 / 5.10 / 4.67, B2 L4096 Di4096 (512) 1.51 / 1.92 / 1.32, B1 L8192 Di5120 (320) 2.59 / 2.14 / 2.15, B1 L32768 Di3968 (248)
+// 5.85 / 6.75 / 7.13.
+template <typename T, bool RESET, bool GATE, int MINB>
+__global__ void __launch_bounds__(128, MINB)
 sscan_bwd_kernel(const T* __restrict__ dy, int sdy, const T* __restrict__ u, int su, const T* __restrict__ delta, int sd,
                  const float* __restrict__ A, const T* __restrict__ Bm, int sB, const T* __restrict__ Cm, int sC,
                  const float* __restrict__ Dp, const T* __restrict__ z, int sz, const float* __restrict__ dbias,
@@ -529,8 +533,11 @@ static void launch_sscan_bwd(const void* dy, int sdy, const void* u, int su, con
                              int sB, const void* Cm, int sC, const float* D, const void* z, int sz, const float* dbias, const int* reset,
                              const float* ckpt, void* du, void* ddelta, void* dz, float* dA, float* partB, float* partC, void* dB,
                              void* dC, float* dD, float* ddbias, int B, int L, int Di, int softplus, cudaStream_t st) {
-  auto kern = reset ? (z ? sscan_bwd_kernel<T, true, true> : sscan_bwd_kernel<T, true, false>)
-                    : (z ? sscan_bwd_kernel<T, false, true> : sscan_bwd_kernel<T, false, false>);
+  const bool few = static_cast<long long>(B) * (Di / SS_C) <= 2 * 148;
+  auto kern = reset ? (z ? (few ? sscan_bwd_kernel<T, true, true, 2> : sscan_bwd_kernel<T, true, true, 4>)
+                         : (few ? sscan_bwd_kernel<T, true, false, 2> : sscan_bwd_kernel<T, true, false, 4>))
+                    : (z ? (few ? sscan_bwd_kernel<T, false, true, 2> : sscan_bwd_kernel<T, false, true, 4>)
+                         : (few ? sscan_bwd_kernel<T, false, false, 2> : sscan_bwd_kernel<T, false, false, 4>));
   kern<<<dim3(Di / SS_C, B), 128, 0, st>>>((const T*)dy, sdy, (const T*)u, su, (const T*)delta, sd, A, (const T*)Bm, sB, (const T*)Cm, sC,
                                            D, (const T*)z, sz, dbias, reset, ckpt, (T*)du, (T*)ddelta, (T*)dz, dA, partB, partC, dD,
                                            ddbias, L, Di, softplus);
