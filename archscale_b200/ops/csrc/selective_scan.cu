@@ -131,8 +131,8 @@ sscan_fwd_kernel(const T* __restrict__ u, int su, const T* __restrict__ delta, i
 #pragma unroll
       for (int j = 0; j < NS / 2; ++j) {
         const float2 e = *reinterpret_cast<const float2*>(&p_h[pi * SS_N + q * NS + 2 * j]);
-        const float2 a = cut ? make_float2(0.f, 0.f) : make_float2(exp2f(sdt * A2[j].x), exp2f(sdt * A2[j].y));
-        h[j] = fma_f32x2(a, h[j], e);
+        // selected, not multiplied by zero: a state that is not finite ends with its document
+        h[j] = cut ? e : fma_f32x2(make_float2(exp2f(sdt * A2[j].x), exp2f(sdt * A2[j].y)), h[j], e);
       }
     }
   }
