@@ -71,6 +71,14 @@ template <typename T> __host__ __device__ __forceinline__ bool rows_vec4(const T
 __device__ __forceinline__ float ss_softplus(float x) { return x > 20.f ? x : log1pf(__expf(x)); }
 __device__ __forceinline__ float ss_sigmoid(float x) { return 1.f / (1.f + __expf(-x)); }
 
+// 2^x · h as (2^(x − cap) · h) · cap with cap = 2^min(x, 126): growing states (A·dt > 0) may gain more than the largest float over
+// a part, and the product is still what the steps give: zero stays zero (not 0·inf), a small state stays finite.  For x ≤ 126
+// the first factor is exactly one.
+__device__ __forceinline__ float2 ss_exp2_cap(float2 x) { return make_float2(exp2f(fminf(x.x, 126.f)), exp2f(fminf(x.y, 126.f))); }
+__device__ __forceinline__ float2 ss_exp2_mul(float2 x, float2 h) {
+  return make_float2(exp2f(fminf(fmaxf(x.x - 126.f, 0.f), 126.f)) * h.x, exp2f(fminf(fmaxf(x.y - 126.f, 0.f), 126.f)) * h.y);
+}
+
 // v[s] (s = 0..W-1) summed over W neighbouring lanes (lane index q inside the group); lane q returns the total of step q.
 template <int W>
 __device__ __forceinline__ float lane_scatter_sum(float (&v)[W], int q) {
@@ -121,7 +129,7 @@ sscan_fwd_kernel(const T* __restrict__ u, int su, const T* __restrict__ delta, i
   const size_t row0 = static_cast<size_t>(b) * L;
   const int z0 = blockIdx.z, parts = gridDim.z;
   const int seg_lo = z0 * (part / SS_T), seg_hi = min(nseg, seg_lo + part / SS_T);
-  float sum_dt = 0.f;
+  float sum_dt = 0.f, sum_lost = 0.f;                // Σdt and what its additions rounded off
   int any_reset = 0;
   if (!END) {
     for (int k = 0; k < z0; ++k) {
@@ -131,8 +139,9 @@ sscan_fwd_kernel(const T* __restrict__ u, int su, const T* __restrict__ delta, i
 #pragma unroll
       for (int j = 0; j < NS / 2; ++j) {
         const float2 e = *reinterpret_cast<const float2*>(&p_h[pi * SS_N + q * NS + 2 * j]);
+        const float2 x = make_float2(sdt * A2[j].x, sdt * A2[j].y);
         // selected, not multiplied by zero: a state that is not finite ends with its document
-        h[j] = cut ? e : fma_f32x2(make_float2(exp2f(sdt * A2[j].x), exp2f(sdt * A2[j].y)), h[j], e);
+        h[j] = cut ? e : fma_f32x2(ss_exp2_mul(x, h[j]), ss_exp2_cap(x), e);
       }
     }
   }
@@ -212,7 +221,7 @@ sscan_fwd_kernel(const T* __restrict__ u, int su, const T* __restrict__ delta, i
 #pragma unroll
           for (int j = 0; j < NS / 2; ++j) h[j] = make_float2(0.f, 0.f);
         }
-        if (END) sum_dt += dd.x;
+        if (END) p[s] = dd.x;
         const float2 dt2 = make_float2(dd.x, dd.x), du2 = make_float2(dd.y, dd.y);
         float2 acc;
 #pragma unroll
@@ -224,7 +233,13 @@ sscan_fwd_kernel(const T* __restrict__ u, int su, const T* __restrict__ delta, i
         }
         if (!END) p[s] = acc.x + acc.y;
       }
-      if (END) continue;
+      if (END) {
+        // a plain chain of equal steps rounds the same way every time: 6e-4 of a state that grows by e^115 over a part
+        const float g = ((p[0] + p[1]) + (p[2] + p[3])) + ((p[4] + p[5]) + (p[6] + p[7])), t = __fadd_rn(sum_dt, g);
+        sum_lost = __fadd_rn(sum_lost, __fsub_rn(g, __fsub_rn(t, sum_dt)));
+        sum_dt = t;
+        continue;
+      }
 #pragma unroll
       for (int s0 = 0; s0 < 8; s0 += TPC) {
         float v[TPC];
@@ -255,7 +270,8 @@ sscan_fwd_kernel(const T* __restrict__ u, int su, const T* __restrict__ delta, i
     const size_t pi = (static_cast<size_t>(b) * parts + z0) * Di + d;
 #pragma unroll
     for (int j = 0; j < NS / 2; ++j) *reinterpret_cast<float2*>(&p_h[pi * SS_N + q * NS + 2 * j]) = h[j];
-    if (q == 0) p_dt[pi] = sum_dt;
+    const float sum = sum_dt + sum_lost;
+    if (q == 0) p_dt[pi] = sum == sum ? sum : sum_dt;    // an infinite Σdt has no remainder
     if (RESET && blockIdx.x == 0 && tid == 0) p_reset[b * parts + z0] = any_reset;
   }
 }

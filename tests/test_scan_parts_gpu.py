@@ -72,3 +72,23 @@ def test_documents_stay_separate(bad, cut):
     y = _run(x, cu)
     assert torch.equal(y[:, cut:], clean[:, cut:])
     assert not bool(torch.isfinite(y[0, 5:cut, 3]).all())
+
+
+def test_growing_states():
+    """exp(A·Σdt) of a part beyond the largest float meets a state that is zero or small: the product is what the steps give."""
+    L, Di = 2304, 48
+    x = _inputs(1, L, Di, 1.0)
+    x["A"], x["delta_bias"] = torch.ones(Di, 16, device="cuda"), torch.zeros(Di, device="cuda")
+    x["delta"] = torch.full((1, L, Di), 0.2, device="cuda")           # e^115 per part of 576 steps
+    x["u"][:, :2100] = 0.0                                            # the state leaves zero in the last part
+    x["u"][:, 2104:] = 0.0
+    y, yr = _run(x, softplus=False), _oracle(x, softplus=False)
+    assert float((y.double() - yr).norm()) <= 1e-4 * float(yr.norm())  # 200 steps, each with the rounded exponential (2^-22)
+    x["delta"][:, :1152] = 0.0                                        # the state 1e-30 in front of the third part grows e^115-fold
+    x["u"].zero_()
+    x["u"][:, 1151] = 1e-30
+    x["delta"][:, 1151] = 1.0
+    x["delta"][:, 1728:] = 0.0
+    y, yr = _run(x, softplus=False), _oracle(x, softplus=False)
+    assert bool(torch.isfinite(yr.float()).all())
+    assert float((y.double() - yr).norm()) <= 1e-4 * float(yr.norm())
