@@ -18,6 +18,7 @@
 //   G_t = C_t·dy'_t + a_{t+1}·G_{t+1}
 // dB/dC (sums over channels) are reduced over the warp's 4 channels by shuffles and over the CTA's 4 warps in shared memory,
 // written as per-CTA partial sums and summed over channel blocks by a second kernel (deterministic, no atomics).
+#include <type_traits>
 #include "sm100.cuh"
 #include "api.h"
 
@@ -110,7 +111,7 @@ sscan_fwd_kernel(const T* __restrict__ u, int su, const T* __restrict__ delta, i
   constexpr int PPT = SS_T * SS_C / 4 / NT;          // 4-element pieces of a [64, 16] tile per thread
   __shared__ __align__(16) float2 s_d[SS_T][SS_C];   // (dt, dt·u)
   __shared__ __align__(16) float s_B[SS_T][SS_N], s_C[SS_T][SS_N], s_y[SS_T][SS_YP];
-  __shared__ int s_reset[SS_T];
+  __shared__ unsigned s_reset[SS_T / 32];            // one bit per step
   const int tid = threadIdx.x;
   const int cl = tid / TPC, q = tid % TPC;
   const int d0 = blockIdx.x * SS_C, b = blockIdx.y, d = d0 + cl;
@@ -181,7 +182,10 @@ sscan_fwd_kernel(const T* __restrict__ u, int su, const T* __restrict__ delta, i
       *reinterpret_cast<float4*>(&s_B[i][pc]) = rB[k].get();
       if (!END) *reinterpret_cast<float4*>(&s_C[i][pc]) = rC[k].get();
     }
-    if (RESET && tid < SS_T) s_reset[tid] = t0 + tid < L ? reset[row0 + t0 + tid] : 0;
+    if (RESET && tid < SS_T) {
+      const unsigned m = __ballot_sync(0xffffffffu, t0 + tid < L && reset[row0 + t0 + tid] != 0);
+      if ((tid & 31) == 0) s_reset[tid >> 5] = m;
+    }
     __syncthreads();
     if (seg + 1 < seg_hi) fetch(t0 + SS_T);
     if (!END && z) {
@@ -200,38 +204,47 @@ sscan_fwd_kernel(const T* __restrict__ u, int su, const T* __restrict__ delta, i
         else *reinterpret_cast<float2*>(cp) = h[0];
       }
       float p[8];
+      // eight steps; the ones that clear the state first are marked in `bits` (CLEAR: there are any)
+      auto steps = [&](auto CLEAR, unsigned bits) {
 #pragma unroll
-      for (int s = 0; s < 8; ++s) {
-        const int i = sb * 8 + s;
-        const float2 dd = s_d[i][cl];
-        float2 Bv[NS / 2], Cv[NS / 2];
-        if constexpr (NS == 4) {
-          const float4 b4 = *reinterpret_cast<const float4*>(&s_B[i][q * 4]);
-          Bv[0] = make_float2(b4.x, b4.y); Bv[1] = make_float2(b4.z, b4.w);
-          if (!END) {
-            const float4 c4 = *reinterpret_cast<const float4*>(&s_C[i][q * 4]);
-            Cv[0] = make_float2(c4.x, c4.y); Cv[1] = make_float2(c4.z, c4.w);
+        for (int s = 0; s < 8; ++s) {
+          const int i = sb * 8 + s;
+          const float2 dd = s_d[i][cl];
+          float2 Bv[NS / 2], Cv[NS / 2];
+          if constexpr (NS == 4) {
+            const float4 b4 = *reinterpret_cast<const float4*>(&s_B[i][q * 4]);
+            Bv[0] = make_float2(b4.x, b4.y); Bv[1] = make_float2(b4.z, b4.w);
+            if (!END) {
+              const float4 c4 = *reinterpret_cast<const float4*>(&s_C[i][q * 4]);
+              Cv[0] = make_float2(c4.x, c4.y); Cv[1] = make_float2(c4.z, c4.w);
+            }
+          } else {
+            Bv[0] = *reinterpret_cast<const float2*>(&s_B[i][q * 2]);
+            if (!END) Cv[0] = *reinterpret_cast<const float2*>(&s_C[i][q * 2]);
           }
-        } else {
-          Bv[0] = *reinterpret_cast<const float2*>(&s_B[i][q * 2]);
-          if (!END) Cv[0] = *reinterpret_cast<const float2*>(&s_C[i][q * 2]);
-        }
-        if (RESET && s_reset[i]) {
-          any_reset = 1;
+          if (decltype(CLEAR)::value && (bits >> s & 1)) {
 #pragma unroll
-          for (int j = 0; j < NS / 2; ++j) h[j] = make_float2(0.f, 0.f);
-        }
-        if (END) p[s] = dd.x;
-        const float2 dt2 = make_float2(dd.x, dd.x), du2 = make_float2(dd.y, dd.y);
-        float2 acc;
+            for (int j = 0; j < NS / 2; ++j) h[j] = make_float2(0.f, 0.f);
+          }
+          if (END) p[s] = dd.x;
+          const float2 dt2 = make_float2(dd.x, dd.x), du2 = make_float2(dd.y, dd.y);
+          float2 acc;
 #pragma unroll
-        for (int j = 0; j < NS / 2; ++j) {
-          const float2 e = mul_f32x2(dt2, A2[j]);
-          const float2 a = make_float2(exp2f(e.x), exp2f(e.y));
-          h[j] = fma_f32x2(a, h[j], mul_f32x2(du2, Bv[j]));
-          if (!END) acc = j == 0 ? mul_f32x2(h[j], Cv[j]) : fma_f32x2(h[j], Cv[j], acc);
+          for (int j = 0; j < NS / 2; ++j) {
+            const float2 e = mul_f32x2(dt2, A2[j]);
+            const float2 a = make_float2(exp2f(e.x), exp2f(e.y));
+            h[j] = fma_f32x2(a, h[j], mul_f32x2(du2, Bv[j]));
+            if (!END) acc = j == 0 ? mul_f32x2(h[j], Cv[j]) : fma_f32x2(h[j], Cv[j], acc);
+          }
+          if (!END) p[s] = acc.x + acc.y;
         }
-        if (!END) p[s] = acc.x + acc.y;
+      };
+      const unsigned bits = RESET ? s_reset[sb >> 2] >> (sb & 3) * 8 & 0xff : 0;
+      if (RESET && bits) {
+        any_reset = 1;
+        steps(std::true_type(), bits);
+      } else {
+        steps(std::false_type(), 0);
       }
       if (END) {
         // a plain chain of equal steps rounds the same way every time: 6e-4 of a state that grows by e^115 over a part
