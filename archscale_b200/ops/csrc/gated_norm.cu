@@ -100,8 +100,10 @@ __global__ void __launch_bounds__(256) gated_rmsnorm_fwd_team_kernel(const T* __
   }
 }
 
-template <typename T, int W>
-__global__ void __launch_bounds__(256, 2) gated_rmsnorm_bwd_team_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ z,
+// K: chunks of 256·W columns that a lane takes part in (1 or 2).  Groups of up to 256 columns need half the registers (K = 1): three
+// CTAs to an SM instead of two.
+template <typename T, int W, int K>
+__global__ void __launch_bounds__(256, K == 1 ? 3 : 2) gated_rmsnorm_bwd_team_kernel(const T* __restrict__ dy, const T* __restrict__ x, const T* __restrict__ z,
                                                                         const float* __restrict__ w, const float* __restrict__ rstd,
                                                                         T* __restrict__ dx, T* __restrict__ dz, float* __restrict__ dw,
                                                                         long long rows, int cols, int gsize, int nbg) {
@@ -113,9 +115,9 @@ __global__ void __launch_bounds__(256, 2) gated_rmsnorm_bwd_team_kernel(const T*
   const int ctas_per_group = gridDim.x / ngroups, cta_in_group = blockIdx.x / ngroups;
   constexpr int TEAMS = 8 / W;
   for (int c = threadIdx.x; c < gsize; c += blockDim.x) gn_dw[c] = 0.f;
-  float wr[2][8], dwa[2][8];
+  float wr[K][8], dwa[K][8];
 #pragma unroll
-  for (int k = 0; k < 2; ++k) {
+  for (int k = 0; k < K; ++k) {
     const int c = (warp % W * 32 + lane) * 8 + k * W * 256;
 #pragma unroll
     for (int i = 0; i < 8; ++i) wr[k][i] = dwa[k][i] = 0.f;
@@ -125,9 +127,9 @@ __global__ void __launch_bounds__(256, 2) gated_rmsnorm_bwd_team_kernel(const T*
   for (long long row = static_cast<long long>(cta_in_group) * TEAMS + warp / W; row < rows; row += static_cast<long long>(ctas_per_group) * TEAMS, ++it) {
     const size_t base = static_cast<size_t>(row) * cols + g0;
     const float rs = rstd[row * ngroups + grp];
-    float xv[2][8], dv[2][8], zv[2][8], sg[2][8];
+    float xv[K][8], dv[K][8], zv[K][8], sg[K][8];
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
+    for (int k = 0; k < K; ++k) {
       const int c = (warp % W * 32 + lane) * 8 + k * W * 256;
       if (c < gsize) {
         gn_ld8(x + base + c, xv[k]);
@@ -137,7 +139,7 @@ __global__ void __launch_bounds__(256, 2) gated_rmsnorm_bwd_team_kernel(const T*
     }
     float dot = 0.f;                               // Σ gw · xin  (xin = what was normalised)
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
+    for (int k = 0; k < K; ++k) {
       const int c = (warp % W * 32 + lane) * 8 + k * W * 256;
       if (c < gsize) {
 #pragma unroll
@@ -150,7 +152,7 @@ __global__ void __launch_bounds__(256, 2) gated_rmsnorm_bwd_team_kernel(const T*
     }
     const float c1 = gn_team_sum<W>(dot, slots[it & 1], warp, lane) * rs * rs * rs / gsize;
 #pragma unroll
-    for (int k = 0; k < 2; ++k) {
+    for (int k = 0; k < K; ++k) {
       const int c = (warp % W * 32 + lane) * 8 + k * W * 256;
       if (c < gsize) {
         float ox[8], oz[8];
@@ -174,7 +176,7 @@ __global__ void __launch_bounds__(256, 2) gated_rmsnorm_bwd_team_kernel(const T*
   for (int turn = 0; turn < TEAMS; ++turn) {       // the teams add their sums in turn
     if (warp / W == turn) {
 #pragma unroll
-      for (int k = 0; k < 2; ++k) {
+      for (int k = 0; k < K; ++k) {
         const int c = (warp % W * 32 + lane) * 8 + k * W * 256;
         if (c < gsize) {
 #pragma unroll
@@ -322,11 +324,21 @@ extern "C" int b200_gated_rmsnorm_bwd(const void* dy, const void* x, const void*
     int per = (148 * 2 + ngroups - 1) / ngroups;     // two CTAs per SM
     const long long need = (rows + teams - 1) / teams;
     if (per > need) per = static_cast<int>(need);
+    if (gsize <= 256) {
+      // up to six CTAs per SM (two waves of three) as long as every warp has three rows: in a narrow group most lanes idle and the
+      // rows of a warp are a chain of load latencies.  ms, two CTAs per SM with K = 2 -> this: 1000 x 1024 in groups of 64
+      // 0.0179 -> 0.0128 (fp32 0.0173 -> 0.0118), 4096 x 512 in groups of 32 0.0584 -> 0.0388, 16384 x 1024 in groups of 128
+      // 0.083 -> 0.078, 8193 x 1536 in groups of 256 0.056 -> 0.033; with fewer rows per warp 1000 x 1024 in groups of 128
+      // 0.0087 -> 0.0092.
+      const long long more = (rows + 3 * teams - 1) / (3 * teams), most = (148 * 6 + ngroups - 1) / ngroups;
+      if (per < more && per < most) per = static_cast<int>(more < most ? more : most);
+    }
     const unsigned grid = static_cast<unsigned>(per * ngroups);
-#define GN_BWD(T, WW)                                                                                                       \
-  gated_rmsnorm_bwd_team_kernel<T, WW><<<grid, 256, sizeof(float) * gsize, st>>>((const T*)dy, (const T*)x, (const T*)z, w, rstd, \
+#define GN_BWD(T, WW, KK)                                                                                                   \
+  gated_rmsnorm_bwd_team_kernel<T, WW, KK><<<grid, 256, sizeof(float) * gsize, st>>>((const T*)dy, (const T*)x, (const T*)z, w, rstd, \
                                                                                  (T*)dx, (T*)dz, dw, rows, cols, gsize, norm_before_gate)
-#define GN_BWD_W(T) do { if (W == 1) GN_BWD(T, 1); else if (W == 2) GN_BWD(T, 2); else if (W == 4) GN_BWD(T, 4); else GN_BWD(T, 8); } while (0)
+#define GN_BWD_W(T) do { if (gsize <= 256) GN_BWD(T, 1, 1); else if (W == 1) GN_BWD(T, 1, 2); else if (W == 2) GN_BWD(T, 2, 2); \
+                         else if (W == 4) GN_BWD(T, 4, 2); else GN_BWD(T, 8, 2); } while (0)
     if (dtype == 1) GN_BWD_W(__nv_bfloat16); else GN_BWD_W(float);
 #undef GN_BWD_W
 #undef GN_BWD
