@@ -111,35 +111,35 @@ __global__ void __launch_bounds__(128) conv1d_fwd_kernel(const T* __restrict__ x
         if (t0 + (g + 1) * U + u < t_end) nx[u].ld(xb + static_cast<size_t>(t0 + (g + 1) * U + u) * xs);
     }
 #pragma unroll
-  for (int u = 0; u < U; ++u) {
-    const int t = t0 + g * U + u;
-    if (t >= t_end) return;
-    cx[u].get(win[W - 1]);
-    const int sid = sb ? sb[t] : 0;
-    sid_hist[W - 1] = sid;
-    float acc[8];
+    for (int u = 0; u < U; ++u) {
+      const int t = t0 + g * U + u;
+      if (t >= t_end) return;
+      cx[u].get(win[W - 1]);
+      const int sid = sb ? sb[t] : 0;
+      sid_hist[W - 1] = sid;
+      float acc[8];
 #pragma unroll
-    for (int e = 0; e < 8; ++e) acc[e] = bs[e];
+      for (int e = 0; e < 8; ++e) acc[e] = bs[e];
 #pragma unroll
-    for (int j = 0; j < W; ++j) {
-      const bool ok = !sb || sid_hist[j] == sid;
-      if (ok) {
+      for (int j = 0; j < W; ++j) {
+        const bool ok = !sb || sid_hist[j] == sid;
+        if (ok) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) acc[e] += wk[j][e] * win[j][e];
+          for (int e = 0; e < 8; ++e) acc[e] += wk[j][e] * win[j][e];
+        }
+      }
+      if (silu) {
+#pragma unroll
+        for (int e = 0; e < 8; ++e) acc[e] = silu_f(acc[e]);
+      }
+      V8<T>::st(yb + static_cast<size_t>(t) * C, acc);
+#pragma unroll
+      for (int j = 0; j < W - 1; ++j) {
+        sid_hist[j] = sid_hist[j + 1];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) win[j][e] = win[j + 1][e];
       }
     }
-    if (silu) {
-#pragma unroll
-      for (int e = 0; e < 8; ++e) acc[e] = silu_f(acc[e]);
-    }
-    V8<T>::st(yb + static_cast<size_t>(t) * C, acc);
-#pragma unroll
-    for (int j = 0; j < W - 1; ++j) {
-      sid_hist[j] = sid_hist[j + 1];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) win[j][e] = win[j + 1][e];
-    }
-  }
   }
 }
 
@@ -151,7 +151,9 @@ __global__ void __launch_bounds__(128) conv1d_fwd_kernel(const T* __restrict__ x
 // thread (W·8 + 8 of them per 128 positions).
 constexpr int CV_TSTEP_BWD = 128;
 
-template <typename T, int W>
+// AHEAD: a group of U steps is loaded while the previous one is worked on; the document ids with it where there are registers for
+// them (bf16 with four taps fills 255 as it is: 0.212 -> 0.217 ms at B4 L4096 C3968 with them).
+template <typename T, int W, bool AHEAD>
 __global__ void __launch_bounds__(128) conv1d_bwd_kernel(const T* __restrict__ dy, const T* __restrict__ x, const float* __restrict__ w,
                                                          const float* __restrict__ bias, const int* __restrict__ seq_idx,
                                                          T* __restrict__ dx, float* __restrict__ dw, float* __restrict__ db, int B, int L,
@@ -185,86 +187,91 @@ __global__ void __launch_bounds__(128) conv1d_bwd_kernel(const T* __restrict__ d
 #pragma unroll
     for (int e = 0; e < 8; ++e) gw[k][e] = 0.f;
   }
-  constexpr int U = sizeof(T) == 2 ? 4 : 2;
+  constexpr int U = !AHEAD ? 1 : sizeof(T) == 2 ? 4 : 2;
+  constexpr bool IDS = sizeof(T) == 4 || W == 2;
   Raw8<T> nx[U], nd[U];
+  int ns[U];
   auto fetch = [&](int t) {
 #pragma unroll
     for (int u = 0; u < U; ++u)
       if (t + u < L && t + u < t_end + W - 1) {
         nx[u].ld(x + (static_cast<size_t>(b) * L + t + u) * xs + c0);
         nd[u].ld(dy + (static_cast<size_t>(b) * L + t + u) * dys + c0);
+        if (IDS) ns[u] = sb ? sb[t + u] : 0;
       }
   };
-  fetch(t0);
+  if (AHEAD) fetch(t0);
 #pragma unroll 1
   for (int tg = t0; tg < t_end + W - 1; tg += U) {
+    if (!AHEAD) fetch(tg);
     Raw8<T> cx[U], cd[U];
+    int cs[U];
 #pragma unroll
-    for (int u = 0; u < U; ++u) { cx[u] = nx[u]; cd[u] = nd[u]; }
-    fetch(tg + U);
+    for (int u = 0; u < U; ++u) { cx[u] = nx[u]; cd[u] = nd[u]; if (IDS) cs[u] = ns[u]; }
+    if (AHEAD) fetch(tg + U);
 #pragma unroll
-  for (int u = 0; u < U; ++u) {
-    const int t = tg + u;
-    if (t >= t_end + W - 1) break;
-    // shift the windows by one step
+    for (int u = 0; u < U; ++u) {
+      const int t = tg + u;
+      if (t >= t_end + W - 1) break;
+      // shift the windows by one step
 #pragma unroll
-    for (int k = 0; k < W - 1; ++k) {
-      sw[k] = sw[k + 1];
+      for (int k = 0; k < W - 1; ++k) {
+        sw[k] = sw[k + 1];
 #pragma unroll
-      for (int e = 0; e < 8; ++e) { xw[k][e] = xw[k + 1][e]; gw[k][e] = gw[k + 1][e]; }
-    }
-    if (t < L) {
-      sw[W - 1] = sb ? sb[t] : 0;
-      cx[u].get(xw[W - 1]);
-      float pre[8], g[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) pre[e] = bs[e];
-#pragma unroll
-      for (int k = 0; k < W; ++k) {
-        if (sw[k] == sw[W - 1]) {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) pre[e] += wk[k][e] * xw[k][e];
-        }
+        for (int e = 0; e < 8; ++e) { xw[k][e] = xw[k + 1][e]; gw[k][e] = gw[k + 1][e]; }
       }
-      cd[u].get(g);
-      if (silu) {
+      if (t < L) {
+        sw[W - 1] = IDS ? cs[u] : sb ? sb[t] : 0;
+        cx[u].get(xw[W - 1]);
+        float pre[8], g[8];
 #pragma unroll
-        for (int e = 0; e < 8; ++e) g[e] *= dsilu_f(pre[e]);
-      }
-#pragma unroll
-      for (int e = 0; e < 8; ++e) gw[W - 1][e] = g[e];
-      if (t < t_end) {                                  // this block owns output step t: its weight / bias gradients
+        for (int e = 0; e < 8; ++e) pre[e] = bs[e];
 #pragma unroll
         for (int k = 0; k < W; ++k) {
           if (sw[k] == sw[W - 1]) {
 #pragma unroll
-            for (int e = 0; e < 8; ++e) dwa[k][e] += g[e] * xw[k][e];
+            for (int e = 0; e < 8; ++e) pre[e] += wk[k][e] * xw[k][e];
           }
         }
+        cd[u].get(g);
+        if (silu) {
 #pragma unroll
-        for (int e = 0; e < 8; ++e) dba[e] += g[e];
-      }
-    } else {
-      sw[W - 1] = -2;                                   // past the end: matches no document
-#pragma unroll
-      for (int e = 0; e < 8; ++e) gw[W - 1][e] = 0.f;
-    }
-    // position tp = t − (W−1) has now seen every output step that read it: slot k of the windows is step tp + k, tap W−1−k
-    const int tp = t - (W - 1);
-    if (tp >= t0 && tp < t_end) {
-      float dxa[8];
-#pragma unroll
-      for (int e = 0; e < 8; ++e) dxa[e] = 0.f;
-#pragma unroll
-      for (int k = 0; k < W; ++k) {
-        if (sw[k] == sw[0]) {
-#pragma unroll
-          for (int e = 0; e < 8; ++e) dxa[e] += wk[W - 1 - k][e] * gw[k][e];
+          for (int e = 0; e < 8; ++e) g[e] *= dsilu_f(pre[e]);
         }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) gw[W - 1][e] = g[e];
+        if (t < t_end) {                                  // this block owns output step t: its weight / bias gradients
+#pragma unroll
+          for (int k = 0; k < W; ++k) {
+            if (sw[k] == sw[W - 1]) {
+#pragma unroll
+              for (int e = 0; e < 8; ++e) dwa[k][e] += g[e] * xw[k][e];
+            }
+          }
+#pragma unroll
+          for (int e = 0; e < 8; ++e) dba[e] += g[e];
+        }
+      } else {
+        sw[W - 1] = -2;                                   // past the end: matches no document
+#pragma unroll
+        for (int e = 0; e < 8; ++e) gw[W - 1][e] = 0.f;
       }
-      V8<T>::st(dx + base + static_cast<size_t>(tp) * C, dxa);
+      // position tp = t − (W−1) has now seen every output step that read it: slot k of the windows is step tp + k, tap W−1−k
+      const int tp = t - (W - 1);
+      if (tp >= t0 && tp < t_end) {
+        float dxa[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) dxa[e] = 0.f;
+#pragma unroll
+        for (int k = 0; k < W; ++k) {
+          if (sw[k] == sw[0]) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) dxa[e] += wk[W - 1 - k][e] * gw[k][e];
+          }
+        }
+        V8<T>::st(dx + base + static_cast<size_t>(tp) * C, dxa);
+      }
     }
-  }
   }
 #pragma unroll
   for (int e = 0; e < 8; ++e) {
@@ -294,12 +301,20 @@ template <typename T>
 static int conv_bwd_t(const void* dy, const void* x, const float* w, const float* bias, const int* seq_idx, void* dx, float* dw,
                       float* db, int B, int L, int C, int W, int silu, int xs, int dys, cudaStream_t st) {
   dim3 grid((C / 8 + 127) / 128, (L + CV_TSTEP_BWD - 1) / CV_TSTEP_BWD, B);
+  // fp32 with three or four taps: loading ahead takes a third CTA per SM its registers (246 against 165).  It loses where three would
+  // have held the grid in one wave, and where a few CTAs read from L2.  W 4, ms, ahead / not: 5 x 64 CTAs (L8192 C5120) 0.164 / 0.152,
+  // 16 CTAs (L1000 C2048) 0.075 / 0.073 packed; 132 CTAs 0.086 / 0.114, 512 0.206 / 0.271, 1024 0.344 / 0.426.
+  const long long ctas = static_cast<long long>(grid.x) * grid.y * grid.z;
+  const bool ahead = sizeof(T) == 2 || W == 2 || (ctas > 64 && (ctas <= 2 * 148 || ctas > 3 * 148));
+#define CONV_BWD(WW, AH) \
+  conv1d_bwd_kernel<T, WW, AH><<<grid, 128, 0, st>>>((const T*)dy, (const T*)x, w, bias, seq_idx, (T*)dx, dw, db, B, L, C, silu, xs, dys)
   switch (W) {
-    case 2: conv1d_bwd_kernel<T, 2><<<grid, 128, 0, st>>>((const T*)dy, (const T*)x, w, bias, seq_idx, (T*)dx, dw, db, B, L, C, silu, xs, dys); break;
-    case 3: conv1d_bwd_kernel<T, 3><<<grid, 128, 0, st>>>((const T*)dy, (const T*)x, w, bias, seq_idx, (T*)dx, dw, db, B, L, C, silu, xs, dys); break;
-    case 4: conv1d_bwd_kernel<T, 4><<<grid, 128, 0, st>>>((const T*)dy, (const T*)x, w, bias, seq_idx, (T*)dx, dw, db, B, L, C, silu, xs, dys); break;
+    case 2: CONV_BWD(2, true); break;
+    case 3: if (ahead) CONV_BWD(3, true); else if constexpr (sizeof(T) == 4) CONV_BWD(3, false); break;
+    case 4: if (ahead) CONV_BWD(4, true); else if constexpr (sizeof(T) == 4) CONV_BWD(4, false); break;
     default: return -1;
   }
+#undef CONV_BWD
   return cudaGetLastError() == cudaSuccess ? 0 : -3;
 }
 
