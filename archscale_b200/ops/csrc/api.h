@@ -198,6 +198,9 @@ int b200_gemm_rs_bf16(const void* A, const void* B, int M, int N, int K, int lda
 int b200_muon_momentum(const float* g, float* m, void* u, long long n, float mu, int nesterov, const float* gscale, cudaStream_t st);
 int b200_seg_update(int mode, float* x, const void* u, int u_dtype, long long n, const long long* bounds, const int* kidx, int nseg,
                     const float* coef, float* acc, cudaStream_t st);
+long long b200_axpy_sq_blocks(long long n);
+int b200_axpy_sq(float* x, const void* u, int u_dtype, long long n, const int* kidx, const float* coef, float* partial, float* acc,
+                 cudaStream_t st);
 int b200_adamw_fused(int mode, float* x, const float* g, float* m, float* v, float* u_out, long long n, float lr, float beta1,
                      float beta2, float eps, float wd, float bc1, float bc2, const float* gscale, float* acc, cudaStream_t st);
 
