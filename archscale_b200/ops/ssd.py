@@ -236,7 +236,7 @@ def ssd_scan(x, dt, A, B, C, D=None, seq_idx: Optional[torch.Tensor] = None, chu
     if fused:
         BN = Bb * nC
         y = _ChunkScanFn.apply(x, dt.view(Bb, nC, c, H), cs, Bh.reshape(BN, c, N), Ch.reshape(BN, c, N), wl.permute(0, 1, 3, 2),
-                               carry.permute(0, 1, 3, 2), keep, None if D is None else D.float().contiguous(),
+                               carry.permute(0, 1, 3, 2), keep, None if D is None else D.float().reshape(H).contiguous(),
                                bc.to(torch.int32).contiguous() if brk is not None else None)
         return y.reshape(Bb, Lp, H, P)[:, :L]
     if G == 1:
