@@ -5,6 +5,7 @@ import torch
 import torch.nn as nn
 
 from archscale_b200 import ops
+from archscale_b200.ops import gemm
 
 
 class Linear(nn.Linear):
@@ -21,6 +22,7 @@ class Linear(nn.Linear):
 
     mxfp8: bool = False
     nvfp4: bool = False
+    widen: bool = False         # odd feature counts on operands widened to a multiple of 8 (``ops.gemm.linear_widened``)
 
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         w, b = self.weight, self.bias
@@ -37,6 +39,8 @@ class Linear(nn.Linear):
         if self.mxfp8 and x.is_cuda:
             from archscale_b200.ops import mxfp8
             return mxfp8.linear_mxfp8(x, w, b)
+        if self.widen and b is None and gemm.widened_ok(x, w):
+            return gemm.linear_widened(x, w)
         return ops.linear(x, w, b)
 
 

@@ -20,20 +20,8 @@ import torch.nn.functional as F
 from archscale_b200 import ops
 from archscale_b200.models.layers import Linear
 from archscale_b200.models.norms import FusedRMSNorm
+from archscale_b200.ops import gemm
 from archscale_b200.utils.init import torch_default_init
-
-
-def _linear_any_width(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
-    """``x @ weightᵀ`` for feature counts that are no multiple of 8 (dt_rank = 124 at 1984 channels): both operands are widened
-    with zeros to the next multiple of 8, so that every row starts on a 16-byte boundary and the product and its two gradients
-    run the tcgen05 GEMM (unaligned rows leave the library only its sm_80 kernels with element-wise loads: 4.6 ms of a step
-    with five such layers at 4 x 4096 tokens).  The output keeps the widened feature count.  A few tokens stay on the library: there the extra
-    launches cost more than they give."""
-    if not (x.is_cuda and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and x.numel() // x.shape[-1] >= 2048
-            and (x.shape[-1] % 8 or weight.shape[0] % 8) and x.shape[-1] >= 64):
-        return F.linear(x, weight)
-    k, n = -x.shape[-1] % 8, -weight.shape[0] % 8
-    return ops.linear(F.pad(x, (0, k)) if k else x, F.pad(weight, (0, k, 0, n)))
 
 
 class Mamba(nn.Module):
@@ -58,6 +46,7 @@ class Mamba(nn.Module):
         self.conv1d = nn.Conv1d(self.d_inner, self.d_inner, bias=conv_bias, kernel_size=d_conv, groups=self.d_inner,
                                 padding=d_conv - 1, **fk)
         self.x_proj = Linear(self.d_inner, self.dt_rank + 2 * d_state, bias=False, **fk)
+        self.x_proj.widen = True
         self.dt_proj = Linear(self.dt_rank, self.d_inner, bias=True, **fk)
         self.A_log = nn.Parameter(torch.ones(self.d_inner, d_state, dtype=torch.float32, device=device))
         self.D = nn.Parameter(torch.ones(self.d_inner, dtype=torch.float32, device=device))
@@ -102,17 +91,12 @@ class Mamba(nn.Module):
                               seq_idx=seq_idx if self.use_cu_seqlen else None, activation="silu", channel_last=True)
         if pad_mask is not None:
             x = x * pad_mask.unsqueeze(-1).to(x.dtype)
-        widths = [self.dt_rank, self.d_state, self.d_state]
-        if sum(widths) % 8 and type(self.x_proj) is Linear and self.x_proj.bias is None and not (self.x_proj.mxfp8 or self.x_proj.nvfp4):
-            x_dbl = _linear_any_width(x, self.x_proj.weight.to(x.dtype))   # (B,L,R+2N), possibly a few zero columns more
-        else:
-            x_dbl = self.x_proj(x)
-        dt, Bm, Cm = torch.split(x_dbl, widths + ([x_dbl.shape[-1] - sum(widths)] if x_dbl.shape[-1] != sum(widths) else []), dim=-1)[:3]
+        x_dbl = self.x_proj(x)                                 # (B,L,R+2N)
+        dt, Bm, Cm = torch.split(x_dbl, [self.dt_rank, self.d_state, self.d_state], dim=-1)
         if self.jamba_norm:
             dt, Bm, Cm = self.dt_layernorm(dt), self.b_layernorm(Bm), self.c_layernorm(Cm)
-        dt = _linear_any_width(dt, self.dt_proj.weight.to(dt.dtype))       # bias is added inside the scan (fp32)
-        if dt.shape[-1] != self.d_inner:
-            dt = dt[..., :self.d_inner]
+        w_dt = self.dt_proj.weight.to(dt.dtype)                # bias is added inside the scan (fp32)
+        dt = gemm.linear_widened(dt, w_dt) if gemm.widened_ok(dt, w_dt) else F.linear(dt, w_dt)
         A = -torch.exp(self.A_log.float())
         y = ops.selective_scan(x, dt, A, Bm, Cm, self.D.float(), z=None if self.gmu_save else z,
                                delta_bias=self.dt_proj.bias.float(), delta_softplus=True, cu_seqlens=cu, channel_last=True)

@@ -200,6 +200,28 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     return torch.nn.functional.linear(x, weight, bias)
 
 
+def widened_ok(x: torch.Tensor, weight: torch.Tensor) -> bool:
+    """Whether :func:`linear_widened` pays: bf16 on the GPU, a feature count that is no multiple of 8, and enough tokens for the extra
+    launches.  x_proj and dt_proj of one layer, forward + backward, ms, library on the unaligned operands / widened: d_model 1984
+    0.110 / 0.107 at 1000 tokens, 0.163 / 0.123 at 2048, 0.706 / 0.380 at 16384; d_model 1088 0.080 / 0.086, 0.104 / 0.095,
+    0.353 / 0.309."""
+    g = getattr(weight, "_fsdp_group", None)
+    return (x.is_cuda and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16
+            and (x.shape[-1] % 8 != 0 or weight.shape[0] % 8 != 0) and x.shape[-1] >= 64 and x.numel() // x.shape[-1] >= 2048
+            and not (g is not None and getattr(g, "ag_pending", False)))
+
+
+def linear_widened(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
+    """``x @ weightᵀ`` for feature counts that are no multiple of 8 (dt_rank = 124 at 1984 channels): both operands are widened
+    with zeros to the next multiple of 8, so that every row of the product and of its two gradients starts on a 16-byte boundary
+    (unaligned rows leave the library only its sm_80 kernels with element-wise loads: 4.6 ms of a step with five such layers at
+    4 x 4096 tokens).  Token counts that are a multiple of 8 then run the tcgen05 GEMM, others the library on the widened operands.
+    The result is a view of the widened product's first columns."""
+    k, n = -x.shape[-1] % 8, -weight.shape[0] % 8
+    y = linear(torch.nn.functional.pad(x, (0, k)) if k else x, torch.nn.functional.pad(weight, (0, k, 0, n)))
+    return y[..., :weight.shape[0]] if n else y
+
+
 # ------------------------------------------------------------------------------------------ fused sibling projections
 def _adjacent(ts) -> bool:
     """True when the tensors are dense 2-D row blocks stored back to back (views of one flat parameter buffer)."""
