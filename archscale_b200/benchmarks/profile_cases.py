@@ -114,6 +114,30 @@ def case_conv1d():
     _run(once)
 
 
+def case_ssd():
+    from archscale_b200.ops.ssd import ssd_scan
+    B, L, H, P, N = 2, 4096, 62, 64, 128
+    mk = lambda *s: torch.randn(*s, device="cuda").bfloat16().requires_grad_()
+    x, Bm, Cm = mk(B, L, H, P), mk(B, L, 1, N), mk(B, L, 1, N)
+    dt, A = (torch.rand(B, L, H, device="cuda") * 0.1).requires_grad_(), (-torch.rand(H, device="cuda") - 0.1).requires_grad_()
+
+    def once():
+        y = ssd_scan(x, dt, A, Bm, Cm)
+        torch.autograd.grad(y, (x, dt, A, Bm, Cm), torch.ones_like(y))
+    _run(once)
+
+
+def case_gated_norm():
+    from archscale_b200.ops.norm import gated_rms_norm
+    x, z = (torch.randn(32768, 3968, device="cuda").bfloat16().requires_grad_() for _ in range(2))
+    w = torch.ones(3968, device="cuda").requires_grad_()
+
+    def once():
+        y = gated_rms_norm(x, w, z)
+        torch.autograd.grad(y, (x, w, z), torch.ones_like(y))
+    _run(once)
+
+
 def case_moe():
     from archscale_b200.ops.grouped_gemm import moe_ffn_cuda
     T, C, E, K, I = 16384, 1024, 64, 8, 256

@@ -187,7 +187,7 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
         umma_commit(s_full);
         return true;
       };
-      auto issue_dp = [&](int it) -> bool {   // dO of the tile is in shared memory (issue_dv waited for it, or the prologue)
+      auto issue_dp = [&](int it) -> bool {   // the caller has waited for dO (do_full) and for its columns (dq_empty)
         tc_fence_after();
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {

@@ -7,10 +7,10 @@
 // everything else has to stay below that.  With one state per thread (what this file did before) every step cost four
 // shared-memory loads, fifteen sixteenths of a shuffle and its selects per state.  Several states per thread share the loads of dt and dt·u, read B and C as vectors, do two states per instruction
 // (fma.rn.f32x2) and add most of the sum over states in registers; the remaining 16/NS lanes use a reduce-scatter over 16/NS
-// steps (lane q ends up with the total of step q).  Measured, one state -> several states per thread, ms:
-//   B4 L4096 Di3968   forward 1.17 -> 0.59   backward 3.91 -> 2.34        B1 L32768 Di3968  forward 4.05 -> 1.70
-//   B8 L4096 Di4096   forward 2.06 -> 1.07   backward 7.35 -> 4.67        B1 L8192 Di5120   forward 1.13 -> 0.56   backward 3.74 -> 2.15
-// (the B1 figures with the time axis split, see b200_selective_scan_parts).
+// steps (lane q ends up with the total of step q).  Measured (L2 flushed, both trees on one box), one state -> several per thread, ms:
+//   B4 L4096 Di3968   forward 1.17 -> 0.59   backward 3.89 -> 2.28        B1 L32768 Di3968  forward 4.05 -> 1.66   backward 8.44 -> 5.78
+//   B8 L4096 Di4096   forward 2.07 -> 1.06   backward 7.29 -> 4.48        B1 L8192 Di5120   forward 1.15 -> 0.55   backward 3.70 -> 2.09
+// (the B1 forwards with the time axis split, see b200_selective_scan_parts).
 //
 // The forward stages tiles of 64 steps through shared memory (the next tile's loads are in flight during the steps) and
 // stores the state entering every 32-step half tile (fp32, L/32 × Di × 16).  The backward walks 32-step tiles in reverse,
@@ -290,9 +290,9 @@ sscan_fwd_kernel(const T* __restrict__ u, int su, const T* __restrict__ delta, i
 }
 
 // MINB: resident CTAs per SM the registers are limited for.  2 (255 registers, hardly any spill) where the grid leaves no more
-// to an SM anyway, else 4 (128 registers).  ms with 2 / 3 / 4: B4 L4096 Di3968 (992 CTAs) 2.91 / 2.84 / 2.34, B8 L4096 Di4096
-// 5.09 / 5.10 / 4.67, B2 L4096 Di4096 (512) 1.51 / 1.92 / 1.32, B1 L8192 Di5120 (320) 2.59 / 2.14 / 2.15, B1 L32768 Di3968 (248)
-// 5.85 / 6.75 / 7.13.
+// to an SM anyway, else 4 (128 registers).  ms with 2 / 3 / 4: B4 L4096 Di3968 (992 CTAs) 2.72 / 2.80 / 2.27, B8 L4096 Di4096
+// 5.04 / 4.91 / 4.47, B2 L4096 Di4096 (512) 1.46 / 1.80 / 1.27, B1 L8192 Di5120 (320) 2.54 / 2.04 / 2.09, B1 L32768 Di3968 (248)
+// 5.77 / 6.69 / 7.01.
 template <typename T, bool RESET, bool GATE, int MINB>
 __global__ void __launch_bounds__(128, MINB)
 sscan_bwd_kernel(const T* __restrict__ dy, int sdy, const T* __restrict__ u, int su, const T* __restrict__ delta, int sd,
@@ -527,7 +527,10 @@ static void launch_sscan_fwd(const void* u, int su, const void* delta, int sd, c
 
 // Parts of the sequence that the forward scan runs side by side.  With few channels the steps cost their latency: splitting the
 // time costs a second pass over the exponentials but multiplies the warps.  Parts are kept at 512 steps or more.  Whole -> split,
-// ms: B1 L32768 Di3968 2.73 -> 1.70, B1 L8192 Di5120 0.76 -> 0.56, but B2 L4096 Di4096 0.432 -> 0.462: the line lies at B·Di = 8192.
+// ms: B·Di 4096: L1536 0.112 -> 0.106, L1600 0.116 -> 0.119, L2048 0.153 -> 0.130, L4096 0.310 -> 0.228; B·Di 7936: L1536 0.156 -> 0.198,
+// L2048 0.207 -> 0.226, L4096 0.413 -> 0.432, L8192 0.825 -> 0.821; B·Di 8192: L4096 0.412 -> 0.447, L32768 3.30 -> 3.52; B1 L32768 Di3968
+// 2.73 -> 1.66.  The line lies at B·Di = 8192; short sequences just below it would be better off whole (every one of these is ahead of
+// one state per thread: 0.239 for B·Di 7936 L1536).
 extern "C" int b200_selective_scan_parts(int B, int L, int Di) {
   const long long width = static_cast<long long>(B) * Di;
   if (width <= 0 || width >= 8192) return 1;
@@ -549,7 +552,9 @@ extern "C" int b200_selective_scan_fwd(const void* u, int su, const void* delta,
                                        float* scratch, cudaStream_t st) {
   if (Di % SS_C || parts < 1 || (parts > 1 && !scratch)) return -1;
   if (B * L == 0) return 0;
-  // four states per thread need B·Di/8 warps to fill the 592 schedulers about three deep; below that two states per thread
+  // four states per thread leave B·Di/8 warps for 592 schedulers; with fewer than about two and a half each, two states per thread.
+  // ms, two / four: B·Di 6144 L1000 0.086 / 0.094, 8192 L4096 0.412 / 0.382, 10240 L1000 0.120 / 0.120, 11904 L4096 0.542 / 0.478,
+  // 12288 L1000 0.139 / 0.124, 15872 L4096 0.627 / 0.581: the true crossing is nearer to 8192 than to 12288.
   const bool ns4 = parts > 1 || static_cast<long long>(B) * Di >= 12288;
   auto run = dtype == 1 ? (ns4 ? launch_sscan_fwd<__nv_bfloat16, 4> : launch_sscan_fwd<__nv_bfloat16, 2>)
                         : (ns4 ? launch_sscan_fwd<float, 4> : launch_sscan_fwd<float, 2>);
