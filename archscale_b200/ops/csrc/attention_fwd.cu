@@ -63,8 +63,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   uint64_t* s_full = bars + 7;        // [2]
   uint64_t* s_empty = bars + 9;       // [2]
   uint64_t* p_full = bars + 11;       // [2]
-  uint64_t* p_empty = bars + 13;      // [2]
-  uint64_t* o_done = bars + 15;       // 1
+  uint64_t* p_empty = bars + 13;      // [2]  P buffer free: P·V of its tile has completed
   uint64_t* v_empty = bars + 16;      // [2]  V stage free: P·V of its tile has completed
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + 18);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr + 1);
@@ -93,7 +92,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       mbar_init(&k_full[s], 1); mbar_init(&v_full[s], 1); mbar_init(&k_empty[s], 1); mbar_init(&v_empty[s], 1);
       mbar_init(&s_full[s], 1); mbar_init(&s_empty[s], 4); mbar_init(&p_full[s], 4); mbar_init(&p_empty[s], 1);
     }
-    mbar_init(o_done, 1);
     *abort_flag = 0;
     mbar_fence_init();
     tma_prefetch_desc(&tmap_q); tma_prefetch_desc(&tmap_k); tma_prefetch_desc(&tmap_v);
@@ -170,7 +168,6 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         }
         umma_commit(&v_empty[st]);
         umma_commit(&p_empty[st]);
-        umma_commit(o_done);
       }
     }
   } else {
@@ -217,8 +214,10 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
         const float m_new = fmaxf(m_used, mx);
         const float alpha = exp2f(m_used - m_new);
         if (t > 0) {
-          // O of all previous tiles must be complete before it is rescaled: wait for P·V of tile t−1
-          if (!mbar_wait(o_done, (t - 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) goto done;
+          // O of all previous tiles must be complete before it is rescaled: wait for P·V of tile t−1, on the barrier of its P
+          // buffer.  (This thread saw that barrier's phase of tile t−3 before it wrote P of t−1, so the parity is not
+          // ambiguous; one barrier flipped by every tile is, with two tiles open.)
+          if (!mbar_wait(&p_empty[st ^ 1], ((t - 1) >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) goto done;
           tc_fence_after();
 #pragma unroll
           for (int c = 0; c < D / 32; ++c) {
@@ -264,7 +263,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
     }
     // epilogue: O / l, LSE
     if (n_tiles > 0) {
-      if (!mbar_wait(o_done, (n_tiles - 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) goto done;
+      if (!mbar_wait(&p_empty[(n_tiles - 1) & 1], ((n_tiles - 1) >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) goto done;
       tc_fence_after();
     }
     const float inv_l = l_sum > 0.f ? 1.f / l_sum : 0.f;
