@@ -94,6 +94,9 @@ int b200_grouped_gemm_bf16(int kind, const void* A, const void* B, void* out, co
 int b200_attn_fwd(const void* q, const void* k, const void* v, void* out, float* lse, const int* row_start, int B, int T,
                   int H, int G, int D, int window_left, float scale, int* status, cudaStream_t stream);
 
+// The forward with two query tiles per CTA (attention_fwd_pair.cu); b200_attn_fwd checks the arguments and calls it.
+int b200_attn_fwd_pair(const void* q, const void* k, const void* v, void* out, float* lse, const int* row_start, int B, int T,
+                       int H, int G, int D, int window_left, float scale, int* status, cudaStream_t stream);
 // Two-stream variant of the forward kernel (attention_fwd2s.cu); same contract.  ARCHSCALE_B200_ATTN_FWD=2stream routes
 // b200_attn_fwd to it.  set_trace: development aid, 16×64 int64 clock stamps of the first CTA, null = off.
 int b200_attn_fwd_2s(const void* q, const void* k, const void* v, void* out, float* lse, const int* row_start, int B, int T,

@@ -1,4 +1,5 @@
-// Causal / sliding-window / packed-varlen attention forward on tcgen05 (GQA, head_dim 64 or 128).
+// Causal / sliding-window / packed-varlen attention forward on tcgen05 (GQA, head_dim 64 or 128): the kernel for small grids
+// (attention_fwd_pair.cu is the one for the others) and the entry point.
 //
 // One CTA per (query tile of 128 rows, head, batch); 224 threads:
 //   warp 0      TMA: Q once, then K/V tiles of 128 keys through a 2-stage ring
@@ -68,7 +69,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + 18);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   // heavy (late) query tiles first: better tail behaviour under causal masking
   const int n_qt = (p.T + ATT_BM - 1) / ATT_BM;
   const int qt = n_qt - 1 - static_cast<int>(blockIdx.x);
@@ -84,7 +85,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   const int lo_first = lo_of(q0);
   const int j_begin = lo_first / ATT_BN;
   const int j_end = r_last / ATT_BN + 1;          // exclusive
-  const int n_tiles = j_end - j_begin;
+  const int n_tiles = __shfl_sync(0xffffffffu, j_end - j_begin, 0);
 
   if (threadIdx.x == 0) {
     mbar_init(q_full, 1);
@@ -100,7 +101,7 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_ptr;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr, 0);
   const uint32_t T_S0 = tmem_base, T_P0 = tmem_base + 256, T_O = tmem_base + 384;
 
   if (warp == 0) {
@@ -126,48 +127,48 @@ attn_fwd_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constan
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {                                              // the whole warp, converged (umma_*_warp elects a lane)
       constexpr uint32_t idesc_s = make_idesc_bf16(ATT_BM, ATT_BN, 0, 0);       // S = Q·Kᵀ  (both K-major)
-      if (!mbar_wait(q_full, 0, abort_flag, p.status, STATUS_TIMEOUT_FULL)) goto done;
+      if (!mbar_wait_warp(q_full, 0, abort_flag, p.status, STATUS_TIMEOUT_FULL)) goto done;
       auto issue_s = [&](int t) -> bool {
         const int st = t & 1; const uint32_t ph = (t >> 1) & 1;
-        if (!mbar_wait(&k_full[st], ph, abort_flag, p.status, STATUS_TIMEOUT_FULL)) return false;
-        if (!mbar_wait(&s_empty[st], ph ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY)) return false;
+        if (!mbar_wait_warp(&k_full[st], ph, abort_flag, p.status, STATUS_TIMEOUT_FULL)) return false;
+        if (!mbar_wait_warp(&s_empty[st], ph ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY)) return false;
         tc_fence_after();
         const uint32_t sk = smem_u32(skv + st * 2 * SM::KV_BYTES);
         const uint32_t sqa = smem_u32(sq);
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
           const uint32_t off = (k / 4) * CHUNK_BYTES + (k % 4) * 32;
-          umma_bf16(T_S0 + st * 128, make_smem_desc(sqa + off, 16, 1024), make_smem_desc(sk + off, 16, 1024), idesc_s,
-                    k != 0 ? 1u : 0u);
+          umma_bf16_warp(T_S0 + st * 128, make_smem_desc(sqa + off, 16, 1024), make_smem_desc(sk + off, 16, 1024), idesc_s,
+                         k != 0 ? 1u : 0u);
         }
-        umma_commit(&s_full[st]);
-        umma_commit(&k_empty[st]);
+        umma_commit_warp(&s_full[st]);
+        umma_commit_warp(&k_empty[st]);
         return true;
       };
-      // One thread can issue a tcgen05.mma only every ~100 cycles: S and P·V are issued by two threads (this one and warp
-      // ATT_PV_WARP) so that neither stream waits behind the other's issue slots.  s_empty / p_empty order the buffer reuse.
+      // S and P·V are issued by two warps (this one and ATT_PV_WARP) so that neither waits behind the other's barriers;
+      // s_empty / p_empty order the buffer reuse.
       for (int t = 0; t < n_tiles; ++t)
         if (!issue_s(t)) goto done;
     }
   } else if (warp == ATT_PV_WARP) {
-    if (lane == 0) {
+    {
       constexpr uint32_t idesc_o = make_idesc_bf16(ATT_BM, D, 0, 1);            // O += P·V  (V is N-major)
       for (int t = 0; t < n_tiles; ++t) {
         const int st = t & 1; const uint32_t ph = (t >> 1) & 1;
-        if (!mbar_wait(&v_full[st], ph, abort_flag, p.status, STATUS_TIMEOUT_FULL)) goto done;
-        if (!mbar_wait(&p_full[st], ph, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) goto done;
+        if (!mbar_wait_warp(&v_full[st], ph, abort_flag, p.status, STATUS_TIMEOUT_FULL)) goto done;
+        if (!mbar_wait_warp(&p_full[st], ph, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) goto done;
         tc_fence_after();
         const uint32_t sv = smem_u32(skv + st * 2 * SM::KV_BYTES + SM::KV_BYTES);
 #pragma unroll
         for (int k = 0; k < ATT_BN / 16; ++k) {
           // A: P columns (two bf16 per 32-bit column → 8 columns per K=16); B: 16 key rows = 2048 bytes further
-          umma_bf16_ts(T_O, T_P0 + st * 64 + k * 8, make_smem_desc(sv + k * 2048, CHUNK_BYTES, 1024), idesc_o,
-                       (t | k) != 0 ? 1u : 0u);
+          umma_bf16_ts_warp(T_O, T_P0 + st * 64 + k * 8, make_smem_desc(sv + k * 2048, CHUNK_BYTES, 1024), idesc_o,
+                            (t | k) != 0 ? 1u : 0u);
         }
-        umma_commit(&v_empty[st]);
-        umma_commit(&p_empty[st]);
+        umma_commit_warp(&v_empty[st]);
+        umma_commit_warp(&p_empty[st]);
       }
     }
   } else {
@@ -334,6 +335,11 @@ extern "C" int b200_attn_fwd(const void* q, const void* k, const void* v, void* 
     if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return -5;
     ctx_bound = true;
   }
+  // Two tiles per CTA where that leaves no SM without work: measured (ms, one tile / two tiles per CTA, D 128, causal)
+  // B8 T4096 H16 G4 0.641 / 0.481, B3 T2731 H16 G4 0.150 / 0.108, B1 T4096 H40 G40 0.232 / 0.223, B3 T1000 H12 G4 (288 tiles)
+  // 0.034 / 0.031; at 256 tiles 0.069 / 0.072 and 0.031 / 0.029, at 128 tiles 0.029 / 0.041.
+  if (static_cast<long long>(B) * H * ((T + ATT_BM - 1) / ATT_BM) > 256)
+    return b200_attn_fwd_pair(q, k, v, out, lse, row_start, B, T, H, G, D, window_left, scale, status, stream);
   CUtensorMap tq, tk, tv;
   int rc = make_tmap_2d_bf16(&tq, q, static_cast<uint64_t>(H) * D, static_cast<uint64_t>(B) * T, static_cast<uint64_t>(H) * D, 64, 128);
   if (rc) return rc;

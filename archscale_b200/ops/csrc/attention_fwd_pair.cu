@@ -233,7 +233,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       constexpr uint32_t idesc_o = make_idesc_bf16(AP_BM, D, 0, 1);           // O += P·V  (V is N-major)
       const uint32_t sqa = smem_u32(sq), skva = smem_u32(skv);
       int idx = blockIdx.x;
-      int n = pair_item(p, idx).n;
+      int n = __shfl_sync(0xffffffffu, pair_item(p, idx).n, 0);       // (shuffles make warp-uniform what they return)
       uint32_t slot = 0, sph = 0;                      // ring position of the next tile to be waited for
       uint32_t step = 0;                               // tiles done by this CTA: phase of p_part / p_full
       auto advance = [&]() { if (++slot == NS) { slot = 0; sph ^= 1; } };
@@ -269,7 +269,7 @@ attn_fwd_pair_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
           const bool last = j == n - 1;
           if (last) {
             if (!next_item_warp(i, idx_next)) goto done;
-            if (idx_next >= 0) n_next = pair_item(p, idx_next).n;
+            if (idx_next >= 0) n_next = __shfl_sync(0xffffffffu, pair_item(p, idx_next).n, 0);
           }
           const bool more = !last || idx_next >= 0;    // there is another S to issue after this P·V
           const uint32_t vslot = slot, vph = sph;

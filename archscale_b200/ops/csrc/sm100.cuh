@@ -82,6 +82,11 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   }
 }
 
+// The same by a whole converged warp; the answer is warp-uniform (a vote), so the control flow that depends on it is too.
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status, int code) {
+  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag, status, code));
+}
+
 // The same bounded wait for roles that are not on the critical path (loaders, read-out warps): it sleeps between polls,
 // so the polling warp leaves the issue slots of its scheduler to the warps that compute.
 __device__ __forceinline__ bool mbar_wait_relaxed(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int* status,
@@ -180,10 +185,23 @@ __device__ __forceinline__ void umma_bf16_ts(uint32_t tmem_d, uint32_t tmem_a, u
       "}\n" ::"r"(tmem_d), "r"(tmem_a), "l"(desc_b), "r"(idesc), "r"(accumulate)
       : "memory");
 }
+// The same issued by a whole converged warp (one lane executes).  In warp-uniform control flow the operands stay in uniform
+// registers and an MMA issues in less than the pipe needs for it; from inside a branch of one lane it took ≈100 cycles
+// (attention forward, M128 N128 K16: 65 of pipe time).
+__device__ __forceinline__ void umma_bf16_warp(uint32_t tmem_d, uint64_t desc_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  if (elect_one_sync()) umma_bf16(tmem_d, desc_a, desc_b, idesc, accumulate);
+}
+__device__ __forceinline__ void umma_bf16_ts_warp(uint32_t tmem_d, uint32_t tmem_a, uint64_t desc_b, uint32_t idesc, uint32_t accumulate) {
+  if (elect_one_sync()) umma_bf16_ts(tmem_d, tmem_a, desc_b, idesc, accumulate);
+}
 // mbarrier arrives once all previously issued tcgen05.mma of this thread have completed.
 __device__ __forceinline__ void umma_commit(uint64_t* bar) {
   asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
                : "memory");
+}
+
+__device__ __forceinline__ void umma_commit_warp(uint64_t* bar) {   // by the lane that umma_*_warp elects
+  if (elect_one_sync()) umma_commit(bar);
 }
 
 // 32 lanes × 32 consecutive fp32 columns → 32 registers per thread (thread t = lane t of the warp's quarter)

@@ -29,7 +29,19 @@ CASES = [
 ]
 
 
-@pytest.mark.parametrize("B,T,H,G,D,win,cu", CASES)
+# more than 256 query tiles: the forward with two tiles per CTA
+PAIR_CASES = [
+    (8, 257, 16, 4, 128, -1, None),         # one row in the last block
+    (7, 385, 16, 16, 64, -1, None),         # one head per KV head: pairs of row blocks, an even number of them
+    (4, 777, 40, 40, 128, 200, None),       # an odd number of row blocks, and a window
+    (5, 1000, 12, 4, 64, 128, None),        # three heads per KV head; the window leaves the first tile of some rows empty
+    (1, 4000, 12, 2, 128, -1, None),        # more key tiles than ring slots
+    (1, 2500, 16, 4, 128, -1, [0, 3, 1150, 1151, 2433, 2500]),   # packed documents
+    (1, 2500, 16, 8, 64, 255, [0, 130, 1920, 2500]),             # packed + window
+]
+
+
+@pytest.mark.parametrize("B,T,H,G,D,win,cu", CASES + PAIR_CASES)
 def test_attention_forward(B, T, H, G, D, win, cu):
     ext = backend.require_extension()
     torch.manual_seed(0)
