@@ -113,7 +113,7 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + 19);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const bool traced = blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0 && lane == 0 && (warp == 1 || warp == 4 || warp == 12);
   // key tile on the slow grid axis: CTAs start in order of decreasing work under a causal mask (tile 0 sees every query)
   const int jt = blockIdx.y, g = blockIdx.x % p.G, b = blockIdx.x / p.G;
@@ -125,7 +125,7 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   if (p.doc_end) r_hi = min(r_hi, p.doc_end[static_cast<size_t>(b) * p.T + k_last] - 1);
   const int i_begin = k0 / B1T, i_end = r_hi / B1T + 1;
   const int tiles_per_head = i_end - i_begin;
-  const int n_iter = tiles_per_head * group;           // ≥ 1
+  const int n_iter = __shfl_sync(0xffffffffu, tiles_per_head * group, 0);   // ≥ 1; warp-uniform for the MMA warp
 
   if (threadIdx.x == 0) {
     mbar_init(kv_full, 1);
@@ -141,7 +141,7 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_ptr;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr, 0);
   const uint32_t T_S = tmem_base, T_DP = tmem_base + 128, T_DV = tmem_base + 256, T_DK = tmem_base + 384;
 
   if (warp < 4) {
@@ -167,24 +167,24 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 #pragma unroll
         for (int c = 0; c < DC; ++c) tma_load_2d(sdo + c * CHUNK_BYTES, &tmap_do, do_full, hq * D + c * 64, b * p.T + q0);
       }
-    } else if (warp == 1 && lane == 0) {
-      // ---------------------------------------------------------------- MMA (one thread, dependency order)
+    } else if (warp == 1) {
+      // ---------------------------------------------------------------- MMA (the whole warp converged, one lane elected per instruction; dependency order)
       constexpr uint32_t idesc_s = make_idesc_bf16(B1T, B1T, 0, 0);        // Sᵀ = K·Qᵀ, dPᵀ = V·dOᵀ (all K-major)
       constexpr uint32_t idesc_acc = make_idesc_bf16(B1T, D, 0, 1);       // dV, dK: B = dO / Q read N-major
       constexpr uint32_t idesc_dq = make_idesc_bf16(B1T, D, 1, 1);        // dQ_i = dS·K: A = dSᵀ tile read MN-major, B = K N-major
-      if (!mbar_wait(kv_full, 0, abort_flag, p.status, STATUS_TIMEOUT_FULL)) goto done;
+      if (!mbar_wait_warp(kv_full, 0, abort_flag, p.status, STATUS_TIMEOUT_FULL)) goto done;
       const uint32_t ska = smem_u32(sk), sva = smem_u32(sv), sdoa = smem_u32(sdo), sdsa = smem_u32(sds);
       auto issue_s = [&](int it) -> bool {
         const int st = it & 1;
-        if (!mbar_wait(&q_full[st], (it >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_FULL)) return false;
+        if (!mbar_wait_warp(&q_full[st], (it >> 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_FULL)) return false;
         tc_fence_after();
         const uint32_t sqa = smem_u32(sqr + st * SM::TILE);
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
           const uint32_t off = (k / 4) * CHUNK_BYTES + (k % 4) * 32;
-          umma_bf16(T_S, make_smem_desc(ska + off, 16, 1024), make_smem_desc(sqa + off, 16, 1024), idesc_s, k != 0);
+          umma_bf16_warp(T_S, make_smem_desc(ska + off, 16, 1024), make_smem_desc(sqa + off, 16, 1024), idesc_s, k != 0);
         }
-        umma_commit(s_full);
+        umma_commit_warp(s_full);
         return true;
       };
       auto issue_dp = [&](int it) -> bool {   // the caller has waited for dO (do_full) and for its columns (dq_empty)
@@ -192,59 +192,59 @@ attn_bwd1_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_consta
 #pragma unroll
         for (int k = 0; k < D / 16; ++k) {
           const uint32_t off = (k / 4) * CHUNK_BYTES + (k % 4) * 32;
-          umma_bf16(T_DP, make_smem_desc(sva + off, 16, 1024), make_smem_desc(sdoa + off, 16, 1024), idesc_s, k != 0);
+          umma_bf16_warp(T_DP, make_smem_desc(sva + off, 16, 1024), make_smem_desc(sdoa + off, 16, 1024), idesc_s, k != 0);
         }
-        umma_commit(dp_full);
+        umma_commit_warp(dp_full);
         return true;
       };
       auto issue_dv = [&](int it) -> bool {   // dV += Pᵀ·dO
-        if (!mbar_wait(p_ready, it & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) return false;
+        if (!mbar_wait_warp(p_ready, it & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) return false;
         tc_fence_after();
 #pragma unroll
         for (int k = 0; k < B1T / 16; ++k)     // packed Pᵀ: 16 queries = 8 columns; group c's 64 queries start at column 64c
-          umma_bf16_ts(T_DV, T_S + (k >> 2) * 64 + (k & 3) * 8, make_smem_desc(sdoa + k * 2048, CHUNK_BYTES, 1024), idesc_acc,
+          umma_bf16_ts_warp(T_DV, T_S + (k >> 2) * 64 + (k & 3) * 8, make_smem_desc(sdoa + k * 2048, CHUNK_BYTES, 1024), idesc_acc,
                        (it | k) != 0);
         return true;
       };
       // prologue: Sᵀ_0, dPᵀ_0, dV_0, Sᵀ_1
       if (!issue_s(0)) goto done;
-      if (!mbar_wait(do_full, 0, abort_flag, p.status, STATUS_TIMEOUT_FULL)) goto done;
+      if (!mbar_wait_warp(do_full, 0, abort_flag, p.status, STATUS_TIMEOUT_FULL)) goto done;
       issue_dp(0);
       if (!issue_dv(0)) goto done;
-      umma_commit(do_empty);                   // dPᵀ_0 and dV_0 have read dO_0
+      umma_commit_warp(do_empty);                   // dPᵀ_0 and dV_0 have read dO_0
       if (1 < n_iter && !issue_s(1)) goto done;
       for (int it = 0; it < n_iter; ++it) {
         const int st = it & 1; const uint32_t ph = it & 1;
         const uint32_t sqa = smem_u32(sqr + st * SM::TILE);
-        if (!mbar_wait(ds_ready, ph, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) goto done;
+        if (!mbar_wait_warp(ds_ready, ph, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) goto done;
         B1_TRACE(0, it);
         tc_fence_after();
 #pragma unroll
         for (int k = 0; k < B1T / 16; ++k)     // dQ_i = dS·K.  A: the dSᵀ tile MN-major (M = queries, K = keys): 16 keys = 2048 bytes
-          umma_bf16(T_DP, make_smem_desc(sdsa + k * 2048, CHUNK_BYTES, 1024), make_smem_desc(ska + k * 2048, CHUNK_BYTES, 1024),
+          umma_bf16_warp(T_DP, make_smem_desc(sdsa + k * 2048, CHUNK_BYTES, 1024), make_smem_desc(ska + k * 2048, CHUNK_BYTES, 1024),
                     idesc_dq, k != 0);
-        umma_commit(dq_full);
+        umma_commit_warp(dq_full);
 #pragma unroll
         for (int k = 0; k < B1T / 16; ++k)     // dK += dSᵀ·Q.  A: the tile K-major (K = queries): chunk k/4, 32 bytes per 16 queries
-          umma_bf16(T_DK, make_smem_desc(sdsa + (k >> 2) * CHUNK_BYTES + (k & 3) * 32, 16, 1024),
+          umma_bf16_warp(T_DK, make_smem_desc(sdsa + (k >> 2) * CHUNK_BYTES + (k & 3) * 32, 16, 1024),
                     make_smem_desc(sqa + k * 2048, CHUNK_BYTES, 1024), idesc_acc, (it | k) != 0);
-        umma_commit(&q_empty[st]);
-        umma_commit(ds_free);
+        umma_commit_warp(&q_empty[st]);
+        umma_commit_warp(ds_free);
         B1_TRACE(1, it);
         if (it + 1 < n_iter) {
-          if (!mbar_wait(do_full, (it + 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_FULL)) goto done;
+          if (!mbar_wait_warp(do_full, (it + 1) & 1, abort_flag, p.status, STATUS_TIMEOUT_FULL)) goto done;
           // dPᵀ of the next tile goes into the columns of dQ_i: wait for the read-out
-          if (!mbar_wait(dq_empty, ph, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY)) goto done;
+          if (!mbar_wait_warp(dq_empty, ph, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY)) goto done;
           B1_TRACE(2, it);
           issue_dp(it + 1);
           B1_TRACE(3, it);
           if (!issue_dv(it + 1)) goto done;
-          umma_commit(do_empty);
+          umma_commit_warp(do_empty);
           if (it + 2 < n_iter && !issue_s(it + 2)) goto done;
           B1_TRACE(4, it);
         }
       }
-      umma_commit(acc_done);
+      umma_commit_warp(acc_done);
     } else if (warp >= 2) {
       // ---------------------------------------------------------------- per-query statistics, one tile ahead of the conversion
       const int t64 = (warp - 2) * 32 + lane;
