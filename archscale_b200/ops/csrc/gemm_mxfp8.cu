@@ -65,6 +65,14 @@ __device__ __forceinline__ void umma_mxf8(uint32_t tmem_d, uint64_t da, uint64_t
       "}\n" ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(tsfa), "r"(tsfb)
       : "memory");
 }
+// by a whole converged warp: see umma_bf16_warp
+__device__ __forceinline__ void tmem_cp_sf_warp(uint32_t taddr, uint64_t desc) {
+  if (elect_one_sync()) tmem_cp_sf(taddr, desc);
+}
+__device__ __forceinline__ void umma_mxf8_warp(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t tsfa, uint32_t tsfb,
+                                               uint32_t accumulate) {
+  if (elect_one_sync()) umma_mxf8(tmem_d, da, db, idesc, tsfa, tsfb, accumulate);
+}
 // e4m3 × e4m3, E8M0 scales, fp32 accumulate, both operands K-major
 __host__ __device__ constexpr uint32_t make_idesc_mxf8(int M, int N) {
   return (static_cast<uint32_t>(N >> 3) << 17) | (1u << 23) | (static_cast<uint32_t>(M >> 4) << 24);
@@ -82,7 +90,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   uint64_t* tmem_empty = bars + 2 * QSTAGES + 2;
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + 2 * QSTAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int cta = blockIdx.x, n_cta = gridDim.x;
   const int num_m = (p.M + QBM - 1) / QBM, num_n = (p.N + QBN - 1) / QBN;
   const int num_tiles = num_m * num_n;
@@ -101,7 +109,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_ptr;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr, 0);
 
   auto tile_coords = [&](int t, int& m0, int& n0) {
     const int per_group = Q_GROUP_M * num_n;
@@ -134,39 +142,39 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {                                              // the whole warp, converged: one lane is elected per instruction
       constexpr uint32_t idesc0 = make_idesc_mxf8(QBM, QBN);
       int stage = 0; uint32_t phase = 0;
       int it = 0;
       for (int t = cta; t < num_tiles; t += n_cta, ++it) {
         const int acc = it & 1; const uint32_t acc_phase = (it >> 1) & 1;
-        if (!mbar_wait(&tmem_empty[acc], acc_phase ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY)) goto done;
+        if (!mbar_wait_warp(&tmem_empty[acc], acc_phase ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY)) goto done;
         tc_fence_after();
         int m0, n0; tile_coords(t, m0, n0);
         const uint32_t d_tmem = tmem_base + acc * QBN;
         const uint32_t tsfa = tmem_base + Q_TMEM_SFA;
         const uint32_t tsfb = tmem_base + Q_TMEM_SFB + ((n0 >> 5) & 3);   // 0 or 2: rows 64.. of the first chunk
         for (int kb = 0; kb < KC; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag, p.status, STATUS_TIMEOUT_FULL)) goto done;
+          if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag, p.status, STATUS_TIMEOUT_FULL)) goto done;
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * QSTAGE_BYTES);
-          tmem_cp_sf(tmem_base + Q_TMEM_SFA, make_sf_desc(sa + QSFA_OFF));
-          tmem_cp_sf(tmem_base + Q_TMEM_SFB, make_sf_desc(sa + QSFB_OFF));
-          tmem_cp_sf(tmem_base + Q_TMEM_SFB + 4, make_sf_desc(sa + QSFB_OFF + 512));
+          tmem_cp_sf_warp(tmem_base + Q_TMEM_SFA, make_sf_desc(sa + QSFA_OFF));
+          tmem_cp_sf_warp(tmem_base + Q_TMEM_SFB, make_sf_desc(sa + QSFB_OFF));
+          tmem_cp_sf_warp(tmem_base + Q_TMEM_SFB + 4, make_sf_desc(sa + QSFB_OFF + 512));
           const uint64_t da = make_smem_desc(sa, 16, 1024);
           const uint64_t db = make_smem_desc(sa + QA_BYTES, 16, 1024);
 #pragma unroll
           for (uint32_t k = 0; k < QBK / 32; ++k) {
             // K-block k of the stage: operands advance 32 bytes, the scale of byte k of each column is used
             const uint32_t idesc = idesc0 | (k << 4) | (k << 29);
-            umma_mxf8(d_tmem, da + static_cast<uint64_t>(k * 2), db + static_cast<uint64_t>(k * 2), idesc,
+            umma_mxf8_warp(d_tmem, da + static_cast<uint64_t>(k * 2), db + static_cast<uint64_t>(k * 2), idesc,
                       tsfa | (k << 30), tsfb | (k << 30), (kb != 0 || k != 0) ? 1u : 0u);
           }
-          umma_commit(&empty_bar[stage]);
+          umma_commit_warp(&empty_bar[stage]);
           if (++stage == QSTAGES) { stage = 0; phase ^= 1; }
         }
-        if (KC == 0) mbar_arrive(&tmem_full[acc]);
-        else umma_commit(&tmem_full[acc]);
+        if (KC == 0) { if (lane == 0) mbar_arrive(&tmem_full[acc]); }
+        else umma_commit_warp(&tmem_full[acc]);
       }
     }
   } else {
@@ -412,6 +420,10 @@ __device__ __forceinline__ void umma_nvf4(uint32_t tmem_d, uint64_t da, uint64_t
       "}\n" ::"r"(tmem_d), "l"(da), "l"(db), "r"(idesc), "r"(accumulate), "r"(tsfa), "r"(tsfb)
       : "memory");
 }
+__device__ __forceinline__ void umma_nvf4_warp(uint32_t tmem_d, uint64_t da, uint64_t db, uint32_t idesc, uint32_t tsfa, uint32_t tsfb,
+                                               uint32_t accumulate) {
+  if (elect_one_sync()) umma_nvf4(tmem_d, da, db, idesc, tsfa, tsfb, accumulate);
+}
 // e2m1 × e2m1 (format code 1 in both operand fields), unsigned E4M3 scales (scale-format bit clear), fp32 accumulate
 __host__ __device__ constexpr uint32_t make_idesc_nvf4(int M, int N) {
   return (1u << 7) | (1u << 10) | (static_cast<uint32_t>(N >> 3) << 17) | (static_cast<uint32_t>(M >> 4) << 24);
@@ -430,7 +442,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   uint64_t* tmem_empty = bars + 2 * FSTAGES + 2;
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + 2 * FSTAGES + 4);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr + 1);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const int cta = blockIdx.x, n_cta = gridDim.x;
   const int num_m = (p.M + QBM - 1) / QBM, num_n = (p.N + QBN - 1) / QBN;
   const int num_tiles = num_m * num_n;
@@ -449,7 +461,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem_base = *tmem_ptr;
+  const uint32_t tmem_base = __shfl_sync(0xffffffffu, *tmem_ptr, 0);
 
   auto tile_coords = [&](int t, int& m0, int& n0) {
     const int per_group = Q_GROUP_M * num_n;
@@ -483,39 +495,39 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
       }
     }
   } else if (warp == 1) {
-    if (lane == 0) {
+    {                                              // the whole warp, converged: one lane is elected per instruction
       constexpr uint32_t idesc = make_idesc_nvf4(QBM, QBN);
       int stage = 0; uint32_t phase = 0;
       int it = 0;
       for (int t = cta; t < num_tiles; t += n_cta, ++it) {
         const int acc = it & 1; const uint32_t acc_phase = (it >> 1) & 1;
-        if (!mbar_wait(&tmem_empty[acc], acc_phase ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY)) goto done;
+        if (!mbar_wait_warp(&tmem_empty[acc], acc_phase ^ 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_EMPTY)) goto done;
         tc_fence_after();
         int m0, n0; tile_coords(t, m0, n0);
         const uint32_t d_tmem = tmem_base + acc * QBN;
         const uint32_t sfb_shift = (n0 >> 5) & 3;                         // 0 or 2: rows 64.. of the first row chunk
         for (int kb = 0; kb < KC; ++kb) {
-          if (!mbar_wait(&full_bar[stage], phase, abort_flag, p.status, STATUS_TIMEOUT_FULL)) goto done;
+          if (!mbar_wait_warp(&full_bar[stage], phase, abort_flag, p.status, STATUS_TIMEOUT_FULL)) goto done;
           tc_fence_after();
           const uint32_t sa = smem_u32(smem + stage * FSTAGE_BYTES);
 #pragma unroll
           for (uint32_t k = 0; k < 4; ++k) {
-            tmem_cp_sf(tmem_base + F_TMEM_SFA + 4 * k, make_sf_desc(sa + FSFA_OFF + 512 * k));
-            tmem_cp_sf(tmem_base + F_TMEM_SFB + 8 * k, make_sf_desc(sa + FSFB_OFF + 512 * k));
-            tmem_cp_sf(tmem_base + F_TMEM_SFB + 8 * k + 4, make_sf_desc(sa + FSFB_OFF + 2048 + 512 * k));
+            tmem_cp_sf_warp(tmem_base + F_TMEM_SFA + 4 * k, make_sf_desc(sa + FSFA_OFF + 512 * k));
+            tmem_cp_sf_warp(tmem_base + F_TMEM_SFB + 8 * k, make_sf_desc(sa + FSFB_OFF + 512 * k));
+            tmem_cp_sf_warp(tmem_base + F_TMEM_SFB + 8 * k + 4, make_sf_desc(sa + FSFB_OFF + 2048 + 512 * k));
           }
           const uint64_t da = make_smem_desc(sa, 16, 1024);
           const uint64_t db = make_smem_desc(sa + FA_BYTES, 16, 1024);
 #pragma unroll
           for (uint32_t k = 0; k < 4; ++k)                               // 64 elements = 32 bytes of K per instruction
-            umma_nvf4(d_tmem, da + static_cast<uint64_t>(k * 2), db + static_cast<uint64_t>(k * 2), idesc,
+            umma_nvf4_warp(d_tmem, da + static_cast<uint64_t>(k * 2), db + static_cast<uint64_t>(k * 2), idesc,
                       tmem_base + F_TMEM_SFA + 4 * k, tmem_base + F_TMEM_SFB + 8 * k + sfb_shift,
                       (kb != 0 || k != 0) ? 1u : 0u);
-          umma_commit(&empty_bar[stage]);
+          umma_commit_warp(&empty_bar[stage]);
           if (++stage == FSTAGES) { stage = 0; phase ^= 1; }
         }
-        if (KC == 0) mbar_arrive(&tmem_full[acc]);
-        else umma_commit(&tmem_full[acc]);
+        if (KC == 0) { if (lane == 0) mbar_arrive(&tmem_full[acc]); }
+        else umma_commit_warp(&tmem_full[acc]);
       }
     }
   } else {
