@@ -1,8 +1,7 @@
 // Fused per-head RMSNorm (QK-norm) + rotary embedding (NeoX halves) for q:[N,H,D] and k:[N,G,D], bf16.
-// One warp per token (all its heads); D ∈ {64, 128} so a lane owns D/32 contiguous elements of a head row and its
-// rotation partner (i ± D/2) lives in lane ^ 16.  Statistics and rotation in fp32.
+// One warp per token (all its heads, two at a time); D ∈ {64, 128}.  Statistics and rotation in fp32.
 // Backward undoes the rotation (conjugate), then applies the RMSNorm backward; the weight gradient
-// is accumulated per warp in registers, per CTA in shared memory and written as per-CTA partials
+// is accumulated per warp in registers, per CTA in shared memory (warps in a fixed order) and written as per-CTA partials
 // (deterministic two-stage reduction).
 #include "sm100.cuh"
 #include "api.h"
@@ -27,19 +26,37 @@ template <> __device__ __forceinline__ void st_row<4>(__nv_bfloat16* p, const fl
 template <> __device__ __forceinline__ void st_row<2>(__nv_bfloat16* p, const float (&v)[2]) {
   *reinterpret_cast<uint32_t*>(p) = pack_bf16x2(v[0], v[1]);
 }
+// EPL packed elements as loaded (half the registers of their fp32 values), and the conversion
+template <int EPL> struct Raw { uint32_t w[EPL / 2]; };
+__device__ __forceinline__ void ld_raw(const __nv_bfloat16* p, Raw<4>& r) {
+  const uint2 u = *reinterpret_cast<const uint2*>(p);
+  r.w[0] = u.x; r.w[1] = u.y;
+}
+__device__ __forceinline__ void ld_raw(const __nv_bfloat16* p, Raw<2>& r) { r.w[0] = *reinterpret_cast<const uint32_t*>(p); }
+__device__ __forceinline__ void st_raw(__nv_bfloat16* p, const Raw<4>& r) { *reinterpret_cast<uint2*>(p) = make_uint2(r.w[0], r.w[1]); }
+__device__ __forceinline__ void st_raw(__nv_bfloat16* p, const Raw<2>& r) { *reinterpret_cast<uint32_t*>(p) = r.w[0]; }
+template <int EPL> __device__ __forceinline__ void expand(const Raw<EPL>& r, float (&v)[EPL]) {
+#pragma unroll
+  for (int i = 0; i < EPL / 2; ++i) { const float2 f = unpack_bf16x2(r.w[i]); v[2 * i] = f.x; v[2 * i + 1] = f.y; }
+}
 template <typename TW> __device__ __forceinline__ float ldw(const TW* w, int i);
 template <> __device__ __forceinline__ float ldw<float>(const float* w, int i) { return w[i]; }
 template <> __device__ __forceinline__ float ldw<__nv_bfloat16>(const __nv_bfloat16* w, int i) { return __bfloat162float(w[i]); }
 
-__device__ __forceinline__ float wsum(float v) {
+// Sum over the 16 lanes of a half warp.
+__device__ __forceinline__ float half_sum(float v) {
 #pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  for (int o = 8; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
   return v;
 }
 
-// One warp per TOKEN: cos / sin and the norm gains are loaded once and serve all H + G heads of the token, there is no
-// per-row index arithmetic, and the heads are walked four at a time so that four 256-byte rows are in flight per warp.
-constexpr int ROPE_U = 4;
+// One warp per TOKEN, half a warp per head: a lane owns EPL elements of the head's first half and the EPL elements they are
+// rotated with, so the rotation needs no exchange and a row sum takes four shuffles for two heads.  (With a row over the whole
+// warp, five shuffles for the sum and EPL for the rotation per head kept the kernels at a third of the copy bandwidth: B8 T4096
+// H16 G4 D128 forward + value copy 0.105 -> 0.081 ms, backward 0.241 -> 0.138; B1 T8192 H40 G20 D64 0.064 / 0.126 -> 0.050 /
+// 0.083.)  cos / sin and the norm gains are loaded once and serve all heads of the token, which are walked 2·ROPE_U at a time so
+// that as many rows are in flight per warp (ROPE_U 4 needs 128 registers backward: 0.138 ms too, 0.099 against 0.091 at H8 G2).
+constexpr int ROPE_U = 2;
 
 // Where the heads of a token sit.  Dense rows [tokens, heads, D] are q_hpg = H, k_gs = D; the output of a fused QKV projection
 // laid out per key/value group as [group][q_per_kv query heads, key head, value head][D] is q_hpg = q_per_kv and
@@ -50,18 +67,79 @@ struct QKLayout {
   int q_hpg;                 // query heads per group
 };
 
-// Copies G head rows of one token between two head strides; kept out of line so that the row copy does not change how the
-// compiler schedules the norm / rotation loops around it (inlined, both kernels ran about twice as long).
+// Copies the G value rows of every token between two layouts (token and head strides): a pass of its own after the loop over
+// tokens, eight rows in flight per warp (inside that loop it is one more load-to-store wait per token: backward 0.171 against
+// 0.126 ms without any copy at B8 T4096 H16 G4 D128).
 template <int EPL>
-__device__ __noinline__ void copy_head_rows(const __nv_bfloat16* src, long long sstride, __nv_bfloat16* dst, long long dstride, int G) {
-  for (int g0 = 0; g0 < G; g0 += ROPE_U) {
-    float x[ROPE_U][EPL];
+__device__ __forceinline__ void copy_value_rows(const __nv_bfloat16* __restrict__ src, long long s_ts, long long s_hs,
+                                                __nv_bfloat16* __restrict__ dst, long long d_ts, long long d_hs, int64_t n_tokens, int G,
+                                                int64_t warp_global, int64_t n_warps, int lane) {
+  const int64_t rows = n_tokens * G;
+  for (int64_t r0 = warp_global * 8; r0 < rows; r0 += n_warps * 8) {
+    Raw<EPL> x[8];
+    int64_t tok = r0 / G;
+    int g = static_cast<int>(r0 - tok * G);
+    const int64_t tok0 = tok;
+    const int g0 = g;
 #pragma unroll
-    for (int u = 0; u < ROPE_U; ++u)
-      if (g0 + u < G) ld_row<EPL>(src + (g0 + u) * sstride, x[u]);
+    for (int u = 0; u < 8; ++u) {
+      if (r0 + u < rows) ld_raw(src + tok * s_ts + g * s_hs + lane * EPL, x[u]);
+      if (++g == G) { g = 0; ++tok; }
+    }
+    tok = tok0; g = g0;
 #pragma unroll
-    for (int u = 0; u < ROPE_U; ++u)
-      if (g0 + u < G) st_row<EPL>(dst + (g0 + u) * dstride, x[u]);
+    for (int u = 0; u < 8; ++u) {
+      if (r0 + u < rows) st_raw(dst + tok * d_ts + g * d_hs + lane * EPL, x[u]);
+      if (++g == G) { g = 0; ++tok; }
+    }
+  }
+}
+
+// The `per` head rows at src (stride hstride), normalised (w: the gains of this lane's elements, first half then second, or
+// has_w false) and rotated (rot), to dense rows at dst.  src / dst point at this lane's first element of head 0.
+template <int EPL>
+__device__ __forceinline__ void fwd_heads(const __nv_bfloat16* src, long long hstride, __nv_bfloat16* dst, float* rstd, int per,
+                                          const float (&w)[2 * EPL], bool has_w, bool rot, const float (&cs)[EPL], const float (&sn)[EPL],
+                                          int lane, float eps) {
+  constexpr int D = EPL * 32;
+  const int sub = lane >> 4;
+  for (int h0 = 0; h0 < per; h0 += 2 * ROPE_U) {
+    Raw<EPL> rlo[ROPE_U], rhi[ROPE_U];
+#pragma unroll
+    for (int u = 0; u < ROPE_U; ++u) {
+      const int h = min(h0 + 2 * u + sub, per - 1);            // past the last head: loaded again, not stored
+      ld_raw(src + h * hstride, rlo[u]);
+      ld_raw(src + h * hstride + D / 2, rhi[u]);
+    }
+#pragma unroll
+    for (int u = 0; u < ROPE_U; ++u) {
+      const int h = h0 + 2 * u + sub;
+      float lo[EPL], hi[EPL];
+      expand<EPL>(rlo[u], lo);
+      expand<EPL>(rhi[u], hi);
+      if (has_w) {
+        float ss = 0.f;
+#pragma unroll
+        for (int e = 0; e < EPL; ++e) ss += lo[e] * lo[e] + hi[e] * hi[e];
+        ss = half_sum(ss);
+        const float rs = rsqrtf(ss / D + eps);
+        if ((lane & 15) == 0 && h < per) rstd[h] = rs;
+#pragma unroll
+        for (int e = 0; e < EPL; ++e) { lo[e] = lo[e] * rs * w[e]; hi[e] = hi[e] * rs * w[EPL + e]; }
+      }
+      if (rot) {
+#pragma unroll
+        for (int e = 0; e < EPL; ++e) {
+          const float a = lo[e], b = hi[e];
+          lo[e] = a * cs[e] - b * sn[e];
+          hi[e] = a * sn[e] + b * cs[e];
+        }
+      }
+      if (h < per) {
+        st_row<EPL>(dst + h * D, lo);
+        st_row<EPL>(dst + h * D + D / 2, hi);
+      }
+    }
   }
 }
 
@@ -78,12 +156,13 @@ __global__ void __launch_bounds__(256, 4) qknorm_rope_fwd_kernel(
   const int lane = threadIdx.x & 31;
   const int64_t warp_global = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
   const int64_t n_warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
-  const int ci = (lane & 15) * EPL;
-  float wq[EPL], wk[EPL];
+  const int ci = (lane & 15) * EPL;                 // this lane's first element of a head row
+  float wq[2 * EPL], wk[2 * EPL];
 #pragma unroll
-  for (int e = 0; e < EPL; ++e) {
-    wq[e] = qw ? ldw<TW>(qw, lane * EPL + e) : 1.f;
-    wk[e] = kw ? ldw<TW>(kw, lane * EPL + e) : 1.f;
+  for (int e = 0; e < 2 * EPL; ++e) {
+    const int c = ci + (e % EPL) + (e / EPL) * (D / 2);
+    wq[e] = qw ? ldw<TW>(qw, c) : 1.f;
+    wk[e] = kw ? ldw<TW>(kw, c) : 1.f;
   }
   for (int64_t tok = warp_global; tok < n_tokens; tok += n_warps) {
     float cs[EPL], sn[EPL];
@@ -92,57 +171,86 @@ __global__ void __launch_bounds__(256, 4) qknorm_rope_fwd_kernel(
       ld_row<EPL>(cosb + co, cs);
       ld_row<EPL>(sinb + co, sn);
     }
-#pragma unroll 1
-    for (int part = 0; part < 2; ++part) {      // the token's query heads, then its key heads
-      // inputs may be column slices of a wider (fused projection) matrix, dense or interleaved per group: see QKLayout.
-      // Heads are walked group by group (one group of H heads for dense rows), so no head index is ever divided.
-      const int per = part ? G : (GROUPED ? L.q_hpg : H), n_groups = (part || !GROUPED) ? 1 : H / L.q_hpg;
-      const long long gstride = (part || !GROUPED) ? 0 : L.q_gs, hstride = (GROUPED && part) ? L.k_gs : D;
-      const bool has_w = part ? kw != nullptr : qw != nullptr;
-      for (int grp = 0; grp < n_groups; ++grp) {
-        const __nv_bfloat16* src = (part ? k + tok * L.k_ts : q + tok * L.q_ts) + grp * gstride + lane * EPL;
-        __nv_bfloat16* dst = (part ? ko + tok * G * D : qo + tok * H * D) + static_cast<long long>(grp) * per * D + lane * EPL;
-        float* rstd = (part ? k_rstd + tok * G : q_rstd + tok * H) + grp * per;
-        for (int h0 = 0; h0 < per; h0 += ROPE_U) {
-          float x[ROPE_U][EPL];
+    // inputs may be column slices of a wider (fused projection) matrix, dense or interleaved per group: see QKLayout.
+    // Query heads are walked group by group (one group of H heads for dense rows), so no head index is ever divided.
+    const int per = GROUPED ? L.q_hpg : H, n_groups = GROUPED ? H / L.q_hpg : 1;
+    for (int grp = 0; grp < n_groups; ++grp)
+      fwd_heads<EPL>(q + tok * L.q_ts + (GROUPED ? grp * L.q_gs : 0) + ci, D, qo + (tok * H + grp * per) * D + ci,
+                     q_rstd + tok * H + grp * per, per, wq, qw != nullptr, cosb != nullptr, cs, sn, lane, eps);
+    fwd_heads<EPL>(k + tok * L.k_ts + ci, GROUPED ? L.k_gs : D, ko + tok * G * D + ci, k_rstd + tok * G, G, wk, kw != nullptr,
+                   cosb != nullptr, cs, sn, lane, eps);
+  }
+  if (WITH_V)                                       // the value heads, copied out of the fused projection into dense rows
+    copy_value_rows<EPL>(v, L.k_ts, GROUPED ? L.k_gs : D, vo, static_cast<long long>(G) * D, D, n_tokens, G, warp_global, n_warps, lane);
+}
+
+// Backward of fwd_heads: rotate back, then the RMSNorm backward; the gain gradient is added into dw.
+template <int EPL>
+__device__ __forceinline__ void bwd_heads(const __nv_bfloat16* gsrc, const __nv_bfloat16* xsrc, long long hstride, __nv_bfloat16* gdst,
+                                          long long o_hstride, const float* rstd, int per, const float (&w)[2 * EPL],
+                                          float (&dw)[2 * EPL], bool has_w, bool rot, const float (&cs)[EPL], const float (&sn)[EPL],
+                                          int lane) {
+  constexpr int D = EPL * 32;
+  const int sub = lane >> 4;
+  for (int h0 = 0; h0 < per; h0 += 2 * ROPE_U) {
+    Raw<EPL> rgl[ROPE_U], rgh[ROPE_U], rxl[ROPE_U], rxh[ROPE_U];
+    float rsv[ROPE_U];
 #pragma unroll
-          for (int u = 0; u < ROPE_U; ++u)
-            if (h0 + u < per) ld_row<EPL>(src + (h0 + u) * hstride, x[u]);
-#pragma unroll
-          for (int u = 0; u < ROPE_U; ++u) {
-            if (h0 + u >= per) continue;          // warp-uniform
-            if (has_w) {
-              float ss = 0.f;
-#pragma unroll
-              for (int e = 0; e < EPL; ++e) ss += x[u][e] * x[u][e];
-              ss = wsum(ss);
-              const float rs = rsqrtf(ss / D + eps);
-              if (lane == 0) rstd[h0 + u] = rs;
-#pragma unroll
-              for (int e = 0; e < EPL; ++e) x[u][e] = x[u][e] * rs * (part ? wk[e] : wq[e]);
-            }
-            if (cosb) {
-              float o[EPL];
-#pragma unroll
-              for (int e = 0; e < EPL; ++e) {
-                const float other = __shfl_xor_sync(0xffffffffu, x[u][e], 16);
-                o[e] = lane < 16 ? x[u][e] * cs[e] - other * sn[e] : other * sn[e] + x[u][e] * cs[e];
-              }
-              st_row<EPL>(dst + (h0 + u) * D, o);
-            } else {
-              st_row<EPL>(dst + (h0 + u) * D, x[u]);
-            }
-          }
-        }
+    for (int u = 0; u < ROPE_U; ++u) {
+      const int h = min(h0 + 2 * u + sub, per - 1);            // past the last head: loaded again, counted and stored nowhere
+      ld_raw(gsrc + h * D, rgl[u]);
+      ld_raw(gsrc + h * D + D / 2, rgh[u]);
+      if (has_w) {
+        ld_raw(xsrc + h * hstride, rxl[u]);
+        ld_raw(xsrc + h * hstride + D / 2, rxh[u]);
+        rsv[u] = rstd[h];
       }
     }
-    if (WITH_V)                                     // the value heads, copied out of the fused projection into dense rows
-      copy_head_rows<EPL>(v + tok * L.k_ts + lane * EPL, GROUPED ? L.k_gs : D, vo + tok * G * D + lane * EPL, D, G);
+#pragma unroll
+    for (int u = 0; u < ROPE_U; ++u) {
+      const int h = h0 + 2 * u + sub;
+      float glo[EPL], ghi[EPL];
+      expand<EPL>(rgl[u], glo);
+      expand<EPL>(rgh[u], ghi);
+      if (rot) {
+#pragma unroll
+        for (int e = 0; e < EPL; ++e) {
+          const float a = glo[e], b = ghi[e];
+          glo[e] = a * cs[e] + b * sn[e];
+          ghi[e] = b * cs[e] - a * sn[e];
+        }
+      }
+      if (has_w) {
+        float xlo[EPL], xhi[EPL], dot = 0.f;
+        expand<EPL>(rxl[u], xlo);
+        expand<EPL>(rxh[u], xhi);
+        const float rs = rsv[u], rs_dw = h < per ? rs : 0.f;
+#pragma unroll
+        for (int e = 0; e < EPL; ++e) {
+          dw[e] += glo[e] * xlo[e] * rs_dw;
+          dw[EPL + e] += ghi[e] * xhi[e] * rs_dw;
+          glo[e] *= w[e];
+          ghi[e] *= w[EPL + e];
+          dot += glo[e] * xlo[e] + ghi[e] * xhi[e];
+        }
+        dot = half_sum(dot);
+        const float c1 = dot * rs * rs * rs / D;
+#pragma unroll
+        for (int e = 0; e < EPL; ++e) {
+          glo[e] = glo[e] * rs - xlo[e] * c1;
+          ghi[e] = ghi[e] * rs - xhi[e] * c1;
+        }
+      }
+      if (h < per) {
+        st_row<EPL>(gdst + h * o_hstride, glo);
+        st_row<EPL>(gdst + h * o_hstride + D / 2, ghi);
+      }
+    }
   }
 }
 
 template <int EPL, typename TW, bool GROUPED, bool WITH_V>
-__global__ void __launch_bounds__(256, 2) qknorm_rope_bwd_kernel(
+__global__ void __launch_bounds__(256, 3) qknorm_rope_bwd_kernel(
     const __nv_bfloat16* __restrict__ dqo, const __nv_bfloat16* __restrict__ dko, const __nv_bfloat16* __restrict__ q,
     const __nv_bfloat16* __restrict__ k, const TW* __restrict__ qw, const TW* __restrict__ kw,
     const __nv_bfloat16* __restrict__ cosb, const __nv_bfloat16* __restrict__ sinb, const float* __restrict__ q_rstd,
@@ -150,19 +258,18 @@ __global__ void __launch_bounds__(256, 2) qknorm_rope_bwd_kernel(
     float* __restrict__ dw_partial /* [grid, 2, D] */, int64_t n_tokens, int T, int H, int G, const QKLayout L,
     const QKLayout LO /* layout of dq, dk (and dv_dst) */, const __nv_bfloat16* __restrict__ dvo, __nv_bfloat16* __restrict__ dv_dst) {
   constexpr int D = EPL * 32;
-  __shared__ float dw_s[2][D];
-  const int lane = threadIdx.x & 31;
-  for (int i = threadIdx.x; i < 2 * D; i += blockDim.x) (&dw_s[0][0])[i] = 0.f;
-  __syncthreads();
+  __shared__ float dw_s[8][2][D];
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t warp_global = (blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x) >> 5;
   const int64_t n_warps = (static_cast<int64_t>(gridDim.x) * blockDim.x) >> 5;
   const int ci = (lane & 15) * EPL;
-  float dwq[EPL], dwk[EPL], wq[EPL], wk[EPL];
+  float dwq[2 * EPL], dwk[2 * EPL], wq[2 * EPL], wk[2 * EPL];
 #pragma unroll
-  for (int e = 0; e < EPL; ++e) {
+  for (int e = 0; e < 2 * EPL; ++e) {
+    const int c = ci + (e % EPL) + (e / EPL) * (D / 2);
     dwq[e] = dwk[e] = 0.f;
-    wq[e] = qw ? ldw<TW>(qw, lane * EPL + e) : 1.f;
-    wk[e] = kw ? ldw<TW>(kw, lane * EPL + e) : 1.f;
+    wq[e] = qw ? ldw<TW>(qw, c) : 1.f;
+    wk[e] = kw ? ldw<TW>(kw, c) : 1.f;
   }
   for (int64_t tok = warp_global; tok < n_tokens; tok += n_warps) {
     float cs[EPL], sn[EPL];
@@ -171,71 +278,31 @@ __global__ void __launch_bounds__(256, 2) qknorm_rope_bwd_kernel(
       ld_row<EPL>(cosb + co, cs);
       ld_row<EPL>(sinb + co, sn);
     }
-#pragma unroll 1
-    for (int part = 0; part < 2; ++part) {
-      const int per = part ? G : (GROUPED ? L.q_hpg : H), n_groups = (part || !GROUPED) ? 1 : H / L.q_hpg;      // LO: same grouping
-      const long long gstride = (part || !GROUPED) ? 0 : L.q_gs, hstride = (GROUPED && part) ? L.k_gs : D;
-      const long long o_gstride = (part || !GROUPED) ? 0 : LO.q_gs, o_hstride = (GROUPED && part) ? LO.k_gs : D;
-      const bool has_w = part ? kw != nullptr : qw != nullptr;
-      for (int grp = 0; grp < n_groups; ++grp) {
-        const long long dense = static_cast<long long>(grp) * per * D + lane * EPL;
-        const __nv_bfloat16* gsrc = (part ? dko + tok * G * D : dqo + tok * H * D) + dense;
-        __nv_bfloat16* gdst = (part ? dk + tok * LO.k_ts : dq + tok * LO.q_ts) + grp * o_gstride + lane * EPL;
-        const __nv_bfloat16* xsrc = (part ? k + tok * L.k_ts : q + tok * L.q_ts) + grp * gstride + lane * EPL;
-        const float* rstd = (part ? k_rstd + tok * G : q_rstd + tok * H) + grp * per;
-        for (int h0 = 0; h0 < per; h0 += ROPE_U) {
-          float g[ROPE_U][EPL], x[ROPE_U][EPL], rs[ROPE_U];
-#pragma unroll
-          for (int u = 0; u < ROPE_U; ++u) {
-            if (h0 + u >= per) continue;
-            ld_row<EPL>(gsrc + (h0 + u) * D, g[u]);
-            if (has_w) { ld_row<EPL>(xsrc + (h0 + u) * hstride, x[u]); rs[u] = rstd[h0 + u]; }
-          }
-#pragma unroll
-          for (int u = 0; u < ROPE_U; ++u) {
-            if (h0 + u >= per) continue;
-            if (cosb) {
-              float o[EPL];
-#pragma unroll
-              for (int e = 0; e < EPL; ++e) {
-                const float other = __shfl_xor_sync(0xffffffffu, g[u][e], 16);
-                o[e] = lane < 16 ? g[u][e] * cs[e] + other * sn[e] : -other * sn[e] + g[u][e] * cs[e];
-              }
-#pragma unroll
-              for (int e = 0; e < EPL; ++e) g[u][e] = o[e];
-            }
-            if (has_w) {
-              float dot = 0.f;
-              float gw[EPL];
-#pragma unroll
-              for (int e = 0; e < EPL; ++e) {
-                gw[e] = g[u][e] * (part ? wk[e] : wq[e]);
-                dot += gw[e] * x[u][e];
-                if (part) dwk[e] += g[u][e] * x[u][e] * rs[u]; else dwq[e] += g[u][e] * x[u][e] * rs[u];
-              }
-              dot = wsum(dot);
-              const float c1 = dot * rs[u] * rs[u] * rs[u] / D;
-#pragma unroll
-              for (int e = 0; e < EPL; ++e) g[u][e] = gw[e] * rs[u] - x[u][e] * c1;
-            }
-            st_row<EPL>(gdst + (h0 + u) * o_hstride, g[u]);
-          }
-        }
-      }
-    }
-    if (WITH_V)                                     // the value gradient takes its slot of the fused-projection gradient
-      copy_head_rows<EPL>(dvo + static_cast<size_t>(tok) * G * D + lane * EPL, D, dv_dst + tok * LO.k_ts + lane * EPL,
-                          GROUPED ? LO.k_gs : D, G);
+    const int per = GROUPED ? L.q_hpg : H, n_groups = GROUPED ? H / L.q_hpg : 1;      // LO: same grouping
+    for (int grp = 0; grp < n_groups; ++grp)
+      bwd_heads<EPL>(dqo + (tok * H + grp * per) * D + ci, q + tok * L.q_ts + (GROUPED ? grp * L.q_gs : 0) + ci, D,
+                     dq + tok * LO.q_ts + (GROUPED ? grp * LO.q_gs : 0) + ci, D, q_rstd + tok * H + grp * per, per, wq, dwq,
+                     qw != nullptr, cosb != nullptr, cs, sn, lane);
+    bwd_heads<EPL>(dko + tok * G * D + ci, k + tok * L.k_ts + ci, GROUPED ? L.k_gs : D, dk + tok * LO.k_ts + ci, GROUPED ? LO.k_gs : D,
+                   k_rstd + tok * G, G, wk, dwk, kw != nullptr, cosb != nullptr, cs, sn, lane);
   }
-  if (qw) {
+  if (WITH_V)                                       // the value gradient takes its slot of the fused-projection gradient
+    copy_value_rows<EPL>(dvo, static_cast<long long>(G) * D, D, dv_dst, LO.k_ts, GROUPED ? LO.k_gs : D, n_tokens, G, warp_global,
+                         n_warps, lane);
+  if (qw) {                                         // the two halves of a warp, then the warps in order
 #pragma unroll
-    for (int e = 0; e < EPL; ++e) {
-      atomicAdd(&dw_s[0][lane * EPL + e], dwq[e]);
-      atomicAdd(&dw_s[1][lane * EPL + e], dwk[e]);
+    for (int e = 0; e < 2 * EPL; ++e) {
+      const float a = dwq[e] + __shfl_xor_sync(0xffffffffu, dwq[e], 16), b = dwk[e] + __shfl_xor_sync(0xffffffffu, dwk[e], 16);
+      const int c = ci + (e % EPL) + (e / EPL) * (D / 2);
+      if (lane < 16) { dw_s[warp][0][c] = a; dw_s[warp][1][c] = b; }
     }
     __syncthreads();
-    for (int i = threadIdx.x; i < 2 * D; i += blockDim.x)
-      dw_partial[static_cast<size_t>(blockIdx.x) * 2 * D + i] = (&dw_s[0][0])[i];
+    for (int i = threadIdx.x; i < 2 * D; i += blockDim.x) {
+      float t = 0.f;
+#pragma unroll
+      for (int w = 0; w < 8; ++w) t += (&dw_s[w][0][0])[i];
+      dw_partial[static_cast<size_t>(blockIdx.x) * 2 * D + i] = t;
+    }
   }
 }
 
