@@ -76,7 +76,7 @@ def swiglu_packed(x: torch.Tensor) -> torch.Tensor:
     I = x.shape[-1] // 2
     if (x.dtype == torch.bfloat16 and I % 8 == 0 and x.is_contiguous()
             and backend.use_cuda_kernel("swiglu", x)):
-        return _SwiGLUPackedFn.apply(x.view(-1, 2 * I)).view(*x.shape[:-1], I)
+        return backend.apply(_SwiGLUPackedFn, x.view(-1, 2 * I)).view(*x.shape[:-1], I)
     g, u = x.chunk(2, dim=-1)
     return swiglu_ref(g, u)
 

@@ -211,7 +211,7 @@ def attention(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, scale: Optional
         if sink is not None:
             out, lse = _AttnSinkFn.apply(q, k, v, sink, float(scale), int(window[0]), cu_seqlens)
         else:
-            out, lse = _AttnFn.apply(q, k, v, float(scale), int(window[0]), cu_seqlens)
+            out, lse = backend.apply(_AttnFn, q, k, v, float(scale), int(window[0]), cu_seqlens)
         return (out, lse) if return_lse else out
     if q.is_cuda and sink is None and not return_lse:
         return _sdpa_fallback(q, k, v, scale, window, cu_seqlens)

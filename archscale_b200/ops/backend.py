@@ -19,6 +19,7 @@ import threading
 from typing import Optional
 
 import torch
+from torch.autograd import forward_ad
 
 _lock = threading.Lock()
 _ext = None
@@ -72,8 +73,11 @@ def _disabled(op: str) -> bool:
 
 def use_cuda_kernel(op: str, *tensors: torch.Tensor) -> bool:
     """True when ``op`` must run its sm_100a kernel for these tensors."""
-    if not tensors or not all(t is None or t.is_cuda for t in tensors):
+    if not tensors:
         return False
+    for t in tensors:
+        if t is not None and not t.is_cuda:
+            return False
     if _disabled(op):
         return False
     if load_extension() is None:
@@ -83,6 +87,31 @@ def use_cuda_kernel(op: str, *tensors: torch.Tensor) -> bool:
             f"op '{op}' got CUDA tensors but the sm_100a extension is not loadable: {_ext_error!r}. "
             "Build it with `python -m archscale_b200.build` (or set ARCHSCALE_B200_ALLOW_FALLBACK=1).")
     return True
+
+
+def plain_call() -> bool:
+    """True when no autograd machinery can see a call: gradients are off, and no functorch transform, forward-mode level or
+    ``torch.jit`` trace is active.  An op then runs its kernel directly instead of through ``autograd.Function.apply`` (8 µs per call, which is what a
+    forward pass over a few dozen tokens spends most of its time on)."""
+    return (not torch.is_grad_enabled() and not torch._C._are_functorch_transforms_active() and forward_ad._current_level < 0
+            and torch._C._get_tracing_state() is None)
+
+
+class NoCtx:
+    """Stands in for an autograd context in a direct call of ``Function.forward``: nothing is kept."""
+
+    needs_input_grad = ()
+
+    def save_for_backward(self, *tensors) -> None:
+        pass
+
+    def mark_non_differentiable(self, *tensors) -> None:
+        pass
+
+
+def apply(fn, *args):
+    """``fn.apply(*args)``, or ``fn.forward`` itself where nothing can need its backward (:func:`plain_call`)."""
+    return fn.forward(NoCtx(), *args) if plain_call() else fn.apply(*args)
 
 
 def has(symbol: str) -> bool:

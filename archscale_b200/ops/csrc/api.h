@@ -94,6 +94,9 @@ int b200_grouped_gemm_bf16(int kind, const void* A, const void* B, void* out, co
 int b200_attn_fwd(const void* q, const void* k, const void* v, void* out, float* lse, const int* row_start, int B, int T,
                   int H, int G, int D, int window_left, float scale, int* status, cudaStream_t stream);
 
+// out[M, Σ n_w] = X · [W_0; …]ᵀ for few rows M, or silu(gate)·up of one W = [gate; up] (gemm_skinny.cu).
+int b200_gemm_skinny(const void* X, const void* const* W, const int* n_w, int n_mats, int swiglu, void* out, int M, int K, int ldx,
+                     const int* ldw, int ldo, int num_sms, int* status, cudaStream_t stream);
 // The forward with two query tiles per CTA (attention_fwd_pair.cu); b200_attn_fwd checks the arguments and calls it.
 int b200_attn_fwd_pair(const void* q, const void* k, const void* v, void* out, float* lse, const int* row_start, int B, int T,
                        int H, int G, int D, int window_left, float scale, int* status, cudaStream_t stream);

@@ -166,9 +166,38 @@ def fused_swiglu_enabled() -> bool:
             and backend.has("gemm_swiglu"))
 
 
+SKINNY_ROWS = 64
+
+
+def _skinny_ok(x: torch.Tensor, ws) -> bool:
+    """Whether the kernel for few rows (``csrc/gemm_skinny.cu``) takes ``x @ [w₀; w₁; …]ᵀ``: no gradients, at most 64 rows (one
+    block of its tokens: beyond that the library's device time, 4 to 16 µs, is less than half of its), dense bf16 rows that the TMA
+    can read (16-byte base, widths that are multiples of 8)."""
+    K = x.shape[-1]
+    if not (x.is_cuda and x.dtype == torch.bfloat16 and 0 < x.numel() <= SKINNY_ROWS * K and K % 8 == 0 and x.is_contiguous()
+            and x.data_ptr() % 16 == 0 and backend.plain_call() and backend.has("gemm_skinny")):
+        return False
+    for w in ws:
+        if not (w.is_cuda and w.dtype == torch.bfloat16 and w.dim() == 2 and w.shape[0] % 8 == 0 and w.shape[0] > 0 and w.stride(1) == 1
+                and w.stride(0) % 8 == 0 and w.stride(0) >= K and w.data_ptr() % 16 == 0):
+            return False
+        g = getattr(w, "_fsdp_group", None)
+        if g is not None and getattr(g, "ag_pending", False):
+            return False
+    return backend.use_cuda_kernel("gemm", x, *ws)
+
+
+def _skinny(x: torch.Tensor, ws, swiglu: bool) -> torch.Tensor:
+    y = backend.require_extension().gemm_skinny(x.view(-1, x.shape[-1]), ws, swiglu)
+    backend.count_launch()
+    return y.view(*x.shape[:-1], y.shape[-1])
+
+
 def linear_swiglu(x: torch.Tensor, weight: torch.Tensor) -> Optional[torch.Tensor]:
     """SwiGLU of ``x @ weightᵀ`` (gate = first half of the output features) in one GEMM launch, or ``None`` when the
     fused kernel does not take this case (the caller then runs ``linear`` + ``swiglu_packed``)."""
+    if weight.shape[0] % 16 == 0 and _skinny_ok(x, (weight,)) and fused_swiglu_enabled():
+        return _skinny(x, [weight], True)
     if not (x.is_cuda and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and weight.dim() == 2
             and weight.shape[0] % 16 == 0 and x.shape[-1] % 8 == 0 and x.shape[-1] >= 64
             and (x.numel() // x.shape[-1]) % 8 == 0 and weight.stride(-1) == 1 and weight.stride(0) % 8 == 0
@@ -179,18 +208,20 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor) -> Optional[torch.Tenso
         return None                                     # this GEMM carries the unit's fused all-gather: keep that path
     if not x.is_contiguous():
         x = x.contiguous()
-    return _LinearSwiGLUFn.apply(x, weight, torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad))
+    return backend.apply(_LinearSwiGLUFn, x, weight, torch.is_grad_enabled() and (x.requires_grad or weight.requires_grad))
 
 
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``x @ weightᵀ + bias``; bf16 CUDA inputs run the tcgen05 kernel for fwd, dgrad and wgrad."""
+    if bias is None and _skinny_ok(x, (weight,)):
+        return _skinny(x, [weight], False)
     if (x.is_cuda and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16
             and x.shape[-1] % 8 == 0 and weight.shape[0] % 8 == 0 and x.shape[-1] >= 64
             and (x.numel() // x.shape[-1]) % 8 == 0
             and backend.use_cuda_kernel("gemm", x, weight)):
         if not x.is_contiguous():
             x = x.contiguous()
-        return _LinearFn.apply(x, weight, bias)
+        return backend.apply(_LinearFn, x, weight, bias)
     g = getattr(weight, "_fsdp_group", None)
     if g is not None and getattr(g, "ag_pending", False):
         weight._fsdp_engine.finish_pending_gather(g)
@@ -290,6 +321,10 @@ def linear_multi(x: torch.Tensor, layers, keep_fused: bool = False):
     slices of its result; otherwise each layer is called on its own.  ``keep_fused``: return the one GEMM's result unsplit
     (a tensor instead of a list) when the layers did run as one GEMM."""
     ws = [l.weight for l in layers]
+    if (len(ws) <= 3 and all(type(l).__name__ == "Linear" and l.bias is None and not l.mxfp8 and not getattr(l, "nvfp4", False)
+                             for l in layers) and _skinny_ok(x, ws)):
+        y = _skinny(x, ws, False)                       # the weights need not be neighbours here
+        return y if keep_fused else list(y.split([w.shape[0] for w in ws], dim=-1))
     fusable = (x.is_cuda and x.dtype == torch.bfloat16 and all(type(l).__name__ == "Linear" and l.bias is None and not l.mxfp8
                                                               and not getattr(l, "nvfp4", False) for l in layers)
                and all(w.dtype == torch.bfloat16 for w in ws) and _adjacent(ws)
@@ -297,7 +332,7 @@ def linear_multi(x: torch.Tensor, layers, keep_fused: bool = False):
                and backend.use_cuda_kernel("gemm", x, ws[0]))
     if not fusable:
         return [l(x) for l in layers]
-    y = _MultiLinearFn.apply(x if x.is_contiguous() else x.contiguous(), *ws)
+    y = backend.apply(_MultiLinearFn, x if x.is_contiguous() else x.contiguous(), *ws)
     if keep_fused:
         return y
     return list(y.split([w.shape[0] for w in ws], dim=-1))

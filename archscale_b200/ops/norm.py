@@ -234,5 +234,5 @@ def add_rms_norm(res: torch.Tensor, h: Optional[torch.Tensor], weight: torch.Ten
     if (fused_cols_ok(res.shape[-1]) and out_dtype == torch.bfloat16 and res.dtype in (torch.float32, torch.bfloat16)
             and (h is None or h.dtype == torch.bfloat16) and backend.has("add_rmsnorm_fwd")
             and backend.use_cuda_kernel("add_rmsnorm", res, h, weight)):
-        return _AddRMSNormFn.apply(res.contiguous(), None if h is None else h.contiguous(), weight, eps, h_scale, bf16_stream)
+        return backend.apply(_AddRMSNormFn, res.contiguous(), None if h is None else h.contiguous(), weight, eps, h_scale, bf16_stream)
     return add_rms_norm_ref(res, h, weight, eps, h_scale, out_dtype, stream_dtype)

@@ -133,7 +133,7 @@ def qk_norm_rope(q, k, q_weight, k_weight, cos, sin, eps: float = 1e-5, position
             and backend.use_cuda_kernel("qknorm_rope", q, k)):
         if cos is not None:
             cos, sin = cos[: q.shape[1]].contiguous(), sin[: q.shape[1]].contiguous()
-        return _QKNormRopeFn.apply(q, k, q_weight, k_weight, cos, sin, eps)
+        return backend.apply(_QKNormRopeFn, q, k, q_weight, k_weight, cos, sin, eps)
     return qk_norm_rope_ref(q, k, q_weight, k_weight, cos, sin, eps, positions)
 
 
@@ -194,7 +194,7 @@ def qkv_norm_rope(qkv, H: int, G: int, grouped: bool, q_weight, k_weight, cos, s
     :func:`qkv_norm_rope_supported` first."""
     if cos is not None:
         cos, sin = cos[: qkv.shape[1]].contiguous(), sin[: qkv.shape[1]].contiguous()
-    return _QKVNormRopeFn.apply(qkv, H, G, grouped, q_weight, k_weight, cos, sin, eps)
+    return backend.apply(_QKVNormRopeFn, qkv, H, G, grouped, q_weight, k_weight, cos, sin, eps)
 
 
 def apply_rotary_emb(x, cos, sin, interleaved: bool = False, positions=None):
