@@ -165,17 +165,29 @@ __global__ void __launch_bounds__(256) combine_rows_kernel(const __nv_bfloat16* 
 #pragma unroll
       for (int e = 0; e < 4; ++e) { const float2 f = unpack_bf16x2(ww[e]); acc[2 * e] = f.x; acc[2 * e + 1] = f.y; }
     }
-    for (int k = 0; k < K; ++k) {
-      const int slot = pair_slot[static_cast<size_t>(t) * K + k];
-      if (slot < 0 || slot >= capacity) {            // a slot outside the row buffer: reported, contributes nothing
-        if (status) atomicCAS(status, 0, STATUS_INDEX_RANGE);
-        continue;
-      }
-      const float wk = w ? w[static_cast<size_t>(t) * K + k] : 1.f;
-      const uint4 v = *reinterpret_cast<const uint4*>(y + static_cast<size_t>(slot) * C + c);
-      const uint32_t ww[4] = {v.x, v.y, v.z, v.w};
+    // four rows in flight (their indices first): one row after the other is a chain of 2·K memory latencies per thread
+    for (int k0 = 0; k0 < K; k0 += 4) {
+      uint4 v[4];
+      float wk[4];
+      bool ok[4];
 #pragma unroll
-      for (int e = 0; e < 4; ++e) { const float2 f = unpack_bf16x2(ww[e]); acc[2 * e] += wk * f.x; acc[2 * e + 1] += wk * f.y; }
+      for (int j = 0; j < 4; ++j) {
+        const int k = k0 + j;
+        const int slot = k < K ? pair_slot[static_cast<size_t>(t) * K + k] : 0;
+        ok[j] = k < K && slot >= 0 && slot < capacity;
+        if (k < K && !ok[j] && status) atomicCAS(status, 0, STATUS_INDEX_RANGE);   // a slot outside the row buffer: reported, contributes nothing
+        if (ok[j]) {
+          v[j] = *reinterpret_cast<const uint4*>(y + static_cast<size_t>(slot) * C + c);
+          wk[j] = w ? w[static_cast<size_t>(t) * K + k] : 1.f;
+        }
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (!ok[j]) continue;
+        const uint32_t ww[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) { const float2 f = unpack_bf16x2(ww[e]); acc[2 * e] += wk[j] * f.x; acc[2 * e + 1] += wk[j] * f.y; }
+      }
     }
     uint4 o;
     o.x = pack_bf16x2(alpha * acc[0], alpha * acc[1]); o.y = pack_bf16x2(alpha * acc[2], alpha * acc[3]);
