@@ -93,7 +93,7 @@ class _ScanFn(torch.autograd.Function):
 
 def _reset_flags(cu_seqlens: torch.Tensor, n_tokens: int) -> torch.Tensor:
     r = torch.zeros(n_tokens + 1, dtype=torch.int32, device=cu_seqlens.device)
-    r[cu_seqlens.long()] = 1
+    r.index_fill_(0, cu_seqlens.long(), 1)      # (an indexed assignment copies the scalar from the host and waits for the device)
     return r[:n_tokens].contiguous()
 
 
