@@ -169,6 +169,9 @@ int b200_selective_scan_bwd(const void* dy, int sdy, const void* u, int su, cons
                             int Di, int softplus, cudaStream_t st);
 int b200_selective_scan_channel_blocks(int Di);
 
+// The MXFP8 GEMM on SM pairs (gemm2_mxfp8.cu), tiles of 256 x nt (192 or 128); b200_gemm_mxfp8 checks the arguments and calls it.
+int b200_gemm2_mxfp8(const void* A, const void* sfa, const void* B, const void* sfb, void* out, int M, int N, int K, int lda, int ldb,
+                     int ldc, float alpha, int out_f32, int accumulate, int nt, int num_sms, int* status, cudaStream_t stream);
 // Block-scaled MXFP8 (gemm_mxfp8.cu): quantisers and the tcgen05 block-scaled GEMM.
 size_t b200_mxfp8_sf_bytes(int rows, int K);
 int b200_mxfp8_quantize(const void* x, int ld, void* q, void* sf, int R, int C, int colwise, cudaStream_t st,

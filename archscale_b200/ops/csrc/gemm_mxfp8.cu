@@ -4,7 +4,8 @@
 //   quantisers   bf16 → e4m3 + E8M0, row-wise (blocks along the contiguous dimension) or column-wise (the
 //                transposed operand is written, blocks along the original rows), so that forward, dgrad and
 //                wgrad of a linear layer are all "NT" GEMMs over K-major fp8 operands.
-//   GEMM         persistent warp-specialised kernel (TMA producer / MMA issuer / 4 epilogue warps) issuing
+//   GEMM         (gemm2_mxfp8.cu has the form on SM pairs for more than one wave of tiles; here the one-CTA kernel)
+//                persistent warp-specialised kernel (TMA producer / MMA issuer / 4 epilogue warps) issuing
 //                tcgen05.mma.kind::mxf8f6f4.block_scale, tile 128 × 192 × 128, 5-stage ring, two TMEM
 //                accumulators (2 × 192 columns) so the epilogue of a tile overlaps the next main loop.
 //
@@ -367,23 +368,41 @@ __global__ void __launch_bounds__(256) mxfp8_quant_colwise_kernel(const __nv_bfl
 typedef CUresult (*EncodeTiledFnQ)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
                                    const cuuint32_t*, const cuuint32_t*, CUtensorMapInterleave, CUtensorMapSwizzle,
                                    CUtensorMapL2promotion, CUtensorMapFloatOOBfill);
-static int make_tmap_2d_u8(CUtensorMap* map, const void* ptr, uint64_t inner, uint64_t outer, uint64_t row_stride_bytes,
-                           uint32_t box_inner, uint32_t box_outer) {
+static EncodeTiledFnQ encode_tiled_fn() {
   static EncodeTiledFnQ fn = nullptr;
   if (!fn) {
     void* ptr_fn = nullptr;
     cudaDriverEntryPointQueryResult qres;
     if (cudaGetDriverEntryPoint("cuTensorMapEncodeTiled", &ptr_fn, cudaEnableDefault, &qres) != cudaSuccess ||
         qres != cudaDriverEntryPointSuccess)
-      return -1;
+      return nullptr;
     fn = reinterpret_cast<EncodeTiledFnQ>(ptr_fn);
   }
+  return fn;
+}
+int make_tmap_2d_u8(CUtensorMap* map, const void* ptr, uint64_t inner, uint64_t outer, uint64_t row_stride_bytes,
+                    uint32_t box_inner, uint32_t box_outer) {
+  EncodeTiledFnQ fn = encode_tiled_fn();
+  if (!fn) return -1;
   cuuint64_t gdim[2] = {inner, outer};
   cuuint64_t gstride[1] = {row_stride_bytes};
   cuuint32_t box[2] = {box_inner, box_outer};
   cuuint32_t estr[2] = {1, 1};
   CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<void*>(ptr), gdim, gstride, box, estr,
                   CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
+                  CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
+}
+// Scale chunks as rows of 512 bytes, one per box; a row past the end reads as zeros.
+int make_tmap_sf_chunks(CUtensorMap* map, const void* ptr, uint64_t chunks) {
+  EncodeTiledFnQ fn = encode_tiled_fn();
+  if (!fn) return -1;
+  cuuint64_t gdim[2] = {128, chunks};
+  cuuint64_t gstride[1] = {512};
+  cuuint32_t box[2] = {128, 1};
+  cuuint32_t estr[2] = {1, 1};
+  CUresult r = fn(map, CU_TENSOR_MAP_DATA_TYPE_UINT32, 2, const_cast<void*>(ptr), gdim, gstride, box, estr,
+                  CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_NONE, CU_TENSOR_MAP_L2_PROMOTION_L2_256B,
                   CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   return r == CUDA_SUCCESS ? 0 : static_cast<int>(r);
 }
@@ -816,6 +835,16 @@ extern "C" int b200_gemm_mxfp8(const void* A, const void* sfa, const void* B, co
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || cudaSetDevice(dev) != cudaSuccess) return -5;
     ctx_bound = true;
+  }
+  // SM pairs as soon as the one-CTA tiles need more than one wave; their tiles 128 columns wide where that takes no more waves
+  // than 192 does.  ms, one CTA / pair 192 / pair 128: 16384x11264x2048 0.348 / 0.313 / 0.389, 16384x2048x2048 0.074 / 0.068 /
+  // 0.082, 2048x2048x16384 0.106 / 0.100 / 0.094, 4096x1024x2816 0.0266 / 0.0266 / 0.0246; one wave: 2048x1024x1024 0.0133 /
+  // 0.0154 / 0.0133, 1024x3072x1024 0.0153 / 0.0154 / 0.0174.
+  const int m1 = (M + QBM - 1) / QBM, n192 = (N + QBN - 1) / QBN, m2 = (M + 255) / 256, n128 = (N + 127) / 128, pairs = num_sms / 2;
+  if (static_cast<long long>(m1) * n192 > num_sms && pairs > 0) {
+    const long long w192 = (static_cast<long long>(m2) * n192 + pairs - 1) / pairs, w128 = (static_cast<long long>(m2) * n128 + pairs - 1) / pairs;
+    return b200_gemm2_mxfp8(A, sfa, B, sfb, out, M, N, K, lda, ldb, ldc, alpha, out_f32, accumulate, w128 <= w192 ? 128 : 192, num_sms,
+                            status, stream);
   }
   CUtensorMap ta, tb;
   int rc = make_tmap_2d_u8(&ta, A, K, M, lda, QBK, QBM);
