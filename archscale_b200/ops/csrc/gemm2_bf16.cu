@@ -244,6 +244,10 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     }
   } else {
     const int q = warp & 3;
+    const bool wide = p.ldc % (OUT_F32 ? 8 : 16) == 0 && reinterpret_cast<uintptr_t>(p.out) % 32 == 0 &&
+                      reinterpret_cast<uintptr_t>(p.cin) % 32 == 0 &&
+                      (!glu || (glu % 16 == 0 && p.ldc2 % 16 == 0 && reinterpret_cast<uintptr_t>(p.out2) % 32 == 0)) &&
+                      (GROUPED < 2 || (static_cast<size_t>(p.M) * p.ldc) % 16 == 0);
     int it = 0;
     for (int t = pair; t < num_tiles; t += n_pair, ++it) {
       Tile2 tl; get_tile(t, tl);
@@ -280,6 +284,10 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         }
       }
       const uint32_t taddr = tmem_base + acc * T2_BN + (static_cast<uint32_t>(q * 32) << 16);
+      // rows of 32-byte multiples: one sector per lane and store.  A warp's rows lie ldc apart, so with 16-byte stores the store
+      // unit is what a tile with a short K or two outputs waits for.  ms, 16-byte / 32-byte accesses: 524288x1024x256 (64
+      // experts) 0.527 / 0.316, 524288x512x1024 with SwiGLU 0.613 / 0.433, 16384x11264x2048 with SwiGLU 0.600 / 0.484,
+      // 5632x1024x1000 added to fp32 0.060 / 0.036, Newton-Schulz of 512 matrices of 1024x256 2.28 / 1.55
       if (glu) {
 #pragma unroll 1
         for (int c = 0; c < T2_HALF / 32; ++c) {
@@ -292,7 +300,26 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             __nv_bfloat16* hg = p.out ? reinterpret_cast<__nv_bfloat16*>(p.out) + tl.out_off + static_cast<size_t>(row) * p.ldc + col : nullptr;
             __nv_bfloat16* oa = reinterpret_cast<__nv_bfloat16*>(p.out2) + static_cast<size_t>(row) * p.ldc2 + col;
 #pragma unroll
-            for (int j = 0; j < 32; j += 8) {
+            for (int jw = 0; jw < 32; jw += 16) {
+              if (wide && col + jw + 16 <= glu) {
+                uint32_t gw[8], uw[8], aw[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                  gw[e] = pack_bf16x2(__uint_as_float(rg[jw + 2 * e]) * alpha, __uint_as_float(rg[jw + 2 * e + 1]) * alpha);
+                  uw[e] = pack_bf16x2(__uint_as_float(ru[jw + 2 * e]) * alpha, __uint_as_float(ru[jw + 2 * e + 1]) * alpha);
+                  const float2 g2 = unpack_bf16x2(gw[e]), u2 = unpack_bf16x2(uw[e]);
+                  aw[e] = pack_bf16x2(g2.x * (1.f / (1.f + __expf(-g2.x))) * u2.x, g2.y * (1.f / (1.f + __expf(-g2.y))) * u2.y);
+                }
+                if (hg) {
+                  store_32b(hg + jw, gw);
+                  store_32b(hg + glu + jw, uw);
+                }
+                store_32b(oa + jw, aw);
+                continue;
+              }
+#pragma unroll
+            for (int jj = 0; jj < 16; jj += 8) {
+              const int j = jw + jj;
               if (col + j < glu) {
                 uint32_t gw[4], uw[4], aw[4];
 #pragma unroll
@@ -308,6 +335,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
                 }
                 *reinterpret_cast<uint4*>(oa + j) = make_uint4(aw[0], aw[1], aw[2], aw[3]);
               }
+            }
             }
           } else if (row < row_limit && col < glu) {    // expert without rows: nothing was accumulated
             __nv_bfloat16* oa = reinterpret_cast<__nv_bfloat16*>(p.out2) + static_cast<size_t>(row) * p.ldc2 + col;
@@ -328,21 +356,36 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         if (row < row_limit && col < p.N) {
           if (OUT_F32) {
             float* o = reinterpret_cast<float*>(p.out) + tl.out_off + static_cast<size_t>(row) * p.ldc + col;
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              if (col + j < p.N) {
-                float4 v = make_float4(__uint_as_float(r[j]) * alpha, __uint_as_float(r[j + 1]) * alpha,
-                                       __uint_as_float(r[j + 2]) * alpha, __uint_as_float(r[j + 3]) * alpha);
-                if (acc_flag) {
-                  const float4 old = *reinterpret_cast<const float4*>(o + j);
-                  v.x += old.x; v.y += old.y; v.z += old.z; v.w += old.w;
-                }
-                *reinterpret_cast<float4*>(o + j) = v;
-              }
-            }
+            store_row32(o, r, alpha, acc_flag, p.N - col, wide);
           } else {
             __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + tl.out_off + static_cast<size_t>(row) * p.ldc + col;
             const __nv_bfloat16* ci = p.cin ? reinterpret_cast<const __nv_bfloat16*>(p.cin) + tl.out_off + static_cast<size_t>(row) * p.ldc + col : nullptr;
+            if (wide && col + 32 <= p.N) {
+              uint32_t cw[2][8];
+              if (ci) { load_32b(ci, cw[0]); load_32b(ci + 16, cw[1]); }
+#pragma unroll
+              for (int j = 0; j < 32; j += 16) {
+                float f[16];
+                uint32_t v[8];
+#pragma unroll
+                for (int e = 0; e < 16; ++e) f[e] = __uint_as_float(r[j + e]) * alpha;
+                if (ci) {
+#pragma unroll
+                  for (int e = 0; e < 8; ++e) {
+                    const float2 c2 = unpack_bf16x2(cw[j / 16][e]);
+                    f[2 * e] += beta * c2.x; f[2 * e + 1] += beta * c2.y;
+                  }
+                }
+#pragma unroll
+                for (int e = 0; e < 8; ++e) v[e] = pack_bf16x2(f[2 * e], f[2 * e + 1]);
+                store_32b(o + j, v);
+                if (GROUPED == 3 && sym && n0 != m0) {      // transposed copy: lanes hold consecutive rows → 64-byte segments
+                  __nv_bfloat16* ot = reinterpret_cast<__nv_bfloat16*>(p.out) + tl.out_off + static_cast<size_t>(col + j) * p.ldc + row;
+#pragma unroll
+                  for (int e = 0; e < 16; ++e) ot[static_cast<size_t>(e) * p.ldc] = __float2bfloat16_rn(f[e]);
+                }
+              }
+            } else
 #pragma unroll
             for (int j = 0; j < 32; j += 8) {
               if (col + j < p.N) {

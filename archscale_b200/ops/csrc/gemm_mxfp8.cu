@@ -180,6 +180,7 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     }
   } else {
     const int q = warp & 3;
+    const bool wide = p.ldc % (OUT_F32 ? 8 : 16) == 0 && reinterpret_cast<uintptr_t>(p.out) % 32 == 0;   // whole sectors per lane
     int it = 0;
     for (int t = cta; t < num_tiles; t += n_cta, ++it) {
       int m0, n0; tile_coords(t, m0, n0);
@@ -199,34 +200,9 @@ gemm_mxfp8_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         }
         const int col = n0 + c * 32;
         if (row < p.M && col < p.N) {
-          if (OUT_F32) {
-            float* o = reinterpret_cast<float*>(p.out) + static_cast<size_t>(row) * p.ldc + col;
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              if (col + j < p.N) {
-                float4 v = make_float4(__uint_as_float(r[j]) * p.alpha, __uint_as_float(r[j + 1]) * p.alpha,
-                                       __uint_as_float(r[j + 2]) * p.alpha, __uint_as_float(r[j + 3]) * p.alpha);
-                if (p.accumulate) {
-                  const float4 old = *reinterpret_cast<const float4*>(o + j);
-                  v.x += old.x; v.y += old.y; v.z += old.z; v.w += old.w;
-                }
-                *reinterpret_cast<float4*>(o + j) = v;
-              }
-            }
-          } else {
-            __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + static_cast<size_t>(row) * p.ldc + col;
-#pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              if (col + j < p.N) {
-                uint4 ov;
-                ov.x = pack_bf16x2(__uint_as_float(r[j]) * p.alpha, __uint_as_float(r[j + 1]) * p.alpha);
-                ov.y = pack_bf16x2(__uint_as_float(r[j + 2]) * p.alpha, __uint_as_float(r[j + 3]) * p.alpha);
-                ov.z = pack_bf16x2(__uint_as_float(r[j + 4]) * p.alpha, __uint_as_float(r[j + 5]) * p.alpha);
-                ov.w = pack_bf16x2(__uint_as_float(r[j + 6]) * p.alpha, __uint_as_float(r[j + 7]) * p.alpha);
-                *reinterpret_cast<uint4*>(o + j) = ov;
-              }
-            }
-          }
+          const size_t at = static_cast<size_t>(row) * p.ldc + col;
+          if (OUT_F32) store_row32(reinterpret_cast<float*>(p.out) + at, r, p.alpha, p.accumulate, p.N - col, wide);
+          else store_row32(reinterpret_cast<__nv_bfloat16*>(p.out) + at, r, p.alpha, p.N - col, wide);
         }
       }
       tc_fence_before();
@@ -551,6 +527,7 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
     }
   } else {
     const int q = warp & 3;
+    const bool wide = p.ldc % (OUT_F32 ? 8 : 16) == 0 && reinterpret_cast<uintptr_t>(p.out) % 32 == 0;   // whole sectors per lane
     const float alpha = p.alpha * __fmul_rn(nvfp4_tensor_scale(*amax_a), nvfp4_tensor_scale(*amax_b));
     int it = 0;
     for (int t = cta; t < num_tiles; t += n_cta, ++it) {
@@ -571,34 +548,9 @@ gemm_nvfp4_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
         }
         const int col = n0 + c * 32;
         if (row < p.M && col < p.N) {
-          if (OUT_F32) {
-            float* o = reinterpret_cast<float*>(p.out) + static_cast<size_t>(row) * p.ldc + col;
-#pragma unroll
-            for (int j = 0; j < 32; j += 4) {
-              if (col + j < p.N) {
-                float4 v = make_float4(__uint_as_float(r[j]) * alpha, __uint_as_float(r[j + 1]) * alpha,
-                                       __uint_as_float(r[j + 2]) * alpha, __uint_as_float(r[j + 3]) * alpha);
-                if (p.accumulate) {
-                  const float4 old = *reinterpret_cast<const float4*>(o + j);
-                  v.x += old.x; v.y += old.y; v.z += old.z; v.w += old.w;
-                }
-                *reinterpret_cast<float4*>(o + j) = v;
-              }
-            }
-          } else {
-            __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + static_cast<size_t>(row) * p.ldc + col;
-#pragma unroll
-            for (int j = 0; j < 32; j += 8) {
-              if (col + j < p.N) {
-                uint4 ov;
-                ov.x = pack_bf16x2(__uint_as_float(r[j]) * alpha, __uint_as_float(r[j + 1]) * alpha);
-                ov.y = pack_bf16x2(__uint_as_float(r[j + 2]) * alpha, __uint_as_float(r[j + 3]) * alpha);
-                ov.z = pack_bf16x2(__uint_as_float(r[j + 4]) * alpha, __uint_as_float(r[j + 5]) * alpha);
-                ov.w = pack_bf16x2(__uint_as_float(r[j + 6]) * alpha, __uint_as_float(r[j + 7]) * alpha);
-                *reinterpret_cast<uint4*>(o + j) = ov;
-              }
-            }
-          }
+          const size_t at = static_cast<size_t>(row) * p.ldc + col;
+          if (OUT_F32) store_row32(reinterpret_cast<float*>(p.out) + at, r, alpha, p.accumulate, p.N - col, wide);
+          else store_row32(reinterpret_cast<__nv_bfloat16*>(p.out) + at, r, alpha, p.N - col, wide);
         }
       }
       tc_fence_before();

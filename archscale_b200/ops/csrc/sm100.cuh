@@ -389,6 +389,69 @@ __device__ __forceinline__ float2 add_f32x2(float2 a, float2 b) {
   return unpack_f32x2(r);
 }
 
+// ------------------------------------------------------------------ 32-byte global accesses (32-byte aligned)
+// A whole sector per lane: rows that lie far apart cost a store half the passes of 16-byte accesses.
+__device__ __forceinline__ void store_32b(void* dst, const uint32_t (&w)[8]) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(dst), "r"(w[0]), "r"(w[1]), "r"(w[2]), "r"(w[3]),
+               "r"(w[4]), "r"(w[5]), "r"(w[6]), "r"(w[7]) : "memory");
+}
+__device__ __forceinline__ void load_32b(const void* src, uint32_t (&w)[8]) {
+  asm volatile("ld.global.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];" : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]),
+               "=r"(w[5]), "=r"(w[6]), "=r"(w[7]) : "l"(src) : "memory");
+}
+
+// 32 columns of one output row, alpha · r (+ what is there with `accumulate`), n ≤ 32 of them inside the matrix (n a multiple of 8
+// for bf16 and of 4 for fp32).  `wide`: the row's address at these columns is a multiple of 32 bytes.
+__device__ __forceinline__ void store_row32(float* o, const uint32_t (&r)[32], float alpha, int accumulate, int n, bool wide) {
+  if (wide && n >= 32) {
+    uint32_t old[4][8];
+    if (accumulate) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) load_32b(o + 8 * j, old[j]);
+    }
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      uint32_t v[8];
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        const float x = __uint_as_float(r[8 * j + e]) * alpha;
+        v[e] = __float_as_uint(accumulate ? x + __uint_as_float(old[j][e]) : x);
+      }
+      store_32b(o + 8 * j, v);
+    }
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < 32; j += 4) {
+    if (j < n) {
+      float4 v = make_float4(__uint_as_float(r[j]) * alpha, __uint_as_float(r[j + 1]) * alpha, __uint_as_float(r[j + 2]) * alpha,
+                             __uint_as_float(r[j + 3]) * alpha);
+      if (accumulate) {
+        const float4 old = *reinterpret_cast<const float4*>(o + j);
+        v.x += old.x; v.y += old.y; v.z += old.z; v.w += old.w;
+      }
+      *reinterpret_cast<float4*>(o + j) = v;
+    }
+  }
+}
+__device__ __forceinline__ void store_row32(__nv_bfloat16* o, const uint32_t (&r)[32], float alpha, int n, bool wide) {
+  uint32_t v[16];
+#pragma unroll
+  for (int e = 0; e < 16; ++e) {
+    __nv_bfloat162 b = __floats2bfloat162_rn(__uint_as_float(r[2 * e]) * alpha, __uint_as_float(r[2 * e + 1]) * alpha);
+    v[e] = *reinterpret_cast<uint32_t*>(&b);
+  }
+  if (wide && n >= 32) {
+    const uint32_t a[8] = {v[0], v[1], v[2], v[3], v[4], v[5], v[6], v[7]}, b[8] = {v[8], v[9], v[10], v[11], v[12], v[13], v[14], v[15]};
+    store_32b(o, a);
+    store_32b(o + 16, b);
+    return;
+  }
+#pragma unroll
+  for (int j = 0; j < 4; ++j)
+    if (8 * j < n) *reinterpret_cast<uint4*>(o + 8 * j) = make_uint4(v[4 * j], v[4 * j + 1], v[4 * j + 2], v[4 * j + 3]);
+}
+
 // ------------------------------------------------------------------ misc
 __device__ __forceinline__ uint32_t ld_acquire_gpu(const uint32_t* p) {
   uint32_t v;
