@@ -15,8 +15,12 @@
 //
 // The value columns of the state are independent, so a CTA owns 128 of them for one (batch, head): X lives in
 // tensor memory as a 128-lane × Dk fp32 accumulator for the whole sequence, a bf16 copy of it sits beside it as
-// the A operand of P = X·Aᵀ (tcgen05.mma with A from tensor memory), and the four epilogue warps (one TMEM lane
-// quarter each, thread = value column) turn P into V, rescale X by the next chunk's decay and emit both.
+// the A operand of P = X·Aᵀ (tcgen05.mma with A from tensor memory), and eight epilogue warps (two per TMEM lane
+// quarter, thread = value column) turn P into V, rescale X by the next chunk's decay and emit both.  A chunk is one chain
+// P -> V -> X -> next P, so its length sets the time: the two warps of a quarter halve both epilogue phases, and states
+// leave in 32-byte pieces per lane.  ms per
+// pass, forward / reversed, before and after both: B1 T4096 H6 Dk256 Dv512 0.341 / 0.351 -> 0.312 / 0.323, B8 0.747 / 0.769 -> 0.634 /
+// 0.652 (the stores alone 0.324 / 0.337 and 0.648 / 0.663).
 // A / Bm / E / F tiles arrive by TMA into 128-byte-swizzled shared memory; C and V move with plain loads / stores
 // (64 bytes per warp and token).  Every wait is bounded.
 #include "sm100.cuh"
@@ -29,7 +33,7 @@ int make_tmap_2d_bf16(CUtensorMap* map, const void* ptr, uint64_t inner, uint64_
 
 constexpr int GC = 64;             // chunk length (tokens)
 constexpr int GDV = 128;           // value columns per CTA = TMEM lanes
-constexpr int GDN_THREADS = 192;   // warp 0 TMA, warp 1 MMA, warps 2..5 epilogue
+constexpr int GDN_THREADS = 320;   // warp 0 TMA, warp 1 MMA, warps 2..9 epilogue (two per TMEM lane quarter)
 constexpr int GCH = GC * 64 * 2;   // one [64 tokens × 64 columns] bf16 shared-memory chunk
 
 struct GdnParams {
@@ -71,9 +75,9 @@ gdn_state_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   uint64_t* ef_full = bars + 4;
   uint64_t* ef_empty = bars + 5;
   uint64_t* bar_p = bars + 6;      // P of this step is in tensor memory
-  uint64_t* bar_v = bars + 7;      // (count 4) sgn_v·Vᵀ is in shared memory, P has been read
+  uint64_t* bar_v = bars + 7;      // (count 8) sgn_v·Vᵀ is in shared memory, P has been read
   uint64_t* bar_x = bars + 8;      // the state update of this step has completed
-  uint64_t* bar_xb = bars + 9;     // (count 4) bf16 X written, fp32 X rescaled for the next step
+  uint64_t* bar_xb = bars + 9;     // (count 8) bf16 X written, fp32 X rescaled for the next step
   uint32_t* tmem_ptr = reinterpret_cast<uint32_t*>(bars + 10);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_ptr + 1);
 
@@ -84,7 +88,7 @@ gdn_state_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
   if (threadIdx.x == 0) {
     for (int s = 0; s < 2; ++s) { mbar_init(&ab_full[s], 1); mbar_init(&ab_empty[s], 1); }
     mbar_init(ef_full, 1); mbar_init(ef_empty, 1);
-    mbar_init(bar_p, 1); mbar_init(bar_v, 4); mbar_init(bar_x, 1); mbar_init(bar_xb, 4);
+    mbar_init(bar_p, 1); mbar_init(bar_v, 8); mbar_init(bar_x, 1); mbar_init(bar_xb, 8);
     *abort_flag = 0;
     mbar_fence_init();
   }
@@ -155,6 +159,7 @@ gdn_state_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
     }
   } else {
     const int q = warp & 3;                              // TMEM lane quarter of this warp
+    const int half = (warp - 2) >> 2;                    // it does tokens 32·half.. of P and columns DK/2·half.. of X
     const int row = q * 32 + lane;                       // value column inside the CTA's block
     const uint32_t lane_off = static_cast<uint32_t>(q * 32) << 16;
     const size_t dvcol = static_cast<size_t>(dvb) * GDV + row;
@@ -164,10 +169,10 @@ gdn_state_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
 #pragma unroll
       for (int e = 0; e < 16; ++e) z[e] = 0u;
 #pragma unroll
-      for (int c = 0; c < (DK + DK / 2) / 16; ++c) tmem_st_32x16(T_X + c * 16 + lane_off, z);
+      for (int c = 0; c < (DK + DK / 2) / 32; ++c) tmem_st_32x16(T_X + (half * ((DK + DK / 2) / 32) + c) * 16 + lane_off, z);
       uint4* xr = reinterpret_cast<uint4*>(p.x_all + ((static_cast<size_t>(bh) * nC + n_first) * p.DV + dvcol) * DK);
 #pragma unroll
-      for (int e = 0; e < DK / 8; ++e) xr[e] = make_uint4(0u, 0u, 0u, 0u);
+      for (int e = 0; e < DK / 16; ++e) xr[half * (DK / 16) + e] = make_uint4(0u, 0u, 0u, 0u);
       tmem_st_wait();
       tc_fence_before();
       __syncwarp();
@@ -178,22 +183,21 @@ gdn_state_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
       const size_t tok0 = static_cast<size_t>(bh) * p.Tp + static_cast<size_t>(n) * GC;
       const unsigned short* crow = reinterpret_cast<const unsigned short*>(p.c_add) + tok0 * p.DV + dvcol;
       unsigned short* vrow = reinterpret_cast<unsigned short*>(p.v_out) + tok0 * p.DV + dvcol;
-      unsigned short cv[GC];
+      unsigned short cv[GC / 2];
 #pragma unroll
-      for (int i = 0; i < GC; ++i) cv[i] = __ldg(crow + static_cast<size_t>(i) * p.DV);
+      for (int i = 0; i < GC / 2; ++i) cv[i] = __ldg(crow + static_cast<size_t>(half * (GC / 2) + i) * p.DV);
       if (!mbar_wait(bar_p, s & 1, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL)) goto done;
       tc_fence_after();
-#pragma unroll
-      for (int hh = 0; hh < 2; ++hh) {
+      {
         uint32_t pr[32];
-        tmem_ld_32x32(T_P + hh * 32 + lane_off, pr);
+        tmem_ld_32x32(T_P + half * 32 + lane_off, pr);
         tmem_ld_wait();
         uint32_t w[16];
 #pragma unroll
         for (int e = 0; e < 16; ++e) {
-          const int i = hh * 32 + 2 * e;
-          const float v0 = __bfloat162float(__ushort_as_bfloat16(cv[i])) + p.sgn_p * __uint_as_float(pr[2 * e]);
-          const float v1 = __bfloat162float(__ushort_as_bfloat16(cv[i + 1])) + p.sgn_p * __uint_as_float(pr[2 * e + 1]);
+          const int i = half * 32 + 2 * e;                 // token
+          const float v0 = __bfloat162float(__ushort_as_bfloat16(cv[2 * e])) + p.sgn_p * __uint_as_float(pr[2 * e]);
+          const float v1 = __bfloat162float(__ushort_as_bfloat16(cv[2 * e + 1])) + p.sgn_p * __uint_as_float(pr[2 * e + 1]);
           const __nv_bfloat16 b0 = __float2bfloat16_rn(v0), b1 = __float2bfloat16_rn(v1);
           vrow[static_cast<size_t>(i) * p.DV] = __bfloat16_as_ushort(b0);
           vrow[static_cast<size_t>(i + 1) * p.DV] = __bfloat16_as_ushort(b1);
@@ -202,7 +206,7 @@ gdn_state_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
         // row `row` of the K-major operand: 16-byte piece j (8 tokens) sits at slot j ^ (row % 8) of the 128-byte row
 #pragma unroll
         for (int jj = 0; jj < 4; ++jj) {
-          const int j = hh * 4 + jj;
+          const int j = half * 4 + jj;
           *reinterpret_cast<uint4*>(svb + row * 128 + ((j ^ (row & 7)) << 4)) =
               make_uint4(w[4 * jj], w[4 * jj + 1], w[4 * jj + 2], w[4 * jj + 3]);
         }
@@ -221,7 +225,7 @@ gdn_state_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
                        : reinterpret_cast<uint4*>(p.x_all + ((static_cast<size_t>(bh) * nC + nn) * p.DV + dvcol) * DK);
       float* xf = (last && p.x_final) ? p.x_final + (static_cast<size_t>(bh) * p.DV + dvcol) * DK : nullptr;
 #pragma unroll 2
-      for (int c = 0; c < DK / 32; ++c) {
+      for (int c = half * (DK / 64); c < (half + 1) * (DK / 64); ++c) {
         uint32_t xv[32];
         tmem_ld_32x32(T_X + c * 32 + lane_off, xv);
         tmem_ld_wait();
@@ -231,7 +235,10 @@ gdn_state_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
           for (int e = 0; e < 16; ++e) xb[e] = pack_bf16x2(__uint_as_float(xv[2 * e]), __uint_as_float(xv[2 * e + 1]));
           tmem_st_32x16(T_XB + c * 16 + lane_off, xb);
 #pragma unroll
-          for (int e = 0; e < 4; ++e) xr[c * 4 + e] = make_uint4(xb[4 * e], xb[4 * e + 1], xb[4 * e + 2], xb[4 * e + 3]);
+          for (int e = 0; e < 2; ++e) {                    // 512 bytes of a row per lane: whole sectors per store
+            const uint32_t v[8] = {xb[8 * e], xb[8 * e + 1], xb[8 * e + 2], xb[8 * e + 3], xb[8 * e + 4], xb[8 * e + 5], xb[8 * e + 6], xb[8 * e + 7]};
+            store_32b(xr + c * 4 + 2 * e, v);
+          }
           uint32_t lo[16], hi[16];
 #pragma unroll
           for (int e = 0; e < 16; ++e) {
