@@ -25,12 +25,25 @@ import torch
 from . import backend
 
 
-def _cuda_ok(a: torch.Tensor, b: torch.Tensor, M: int, N: int, K: int) -> bool:
-    return (a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and K % 8 == 0 and N % 8 == 0 and M % 8 == 0
-            and K >= 64 and M >= 1 and a.dim() == 2 and b.dim() == 2
+def _operands_ok(a: torch.Tensor, b: torch.Tensor) -> bool:
+    return (a.dtype == torch.bfloat16 and b.dtype == torch.bfloat16 and a.dim() == 2 and b.dim() == 2
             and a.stride(-1) == 1 and b.stride(-1) == 1
             and a.stride(0) % 8 == 0 and b.stride(0) % 8 == 0
             and a.data_ptr() % 16 == 0 and b.data_ptr() % 16 == 0)
+
+
+def _cuda_ok(a: torch.Tensor, b: torch.Tensor, M: int, N: int, K: int) -> bool:
+    """Operands of ``y[M,N]`` with K products each: feature counts N and K multiples of 8 (rows of 16-byte multiples), any number
+    of rows (tokens) M.  Whole training steps, ms, token counts that are no multiple of 8 through the library (whose weight
+    gradient is a bf16 tensor to be added to the fp32 buffer, and which leaves SwiGLU to a kernel of its own) / through the own
+    GEMM: dense 8 layers 1001 tokens 13.6 / 11.5, 4001 13.7 / 12.2, 16385 38.5 / 38.5; dense 16 layers 8191 92.9 / 88.5; hybrids of
+    16 layers 2001 to 8193 tokens 69.3 / 64.8 to 104.8 / 100.5."""
+    return K % 8 == 0 and N % 8 == 0 and K >= 64 and M >= 1 and _operands_ok(a, b)
+
+
+def _cuda_ok_tn(a: torch.Tensor, b: torch.Tensor, M: int, N: int, K: int) -> bool:
+    """The same for a weight gradient, whose K is the number of rows (tokens)."""
+    return M % 8 == 0 and N % 8 == 0 and K >= 64 and M >= 1 and _operands_ok(a, b)
 
 
 def matmul_nt(a: torch.Tensor, b: torch.Tensor, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
@@ -59,7 +72,7 @@ def matmul_tn(a: torch.Tensor, b: torch.Tensor, out_dtype: Optional[torch.dtype]
     """a:(K,M) b:(K,N) → aᵀ @ b : (M,N)."""
     K, M = a.shape
     N = b.shape[1]
-    if _cuda_ok(a, b, M, N, K) and backend.use_cuda_kernel("gemm", a, b):
+    if _cuda_ok_tn(a, b, M, N, K) and backend.use_cuda_kernel("gemm", a, b):
         backend.count_launch()
         return backend.require_extension().gemm_bf16(a, b, 2, out_dtype or torch.bfloat16, None)
     out = a.t() @ b
@@ -70,7 +83,7 @@ def matmul_tn_acc_(c: torch.Tensor, a: torch.Tensor, b: torch.Tensor) -> torch.T
     """c (fp32, (M,N)) += aᵀ @ b with a:(K,M), b:(K,N)."""
     K, M = a.shape
     N = b.shape[1]
-    if c.dtype == torch.float32 and c.is_contiguous() and _cuda_ok(a, b, M, N, K) and backend.use_cuda_kernel("gemm", a, b, c):
+    if c.dtype == torch.float32 and c.is_contiguous() and _cuda_ok_tn(a, b, M, N, K) and backend.use_cuda_kernel("gemm", a, b, c):
         backend.count_launch()
         backend.require_extension().gemm_bf16(a, b, 2, torch.float32, c)
         return c
@@ -91,7 +104,7 @@ class _LinearFn(torch.autograd.Function):
         g = getattr(weight, "_fsdp_group", None)
         if g is not None and getattr(g, "ag_pending", False):
             eng = weight._fsdp_engine
-            if weight._fsdp_first and _cuda_ok(x2, weight, x2.shape[0], weight.shape[0], x2.shape[1]):
+            if weight._fsdp_first and x2.shape[0] % 8 == 0 and _cuda_ok(x2, weight, x2.shape[0], weight.shape[0], x2.shape[1]):
                 # FSDP forward: this GEMM also gathers the unit's matrix parameters from all ranks
                 g.ag_pending = False
                 y = eng.symm.ag_gemm(x2, g, weight.shape[0])
@@ -200,7 +213,7 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor) -> Optional[torch.Tenso
         return _skinny(x, [weight], True)
     if not (x.is_cuda and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and weight.dim() == 2
             and weight.shape[0] % 16 == 0 and x.shape[-1] % 8 == 0 and x.shape[-1] >= 64
-            and (x.numel() // x.shape[-1]) % 8 == 0 and weight.stride(-1) == 1 and weight.stride(0) % 8 == 0
+            and x.numel() > 0 and weight.stride(-1) == 1 and weight.stride(0) % 8 == 0
             and weight.data_ptr() % 16 == 0 and fused_swiglu_enabled() and backend.use_cuda_kernel("gemm", x, weight)):
         return None
     g = getattr(weight, "_fsdp_group", None)
@@ -217,7 +230,7 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
         return _skinny(x, [weight], False)
     if (x.is_cuda and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16
             and x.shape[-1] % 8 == 0 and weight.shape[0] % 8 == 0 and x.shape[-1] >= 64
-            and (x.numel() // x.shape[-1]) % 8 == 0
+            and x.numel() > 0
             and backend.use_cuda_kernel("gemm", x, weight)):
         if not x.is_contiguous():
             x = x.contiguous()
@@ -246,7 +259,7 @@ def linear_widened(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
     """``x @ weightᵀ`` for feature counts that are no multiple of 8 (dt_rank = 124 at 1984 channels): both operands are widened
     with zeros to the next multiple of 8, so that every row of the product and of its two gradients starts on a 16-byte boundary
     (unaligned rows leave the library only its sm_80 kernels with element-wise loads: 4.6 ms of a step with five such layers at
-    4 x 4096 tokens).  Token counts that are a multiple of 8 then run the tcgen05 GEMM, others the library on the widened operands.
+    4 x 4096 tokens).
     The result is a view of the widened product's first columns."""
     k, n = -x.shape[-1] % 8, -weight.shape[0] % 8
     y = linear(torch.nn.functional.pad(x, (0, k)) if k else x, torch.nn.functional.pad(weight, (0, k, 0, n)))
@@ -279,7 +292,7 @@ class _MultiLinearFn(torch.autograd.Function):
         g = getattr(weights[0], "_fsdp_group", None)
         if g is not None and getattr(g, "ag_pending", False):
             eng = weights[0]._fsdp_engine
-            if weights[0]._fsdp_first and _cuda_ok(x2, w_cat, x2.shape[0], w_cat.shape[0], x2.shape[1]):
+            if weights[0]._fsdp_first and x2.shape[0] % 8 == 0 and _cuda_ok(x2, w_cat, x2.shape[0], w_cat.shape[0], x2.shape[1]):
                 g.ag_pending = False
                 y = eng.symm.ag_gemm(x2, g, w_cat.shape[0])
             else:
@@ -328,7 +341,7 @@ def linear_multi(x: torch.Tensor, layers, keep_fused: bool = False):
     fusable = (x.is_cuda and x.dtype == torch.bfloat16 and all(type(l).__name__ == "Linear" and l.bias is None and not l.mxfp8
                                                               and not getattr(l, "nvfp4", False) for l in layers)
                and all(w.dtype == torch.bfloat16 for w in ws) and _adjacent(ws)
-               and (x.numel() // x.shape[-1]) % 8 == 0 and x.shape[-1] % 8 == 0 and x.shape[-1] >= 64
+               and x.numel() > 0 and x.shape[-1] % 8 == 0 and x.shape[-1] >= 64
                and backend.use_cuda_kernel("gemm", x, ws[0]))
     if not fusable:
         return [l(x) for l in layers]
