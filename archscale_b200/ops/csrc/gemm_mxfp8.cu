@@ -261,84 +261,93 @@ __global__ void __launch_bounds__(256) mxfp8_quant_rowwise_kernel(const __nv_bfl
   }
   const uint32_t ex = e8m0_for_amax(amax);
   const float inv = __uint_as_float((254u - ex) << 23);
-  uint4* dst = reinterpret_cast<uint4*>(q + static_cast<size_t>(r) * C + kb * 32);
+  uint32_t o[8];
 #pragma unroll
-  for (int i = 0; i < 2; ++i) {
-    uint4 o;
-    o.x = cvt4_e4m3(v[i * 16 + 0] * inv, v[i * 16 + 1] * inv, v[i * 16 + 2] * inv, v[i * 16 + 3] * inv);
-    o.y = cvt4_e4m3(v[i * 16 + 4] * inv, v[i * 16 + 5] * inv, v[i * 16 + 6] * inv, v[i * 16 + 7] * inv);
-    o.z = cvt4_e4m3(v[i * 16 + 8] * inv, v[i * 16 + 9] * inv, v[i * 16 + 10] * inv, v[i * 16 + 11] * inv);
-    o.w = cvt4_e4m3(v[i * 16 + 12] * inv, v[i * 16 + 13] * inv, v[i * 16 + 14] * inv, v[i * 16 + 15] * inv);
-    dst[i] = o;
-  }
+  for (int i = 0; i < 8; ++i) o[i] = cvt4_e4m3(v[4 * i] * inv, v[4 * i + 1] * inv, v[4 * i + 2] * inv, v[4 * i + 3] * inv);
+  store_32b(q + static_cast<size_t>(r) * C + kb * 32, o);
   sf[sf_offset(r, kb, nblk >> 2)] = static_cast<uint8_t>(ex);
 }
 
+// 32 packed bf16 pairs → the larger magnitude per half.  (Magnitudes and maxima of bf16 values are exact.)  NaN is dropped, as
+// fmaxf drops it.
+__device__ __forceinline__ __nv_bfloat162 absmax2(__nv_bfloat162 m, uint32_t v) {
+  return __hmax2(m, __habs2(*reinterpret_cast<const __nv_bfloat162*>(&v)));
+}
 // Column-wise: writes the transposed operand qT [C, R] with scale blocks along R; with ROWS it also writes the row-wise
 // operand q [R, C] from the same shared-memory tile (one read of a tensor that is needed in both orientations).
 // R % 128 == 0, C % 64 == 0 (ROWS: C % 128 == 0).
+// Memory-bound: 2 bytes read and 2 (ROWS) written per element.  Half of the threads take two neighbouring columns each (a pair
+// per shared-memory load, magnitudes compared two at a time), the other half two row blocks each; a block of 32 bytes is one
+// store and the four scale bytes of a column one word.  ms, both orientations, one column per thread and 16-byte stores / this form:
+// 16384x2048 0.041 / 0.035, 16384x11264 0.186 / 0.152 (4.8 TB/s).
 template <int ROWS>
-__global__ void __launch_bounds__(256) mxfp8_quant_colwise_kernel(const __nv_bfloat16* __restrict__ x, int ld,
+__global__ void __launch_bounds__(ROWS ? 256 : 128) mxfp8_quant_colwise_kernel(const __nv_bfloat16* __restrict__ x, int ld,
                                                                  uint8_t* __restrict__ qT, uint8_t* __restrict__ sfT,
                                                                  uint8_t* __restrict__ q, uint8_t* __restrict__ sf, int R, int C) {
+  constexpr int NTHR = ROWS ? 256 : 128;
   __shared__ __align__(16) __nv_bfloat16 s[128][72];
+  __shared__ uint32_t s_sf[64];                       // scale bytes of a column's four blocks
   const int r0 = blockIdx.y * 128, c0 = blockIdx.x * 64, tid = threadIdx.x;
 #pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int idx = tid + 256 * i, row = idx >> 3, cv = idx & 7;
+  for (int i = 0; i < 1024 / NTHR; ++i) {
+    const int idx = tid + NTHR * i, row = idx >> 3, cv = idx & 7;
     const uint4 u = *reinterpret_cast<const uint4*>(x + static_cast<size_t>(r0 + row) * ld + c0 + cv * 8);
     *reinterpret_cast<uint4*>(&s[row][cv * 8]) = u;
   }
   __syncthreads();
-  {
-    const int c = tid & 63, rb = tid >> 6;
-    float v[32];
-    float amax = 0.f;
+  if (tid < 128) {
+    const int cp = (tid & 31) * 2, rb = tid >> 5;      // columns cp, cp + 1; rows 32·rb ..
+    uint32_t v[32];
+    __nv_bfloat162 m = __float2bfloat162_rn(0.f);
 #pragma unroll
-    for (int j = 0; j < 32; ++j) { v[j] = __bfloat162float(s[rb * 32 + j][c]); amax = fmaxf(amax, fabsf(v[j])); }
-    const uint32_t ex = e8m0_for_amax(amax);
-    const float inv = __uint_as_float((254u - ex) << 23);
-    uint4* dst = reinterpret_cast<uint4*>(qT + static_cast<size_t>(c0 + c) * R + r0 + rb * 32);
-#pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      uint4 o;
-      o.x = cvt4_e4m3(v[i * 16 + 0] * inv, v[i * 16 + 1] * inv, v[i * 16 + 2] * inv, v[i * 16 + 3] * inv);
-      o.y = cvt4_e4m3(v[i * 16 + 4] * inv, v[i * 16 + 5] * inv, v[i * 16 + 6] * inv, v[i * 16 + 7] * inv);
-      o.z = cvt4_e4m3(v[i * 16 + 8] * inv, v[i * 16 + 9] * inv, v[i * 16 + 10] * inv, v[i * 16 + 11] * inv);
-      o.w = cvt4_e4m3(v[i * 16 + 12] * inv, v[i * 16 + 13] * inv, v[i * 16 + 14] * inv, v[i * 16 + 15] * inv);
-      dst[i] = o;
+    for (int j = 0; j < 32; ++j) {
+      v[j] = *reinterpret_cast<const uint32_t*>(&s[rb * 32 + j][cp]);
+      m = absmax2(m, v[j]);
     }
-    sfT[sf_offset(c0 + c, (r0 >> 5) + rb, R >> 7)] = static_cast<uint8_t>(ex);
-  }
-  if (ROWS) {
-    const int row = tid >> 1, blk = tid & 1;                              // 128 rows × 2 blocks of 32 columns
-    float v[32];
-    float amax = 0.f;
+    const uint32_t ex0 = e8m0_for_amax(__low2float(m)), ex1 = e8m0_for_amax(__high2float(m));
+    const float i0 = __uint_as_float((254u - ex0) << 23), i1 = __uint_as_float((254u - ex1) << 23);
+    uint32_t o0[8], o1[8];
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const uint4 u = *reinterpret_cast<const uint4*>(&s[row][blk * 32 + i * 8]);
-      const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+    for (int i = 0; i < 8; ++i) {
+      const float2 f0 = unpack_bf16x2(v[4 * i]), f1 = unpack_bf16x2(v[4 * i + 1]), f2 = unpack_bf16x2(v[4 * i + 2]), f3 = unpack_bf16x2(v[4 * i + 3]);
+      o0[i] = cvt4_e4m3(f0.x * i0, f1.x * i0, f2.x * i0, f3.x * i0);
+      o1[i] = cvt4_e4m3(f0.y * i1, f1.y * i1, f2.y * i1, f3.y * i1);
+    }
+    uint8_t* dst = qT + static_cast<size_t>(c0 + cp) * R + r0 + rb * 32;      // R % 128 == 0: multiples of 32 bytes
+    store_32b(dst, o0);
+    store_32b(dst + R, o1);
+    uint8_t* sb = reinterpret_cast<uint8_t*>(s_sf);
+    sb[cp * 4 + rb] = static_cast<uint8_t>(ex0);
+    sb[cp * 4 + 4 + rb] = static_cast<uint8_t>(ex1);
+  } else {
 #pragma unroll
-      for (int e = 0; e < 4; ++e) {
-        const float2 f = unpack_bf16x2(w[e]);
-        v[i * 8 + 2 * e] = f.x; v[i * 8 + 2 * e + 1] = f.y;
-        amax = fmaxf(amax, fmaxf(fabsf(f.x), fabsf(f.y)));
+    for (int h = 0; h < 2; ++h) {                      // 128 rows × 2 blocks of 32 columns
+      const int item = tid - 128 + 128 * h, row = item >> 1, blk = item & 1;
+      uint32_t v[16];
+      __nv_bfloat162 m = __float2bfloat162_rn(0.f);
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const uint4 u = *reinterpret_cast<const uint4*>(&s[row][blk * 32 + i * 8]);
+        v[4 * i] = u.x; v[4 * i + 1] = u.y; v[4 * i + 2] = u.z; v[4 * i + 3] = u.w;
+#pragma unroll
+        for (int e = 0; e < 4; ++e) m = absmax2(m, v[4 * i + e]);
       }
-    }
-    const uint32_t ex = e8m0_for_amax(amax);
-    const float inv = __uint_as_float((254u - ex) << 23);
-    uint4* dst = reinterpret_cast<uint4*>(q + static_cast<size_t>(r0 + row) * C + c0 + blk * 32);
+      const uint32_t ex = e8m0_for_amax(fmaxf(__low2float(m), __high2float(m)));
+      const float inv = __uint_as_float((254u - ex) << 23);
+      uint32_t o[8];
 #pragma unroll
-    for (int i = 0; i < 2; ++i) {
-      uint4 o;
-      o.x = cvt4_e4m3(v[i * 16 + 0] * inv, v[i * 16 + 1] * inv, v[i * 16 + 2] * inv, v[i * 16 + 3] * inv);
-      o.y = cvt4_e4m3(v[i * 16 + 4] * inv, v[i * 16 + 5] * inv, v[i * 16 + 6] * inv, v[i * 16 + 7] * inv);
-      o.z = cvt4_e4m3(v[i * 16 + 8] * inv, v[i * 16 + 9] * inv, v[i * 16 + 10] * inv, v[i * 16 + 11] * inv);
-      o.w = cvt4_e4m3(v[i * 16 + 12] * inv, v[i * 16 + 13] * inv, v[i * 16 + 14] * inv, v[i * 16 + 15] * inv);
-      dst[i] = o;
+      for (int i = 0; i < 8; ++i) {
+        const float2 f0 = unpack_bf16x2(v[2 * i]), f1 = unpack_bf16x2(v[2 * i + 1]);
+        o[i] = cvt4_e4m3(f0.x * inv, f0.y * inv, f1.x * inv, f1.y * inv);
+      }
+      store_32b(q + static_cast<size_t>(r0 + row) * C + c0 + blk * 32, o);
+      const uint32_t other = __shfl_xor_sync(0xffffffffu, ex, 1);             // the row's two blocks are neighbouring lanes
+      if (blk == 0)
+        *reinterpret_cast<uint16_t*>(sf + sf_offset(r0 + row, c0 >> 5, C >> 7)) = static_cast<uint16_t>(ex | (other << 8));
     }
-    sf[sf_offset(r0 + row, (c0 >> 5) + blk, C >> 7)] = static_cast<uint8_t>(ex);
   }
+  __syncthreads();
+  if (tid < 64) *reinterpret_cast<uint32_t*>(sfT + sf_offset(c0 + tid, r0 >> 5, R >> 7)) = s_sf[tid];
 }
 
 typedef CUresult (*EncodeTiledFnQ)(CUtensorMap*, CUtensorMapDataType, cuuint32_t, void*, const cuuint64_t*, const cuuint64_t*,
@@ -766,7 +775,7 @@ extern "C" int b200_mxfp8_quantize(const void* x, int ld, void* q, void* sf, int
         (const __nv_bfloat16*)x, ld, (uint8_t*)q, (uint8_t*)sf, R, C);
   } else if (colwise == 1) {
     if (R % 128 || C % 64) return -1;
-    mxfp8_quant_colwise_kernel<0><<<dim3(C / 64, R / 128), 256, 0, st>>>((const __nv_bfloat16*)x, ld, (uint8_t*)q, (uint8_t*)sf,
+    mxfp8_quant_colwise_kernel<0><<<dim3(C / 64, R / 128), 128, 0, st>>>((const __nv_bfloat16*)x, ld, (uint8_t*)q, (uint8_t*)sf,
                                                                          nullptr, nullptr, R, C);
   } else {
     if (R % 128 || C % 128 || !qT || !sfT) return -1;
