@@ -554,11 +554,8 @@ class ShardedOptimizer:
             stack = views[0] if len(views) == 1 else torch.cat(views)
             O = self._orthogonalise(stack)
             sq = torch.linalg.vector_norm(O, dim=(-2, -1), dtype=torch.float32).square()
-            i = 0
-            for gid, run in runs:
-                n = len(run)
-                staged[gid][2][run[0].offset:run[0].offset + n * r * c].view(n, r, c).copy_(O[i:i + n])
-                i += n
+            dst = [staged[gid][2][run[0].offset:run[0].offset + len(run) * r * c].view(len(run), r, c) for gid, run in runs]
+            torch._foreach_copy_(dst, list(O.split([len(run) for _, run in runs])))      # one launch instead of one per run
             idx = self._norm_idx_cache.get((r, c))
             if idx is None:
                 idx = self._norm_idx_cache[(r, c)] = torch.tensor([mt.norm_idx for _, run in runs for mt in run],
