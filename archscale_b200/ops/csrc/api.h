@@ -267,6 +267,13 @@ int b200_ssd_intra_bwd(const void* x, int x_dtype, const float* dt, const float*
                        float* dx, float* ddt, float* dcs, float* dCB, int B, int nC, int H, int G, int P, int hsplit, cudaStream_t st);
 // (I + A)^-1 for [n_mat, 64, 64] strictly lower-triangular fp32 matrices (tri_inverse.cu)
 int b200_tri_inverse64(const float* A, float* T, int n_mat, cudaStream_t st);
+// The 64×64 pieces of the chunked gated delta rule around the inverse (gdn_pieces.cu).
+int b200_gdn_mask_fwd(const float* Gk, const float* Gq, const float* gc, const float* beta, float* A, void* qk, int n, cudaStream_t st);
+int b200_gdn_mask_bwd(const float* dA, const void* dqk, const float* Gk, const float* Gq, const float* gc, const float* beta, void* dGk,
+                      void* dGq, float* dgc, float* dbeta, int n, cudaStream_t st);
+int b200_gdn_cols_fwd(const float* T, const float* gc, const float* beta, void* Tu, void* Tw, int n, cudaStream_t st);
+int b200_gdn_cols_bwd(const void* dTu, const void* dTw, const float* T, const float* gc, const float* beta, float* dT, float* dgc,
+                      float* dbeta, int n, cudaStream_t st);
 // One pass of the chunked gated-delta-rule recurrence (gdn_chunk.cu)
 int b200_gdn_state(const void* a_op, const void* c_add, const void* bm_op, const void* e_op, const void* f_op,
                    const float* decay, void* v_out, void* x_all, float* x_final, int BH, int Tp, int DK, int DV,

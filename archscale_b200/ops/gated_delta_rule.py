@@ -216,16 +216,56 @@ class _BmmNTf32(torch.autograd.Function):
         return gb @ b, gb.transpose(-1, -2) @ a
 
 
+class _MaskFn(torch.autograd.Function):
+    """Gram blocks ``Gk = k̂·k̂ᵀ``, ``Gq = q̂·k̂ᵀ`` (fp32) → the strictly lower ``A = Gk ∘ decay ∘ β`` (fp32) and the lower ``Gq ∘ decay``
+    (bf16), ``decay[i, j] = exp(gc_i − gc_j)``; one pass each way (``csrc/gdn_pieces.cu``)."""
+
+    @staticmethod
+    def forward(ctx, Gk, Gq, gc, beta):
+        out = backend.require_extension().gdn_mask_fwd(Gk, Gq, gc, beta)
+        backend.count_launch()
+        ctx.save_for_backward(Gk, Gq, gc, beta)
+        return out
+
+    @staticmethod
+    def backward(ctx, dA, dqk):
+        Gk, Gq, gc, beta = ctx.saved_tensors
+        dA = torch.zeros_like(Gk) if dA is None else dA.contiguous()
+        dqk = torch.zeros(Gk.shape, dtype=torch.bfloat16, device=Gk.device) if dqk is None else dqk.contiguous()
+        dGk, dGq, dgc, dbeta = backend.require_extension().gdn_mask_bwd(dA, dqk, Gk, Gq, gc, beta)
+        backend.count_launch()
+        return dGk, dGq, dgc, dbeta
+
+
+class _ColsFn(torch.autograd.Function):
+    """``(T ∘ β_j, T ∘ β_j·exp(gc_j))`` in bf16 for the products with values and keys (``csrc/gdn_pieces.cu``)."""
+
+    @staticmethod
+    def forward(ctx, Tm, gc, beta):
+        out = backend.require_extension().gdn_cols_fwd(Tm, gc, beta)
+        backend.count_launch()
+        ctx.save_for_backward(Tm, gc, beta)
+        return out
+
+    @staticmethod
+    def backward(ctx, dTu, dTw):
+        Tm, gc, beta = ctx.saved_tensors
+        z = lambda t: torch.zeros(Tm.shape, dtype=torch.bfloat16, device=Tm.device) if t is None else t.contiguous()
+        dT, dgc, dbeta = backend.require_extension().gdn_cols_bwd(z(dTu), z(dTw), Tm, gc, beta)
+        backend.count_launch()
+        return dT, dgc, dbeta
+
+
 def _prepare_kernel_ok(q, k, v, chunk: int, l2norm: bool) -> bool:
     Dk, Dv = q.shape[-1], v.shape[-1]
     return (q.is_cuda and l2norm and chunk == 64 and q.dtype == torch.bfloat16 and k.dtype == torch.bfloat16 and v.dtype == torch.bfloat16
             and (Dk, Dv) in ((128, 128), (128, 256), (256, 256), (256, 512)) and backend.has("gdn_prepare_fwd")
-            and backend.has("gdn_state") and backend.use_cuda_kernel("gated_delta_rule", q, k, v))
+            and backend.has("gdn_state") and backend.has("gdn_mask_fwd") and backend.use_cuda_kernel("gated_delta_rule", q, k, v))
 
 
 def _chunk_fused_prepare(q, k, v, g, beta, scale: float, eps: float = 1e-6):
-    """The chunked form with the row-wise work on the prepare kernels and bf16 operands for every product; the 64×64
-    pieces (decay matrix, masks, triangular inverse, its column scalings) stay small fp32 PyTorch ops."""
+    """The chunked form with the row-wise work on the prepare kernels, the 64×64 pieces (decay matrix, masks, triangular inverse,
+    its column scalings) on kernels of their own in fp32, and bf16 operands for every product."""
     B, T, H, Dk = q.shape
     Dv = v.shape[-1]
     c = 64
@@ -240,14 +280,10 @@ def _chunk_fused_prepare(q, k, v, g, beta, scale: float, eps: float = 1e-6):
     qn, kn, vc, kd, qg = _PrepareFn.apply(q, k, v, gc.view(B * H, Tp), float(scale), eps)
     r4 = lambda t: t.view(B * H, nC, c, t.shape[-1])
     qn, kn, vc, kd, qg = r4(qn), r4(kn), r4(vc), r4(kd), r4(qg)
-    dec = torch.exp(gc.unsqueeze(-1) - gc.unsqueeze(-2))                 # [i, j] = exp(gc_i − gc_j)
-    strict = torch.tril(torch.ones(c, c, device=q.device, dtype=torch.bool), -1)
-    incl = torch.tril(torch.ones(c, c, device=q.device, dtype=torch.bool), 0)
-    A = (_BmmNTf32.apply(kn, kn) * dec * beta.unsqueeze(-1)).masked_fill(~strict, 0.0)
-    Tm = unit_lower_inverse(A)
-    u = (Tm * beta.unsqueeze(-2)).to(q.dtype) @ vc                       # (I + A)⁻¹ · diag(β) · v
-    w = (Tm * (beta * torch.exp(gc)).unsqueeze(-2)).to(q.dtype) @ kn     # (I + A)⁻¹ · diag(β·exp(gc)) · k̂
-    qk = (_BmmNTf32.apply(qn, kn) * dec).masked_fill(~incl, 0.0)
+    beta = beta.contiguous()
+    A, qk = _MaskFn.apply(_BmmNTf32.apply(kn, kn), _BmmNTf32.apply(qn, kn), gc, beta)
+    Tu, Tw = _ColsFn.apply(unit_lower_inverse(A), gc, beta)
+    u, w = Tu @ vc, Tw @ kn                                              # (I + A)⁻¹ · diag(β) · v,  (I + A)⁻¹ · diag(β·exp(gc)) · k̂
     o = _chunk_core(w, u, kd, qg, qk, torch.exp(gc[..., -1]))            # (B·H, nC, c, Dv)
     return o.reshape(B, H, Tp, Dv).permute(0, 2, 1, 3)[:, :T].to(v.dtype)
 
