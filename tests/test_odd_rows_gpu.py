@@ -56,3 +56,18 @@ def test_layers_agree_with_the_library_route(T):
         assert _rel(y, r) < 2.0 ** -7
         for a, b in zip(got, want):
             assert _rel(a, b) < 2.0 ** -7                       # gradients pass one more bf16 tensor each
+
+
+@pytest.mark.parametrize("T", [1, 67, 1001])
+def test_a_small_bias_is_added_before_the_rounding(T):
+    torch.manual_seed(2)
+    x, w = _mk(T, 256), _mk(512, 256)
+    b = torch.full((512,), 2.0 ** -9, device="cuda", dtype=torch.bfloat16)      # far below an ulp of most of the products (up to 2^-4)
+    y, ref = gemm.linear(x, w, b), x.double() @ w.double().t() + b.double()
+    # half an ulp (at most 2^-8 of the value), and fp32 sums of 256 products of magnitude below 8
+    assert bool(((y.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 256 * 8 * 2.0 ** -24).all())
+    # the bias survives on average; a second rounding drops it where an ulp exceeds 2^-8: the mean of n rounding errors, each
+    # within ulp / 2 <= 2^-8 |ref|, stays within 6 of its standard deviations
+    err = (y.double() - ref)
+    if T > 1:
+        assert abs(float(err.mean())) < 6 * 2.0 ** -8 * float(ref.norm()) / ref.numel()
