@@ -273,10 +273,12 @@ def linear_widened(x: torch.Tensor, weight: torch.Tensor) -> torch.Tensor:
 
 # ------------------------------------------------------------------------------------------ fused sibling projections
 def _adjacent(ts) -> bool:
-    """True when the tensors are dense 2-D row blocks stored back to back (views of one flat parameter buffer)."""
+    """True when the tensors are dense 2-D row blocks stored back to back in one storage (views of one flat parameter buffer).
+    Separate tensors can lie back to back too (the allocator cuts large ones from one segment), but no view spans them."""
     for a, b in zip(ts[:-1], ts[1:]):
         if not (a.is_contiguous() and b.is_contiguous() and a.dtype == b.dtype and a.shape[1] == b.shape[1]
-                and a.data_ptr() + a.numel() * a.element_size() == b.data_ptr()):
+                and a.data_ptr() + a.numel() * a.element_size() == b.data_ptr()
+                and a.untyped_storage().data_ptr() == b.untyped_storage().data_ptr()):
             return False
     return True
 
