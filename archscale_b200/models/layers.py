@@ -43,6 +43,8 @@ class Linear(nn.Linear):
             return gemm.linear_widened(x, w)
         return ops.linear(x, w, b)
 
+    plain_forward = forward     # what ``ops.gemm.plain_linear`` compares with: a replaced ``forward`` is never passed by
+
 
 def apply_mxfp8(model: nn.Module, skip=("lm_head", "lc_proj")) -> int:
     """Switch every :class:`Linear` of ``model`` to the MXFP8 path, except modules whose name contains one of

@@ -21,6 +21,7 @@ from __future__ import annotations
 from typing import Optional
 
 import torch
+from torch.nn.modules.module import _has_any_global_hook
 
 from . import backend
 
@@ -335,19 +336,28 @@ class _MultiLinearFn(torch.autograd.Function):
         return (dx,) + tuple(outs)
 
 
+def plain_linear(l) -> bool:
+    """True when a call of the layer ``l`` is the product with its weight and nothing else, so that a fused route may pass the
+    module by: a ``Linear`` without bias or low-precision operands, hooks, or another ``forward`` than its own."""
+    d = l.__dict__
+    return (type(l).__name__ == "Linear" and type(l).forward is getattr(type(l), "plain_forward", None) and "forward" not in d
+            and l.bias is None and not l.mxfp8 and not l.nvfp4
+            and not (d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"])
+            and l._compiled_call_impl is None and not _has_any_global_hook())
+
+
 def linear_multi(x: torch.Tensor, layers, keep_fused: bool = False):
-    """Outputs of several bias-free ``Linear`` layers that share the input ``x``.  When their weights sit back to back in
-    memory (consecutive views of the flat parameter buffer) the layers run as one GEMM and the outputs are column
+    """Outputs of several ``Linear`` layers that share the input ``x``.  When all are :func:`plain_linear` and their weights sit back to
+    back in memory (consecutive views of the flat parameter buffer) the layers run as one GEMM and the outputs are column
     slices of its result; otherwise each layer is called on its own.  ``keep_fused``: return the one GEMM's result unsplit
     (a tensor instead of a list) when the layers did run as one GEMM."""
+    if not all(plain_linear(l) for l in layers):
+        return [l(x) for l in layers]
     ws = [l.weight for l in layers]
-    if (len(ws) <= 3 and all(type(l).__name__ == "Linear" and l.bias is None and not l.mxfp8 and not getattr(l, "nvfp4", False)
-                             for l in layers) and _skinny_ok(x, ws)):
+    if len(ws) <= 3 and _skinny_ok(x, ws):
         y = _skinny(x, ws, False)                       # the weights need not be neighbours here
         return y if keep_fused else list(y.split([w.shape[0] for w in ws], dim=-1))
-    fusable = (x.is_cuda and x.dtype == torch.bfloat16 and all(type(l).__name__ == "Linear" and l.bias is None and not l.mxfp8
-                                                              and not getattr(l, "nvfp4", False) for l in layers)
-               and all(w.dtype == torch.bfloat16 for w in ws) and _adjacent(ws)
+    fusable = (x.is_cuda and x.dtype == torch.bfloat16 and all(w.dtype == torch.bfloat16 for w in ws) and _adjacent(ws)
                and x.numel() > 0 and x.shape[-1] % 8 == 0 and x.shape[-1] >= 64
                and backend.use_cuda_kernel("gemm", x, ws[0]))
     if not fusable:

@@ -1,0 +1,46 @@
+"""Fused linear routes on the GPU: what they must not lose of the layers they stand for."""
+import pytest
+import torch
+
+from archscale_b200.config import Config
+from archscale_b200.models.gpt import LLaMAMLP
+from archscale_b200.models.layers import Linear
+from archscale_b200.ops import gemm
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("neighbours", [False, True])
+@pytest.mark.parametrize("T", [8, 41, 64, 65, 72])
+def test_hooks_of_the_projections_act_at_every_token_count(T, neighbours):
+    torch.manual_seed(0)
+    layers = [Linear(256, n, bias=False, device="cuda", dtype=torch.bfloat16) for n in (256, 64, 64)]
+    if neighbours:
+        flat = torch.cat([l.weight.detach() for l in layers])
+        for l, w in zip(layers, flat.split([256, 64, 64])):
+            l.weight = torch.nn.Parameter(w)
+    x = torch.randn(1, T, 256, device="cuda").bfloat16()
+    for grad in (False, True):
+        with torch.set_grad_enabled(grad):
+            plain = list(gemm.linear_multi(x, layers))
+            h = layers[0].register_forward_hook(lambda m, a, y: y + 1)
+            layers[2].forward = lambda x: x.new_zeros(*x.shape[:-1], 64)
+            y = gemm.linear_multi(x, layers, keep_fused=True)
+            assert not torch.is_tensor(y)
+            tol = dict(rtol=2.0 ** -7, atol=2.0 ** -7)        # the fused product may sum in another order: one rounding to bf16 each
+            torch.testing.assert_close(y[0], plain[0] + 1, **tol)
+            torch.testing.assert_close(y[1], plain[1], **tol)
+            assert not y[2].any()
+            h.remove()
+            del layers[2].forward
+
+
+@pytest.mark.parametrize("T", [41, 64, 65, 72])
+def test_a_hook_on_the_up_projection_acts_at_every_token_count(T):
+    cfg = Config.from_name("transformer_gqa4_d8", n_embd=256, n_head=2, n_query_groups=1, head_dim=128, intermediate_size=704)
+    mlp = LLaMAMLP(cfg).cuda().bfloat16()
+    mlp.reset_parameters()
+    mlp.w1.register_forward_hook(lambda m, a, y: torch.zeros_like(y))
+    with torch.no_grad():
+        y, _ = mlp(torch.randn(1, T, 256, device="cuda").bfloat16(), 0)
+    assert not y.any()
