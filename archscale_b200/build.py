@@ -23,6 +23,7 @@ BUILD = os.path.join(PKG, "_build")
 OUT = os.path.join(PKG, "_C.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 ARCH = ["-gencode", "arch=compute_100a,code=sm_100a"]
+PRECISE = {"gdn_pieces.cu"}     # built without --use_fast_math: expf at its documented accuracy, subnormal numbers kept
 
 
 def _newer(src: str, dst: str, headers) -> bool:
@@ -57,8 +58,9 @@ def build(force: bool = False, verbose: bool = False) -> str:
         obj = os.path.join(BUILD, os.path.basename(src) + ".o")
         objs.append(obj)
         if force or _newer(src, obj, headers):
-            jobs.append([NVCC, *ARCH, "-O3", "-std=c++17", "-lineinfo", "--use_fast_math", "-Xcompiler", "-fPIC",
-                         "-Xptxas", "-v" if verbose else "-O3", "-I", CSRC, "-c", src, "-o", obj])
+            fast = [] if os.path.basename(src) in PRECISE else ["--use_fast_math"]
+            jobs.append([NVCC, *ARCH, "-O3", "-std=c++17", "-lineinfo", *fast, "-Xcompiler", "-fPIC", "-Xptxas",
+                         "-v" if verbose else "-O3", "-I", CSRC, "-c", src, "-o", obj])
     inc = [f"-I{p}" for p in ce.include_paths(device_type="cuda")] + [f"-I{sysconfig.get_paths()['include']}", f"-I{CSRC}"]
     bobj = os.path.join(BUILD, "bindings.cpp.o")
     bsrc = os.path.join(CSRC, "bindings.cpp")
