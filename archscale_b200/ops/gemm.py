@@ -185,8 +185,7 @@ SKINNY_ROWS = 64
 
 def _skinny_ok(x: torch.Tensor, ws) -> bool:
     """Whether the kernel for few rows (``csrc/gemm_skinny.cu``) takes ``x @ [w₀; w₁; …]ᵀ``: no gradients, at most 64 rows (one
-    block of its tokens: beyond that the library's device time, 4 to 16 µs, is less than half of its), dense bf16 rows that the TMA
-    can read (16-byte base, widths that are multiples of 8)."""
+    block of its tokens), dense bf16 rows that the TMA can read (16-byte base, widths that are multiples of 8)."""
     K = x.shape[-1]
     if not (x.is_cuda and x.dtype == torch.bfloat16 and 0 < x.numel() <= SKINNY_ROWS * K and K % 8 == 0 and x.is_contiguous()
             and x.data_ptr() % 16 == 0 and backend.plain_call() and backend.has("gemm_skinny")):

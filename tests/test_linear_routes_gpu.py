@@ -37,10 +37,10 @@ def test_hooks_of_the_projections_act_at_every_token_count(T, neighbours):
 
 @pytest.mark.parametrize("T", [41, 64, 65, 72])
 def test_a_hook_on_the_up_projection_acts_at_every_token_count(T):
-    cfg = Config.from_name("transformer_gqa4_d8", n_embd=256, n_head=2, n_query_groups=1, head_dim=128, intermediate_size=704)
+    cfg = Config.from_name("transformer_gqa4_d8", intermediate_size=704)
     mlp = LLaMAMLP(cfg).cuda().bfloat16()
     mlp.reset_parameters()
     mlp.w1.register_forward_hook(lambda m, a, y: torch.zeros_like(y))
     with torch.no_grad():
-        y, _ = mlp(torch.randn(1, T, 256, device="cuda").bfloat16(), 0)
+        y, _ = mlp(torch.randn(1, T, cfg.n_embd, device="cuda").bfloat16(), 0)
     assert not y.any()
