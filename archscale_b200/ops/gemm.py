@@ -208,12 +208,17 @@ def _skinny(x: torch.Tensor, ws, swiglu: bool) -> torch.Tensor:
 
 def linear_swiglu(x: torch.Tensor, weight: torch.Tensor) -> Optional[torch.Tensor]:
     """SwiGLU of ``x @ weightᵀ`` (gate = first half of the output features) in one GEMM launch, or ``None`` when the
-    fused kernel does not take this case (the caller then runs ``linear`` + ``swiglu_packed``)."""
+    fused kernel does not take this case (the caller then runs ``linear`` + ``swiglu_packed``).
+
+    Without gradients, fewer than 768 tokens in a number that is no multiple of 8 are such a case (see :func:`linear`).  Whole forward
+    passes in a graph, ms, library and activation / fused: dense 8 layers 67 tokens 0.428 / 0.456, 257 0.484 / 0.505, 777 0.649 / 0.673,
+    1001 0.716 / 0.720; 16 layers 257 1.361 / 1.504, 513 1.753 / 1.755, 1001 2.196 / 2.119; launched one by one 2 % apart."""
     if weight.shape[0] % 16 == 0 and _skinny_ok(x, (weight,)) and fused_swiglu_enabled():
         return _skinny(x, [weight], True)
     if not (x.is_cuda and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and weight.dim() == 2
-            and weight.shape[0] % 16 == 0 and x.shape[-1] % 8 == 0 and x.shape[-1] >= 64
-            and x.numel() > 0 and weight.stride(-1) == 1 and weight.stride(0) % 8 == 0
+            and weight.shape[0] % 16 == 0 and x.shape[-1] % 8 == 0 and x.shape[-1] >= 64 and x.numel() > 0
+            and ((x.numel() // x.shape[-1]) % 8 == 0 or x.numel() >= 768 * x.shape[-1] or not backend.plain_call())
+            and weight.stride(-1) == 1 and weight.stride(0) % 8 == 0
             and weight.data_ptr() % 16 == 0 and fused_swiglu_enabled() and backend.use_cuda_kernel("gemm", x, weight)):
         return None
     g = getattr(weight, "_fsdp_group", None)
@@ -227,15 +232,20 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor) -> Optional[torch.Tenso
 def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
     """``x @ weightᵀ + bias``; bf16 CUDA inputs run the tcgen05 kernel for fwd, dgrad and wgrad.
 
-    With a bias, token counts that are no multiple of 8 stay with the library, which adds it before the one rounding to bf16.
+    Without gradients, token counts beyond 64 that are no multiple of 8 stay with the library: the own GEMM's gain at such counts lies in
+    the backward pass.  µs of one product in a graph, library / own: 1024x1024 at 65 tokens 5.0 / 9.8, 1001 5.2 / 11.0, 4001 9.1 / 11.8,
+    16383 26.0 / 28.5; 5632x1024 at 257 6.8 / 11.2, 1001 12.6 / 16.2, 4001 37.1 / 34.9, 8191 69.5 / 68.8; 2048x2048 at 1001 9.3 / 15.7, 16383
+    91.7 / 96.0; host 11 / 15.
+
+    With a bias they stay there with gradients too: the library adds it before the one rounding to bf16.
     ``_LinearFn`` adds it to the rounded product, where a bias below half a unit in the last place is lost: with biases of
     some 1e-4 the second training step's loss moved by 4e-4 to 8e-4 of its value at 1001 to 9001 tokens (now by 2e-4 at most).
     Eight-layer hybrid steps, library everywhere / only here, ms: 1001 tokens 77.0 / 72.3, 4001 100.0 / 98.5, 9001 152.0 / 143.4."""
     if bias is None and _skinny_ok(x, (weight,)):
         return _skinny(x, [weight], False)
     if (x.is_cuda and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16
-            and x.shape[-1] % 8 == 0 and weight.shape[0] % 8 == 0 and x.shape[-1] >= 64
-            and x.numel() > 0 and (bias is None or (x.numel() // x.shape[-1]) % 8 == 0)
+            and x.shape[-1] % 8 == 0 and weight.shape[0] % 8 == 0 and x.shape[-1] >= 64 and x.numel() > 0
+            and ((x.numel() // x.shape[-1]) % 8 == 0 or (bias is None and not backend.plain_call()))
             and backend.use_cuda_kernel("gemm", x, weight)):
         if not x.is_contiguous():
             x = x.contiguous()
@@ -338,9 +348,9 @@ class _MultiLinearFn(torch.autograd.Function):
 def plain_linear(l) -> bool:
     """True when a call of the layer ``l`` is the product with its weight and nothing else, so that a fused route may pass the
     module by: a ``Linear`` without bias or low-precision operands, hooks, or another ``forward`` than its own."""
-    d = l.__dict__
-    return (type(l).__name__ == "Linear" and type(l).forward is getattr(type(l), "plain_forward", None) and "forward" not in d
-            and l.bias is None and not l.mxfp8 and not l.nvfp4
+    cls, d = type(l), l.__dict__
+    return (cls.__name__ == "Linear" and cls.forward is getattr(cls, "plain_forward", None) and "forward" not in d
+            and d["_parameters"].get("bias") is None and not l.mxfp8 and not l.nvfp4
             and not (d["_forward_hooks"] or d["_forward_pre_hooks"] or d["_backward_hooks"] or d["_backward_pre_hooks"])
             and l._compiled_call_impl is None and not _has_any_global_hook())
 

@@ -1,11 +1,12 @@
 """Fused linear routes on the GPU: what they must not lose of the layers they stand for."""
 import pytest
 import torch
+import torch.nn.functional as F
 
 from archscale_b200.config import Config
 from archscale_b200.models.gpt import LLaMAMLP
 from archscale_b200.models.layers import Linear
-from archscale_b200.ops import gemm
+from archscale_b200.ops import backend, gemm
 
 pytestmark = pytest.mark.gpu
 
@@ -44,3 +45,21 @@ def test_a_hook_on_the_up_projection_acts_at_every_token_count(T):
     with torch.no_grad():
         y, _ = mlp(torch.randn(1, T, cfg.n_embd, device="cuda").bfloat16(), 0)
     assert not y.any()
+
+
+@pytest.mark.parametrize("T", [65, 257, 1001, 4099])
+def test_odd_token_counts_without_gradients_run_the_library(T):
+    torch.manual_seed(0)
+    x, w = torch.randn(T, 256, device="cuda").bfloat16(), (torch.randn(264, 256, device="cuda") / 16).bfloat16()
+    n0 = backend.launches()
+    with torch.no_grad():
+        y = gemm.linear(x, w)
+    assert backend.launches() == n0 and torch.equal(y, F.linear(x, w))
+    gemm.linear(x, w.requires_grad_())                       # with gradients: the own GEMM, whose backward pays
+    assert backend.launches() == n0 + 1
+    with torch.no_grad():
+        gemm.linear(x[:T // 8 * 8], w)
+        assert backend.launches() == n0 + 2
+        w2 = w[:256]
+        assert (gemm.linear_swiglu(x, w2) is None) == (T < 768)
+        assert gemm.linear_swiglu(x[:T // 8 * 8], w2) is not None
