@@ -210,14 +210,14 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor) -> Optional[torch.Tenso
     """SwiGLU of ``x @ weightᵀ`` (gate = first half of the output features) in one GEMM launch, or ``None`` when the
     fused kernel does not take this case (the caller then runs ``linear`` + ``swiglu_packed``).
 
-    Without gradients, fewer than 768 tokens in a number that is no multiple of 8 are such a case (see :func:`linear`).  Whole forward
-    passes in a graph, ms, library and activation / fused: dense 8 layers 67 tokens 0.428 / 0.456, 257 0.484 / 0.505, 777 0.649 / 0.673,
-    1001 0.716 / 0.720; 16 layers 257 1.361 / 1.504, 513 1.753 / 1.755, 1001 2.196 / 2.119; launched one by one 2 % apart."""
+    Token counts that are no multiple of 8 take it without gradients too (unlike single products, see :func:`linear`): one launch
+    instead of two.  Whole forward passes, launched one by one, ms, library and activation / fused: dense 8 layers 67 tokens 2.20 / 2.05,
+    257 2.20 / 2.05.  In a graph, where only device time counts, the fused kernel's 256-row tiles lose below some 800 tokens: 67 0.428 /
+    0.456, 257 0.484 / 0.505, 777 0.649 / 0.673, 1001 0.716 / 0.720; 16 layers 257 1.361 / 1.504, 513 1.753 / 1.755, 1001 2.196 / 2.119."""
     if weight.shape[0] % 16 == 0 and _skinny_ok(x, (weight,)) and fused_swiglu_enabled():
         return _skinny(x, [weight], True)
     if not (x.is_cuda and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and weight.dim() == 2
             and weight.shape[0] % 16 == 0 and x.shape[-1] % 8 == 0 and x.shape[-1] >= 64 and x.numel() > 0
-            and ((x.numel() // x.shape[-1]) % 8 == 0 or x.numel() >= 768 * x.shape[-1] or not backend.plain_call())
             and weight.stride(-1) == 1 and weight.stride(0) % 8 == 0
             and weight.data_ptr() % 16 == 0 and fused_swiglu_enabled() and backend.use_cuda_kernel("gemm", x, weight)):
         return None

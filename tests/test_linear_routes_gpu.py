@@ -60,6 +60,3 @@ def test_odd_token_counts_without_gradients_run_the_library(T):
     with torch.no_grad():
         gemm.linear(x[:T // 8 * 8], w)
         assert backend.launches() == n0 + 2
-        w2 = w[:256]
-        assert (gemm.linear_swiglu(x, w2) is None) == (T < 768)
-        assert gemm.linear_swiglu(x[:T // 8 * 8], w2) is not None
