@@ -9,9 +9,9 @@
 extern "C" {
 #endif
 
-// D = alpha·op(A)·op(B) (+beta·C).  mode 0: A[M,K]·B[N,K]ᵀ, 1: A[M,K]·B[K,N], 2: A[K,M]ᵀ·B[K,N].
+// D = alpha·op(A)·op(B) (+beta·C, rows of C ldci elements apart; 0: one row, a bias, for all).  mode 0: A[M,K]·B[N,K]ᵀ, 1: A[M,K]·B[K,N], 2: A[K,M]ᵀ·B[K,N].
 int b200_gemm_bf16(int mode, const void* A, const void* B, void* out, const void* cin, int M, int N, int K, int lda,
-                   int ldb, int ldc, float alpha, float beta, int out_f32, int accumulate, int num_sms, int* status,
+                   int ldb, int ldc, int ldci, float alpha, float beta, int out_f32, int accumulate, int num_sms, int* status,
                    cudaStream_t stream);
 
 int b200_gemm_bf16_batched(int mode, const void* A, const void* B, void* out, const void* cin, int batch, int M, int N,
@@ -121,7 +121,7 @@ int b200_attn_bwd(const void* d_out, const void* q, const void* k, const void* v
 
 // ---- peer-memory collectives (comm.cu).  `bases[p]` = local mapping of rank p's symmetric heap.
 // Forward GEMM with the FSDP all-gather of the whole flat parameter group fused in (gemm_bf16.cu).
-int b200_ag_gemm_bf16(const void* A, void* out, int M, int N, int K, int lda, int ldc, const void* const* bases,
+int b200_ag_gemm_bf16(const void* A, void* out, const void* bias, int M, int N, int K, int lda, int ldc, const void* const* bases,
                       size_t src_off, void* dst, size_t shard_bytes, size_t b_off, uint32_t* flags, uint32_t epoch,
                       int rank, int world, int n_copy, int num_sms, int* status, cudaStream_t stream);
 void b200_set_peer_wait_limit_cycles(long long cycles);
@@ -227,7 +227,7 @@ int b200_diff_combine_bwd(const void* dy, const void* a1, const void* a2, const 
 
 // 2-CTA (cta_group::2) variant of b200_gemm_bf16: one 256×256 tile per pair of SMs (gemm2_bf16.cu)
 int b200_gemm2_bf16(int mode, const void* A, const void* B, void* out, const void* cin, int M, int N, int K,
-                    int lda, int ldb, int ldc, float alpha, float beta, int out_f32, int accumulate,
+                    int lda, int ldb, int ldc, int ldci, float alpha, float beta, int out_f32, int accumulate,
                     int num_sms, int* status, cudaStream_t stream);
 
 int b200_grouped_gemm2_bf16(int kind, const void* A, const void* B, void* out, const int* offsets, int E,

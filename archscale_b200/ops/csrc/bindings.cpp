@@ -73,12 +73,12 @@ at::Tensor gemm_bf16(const at::Tensor& a, const at::Tensor& b, int64_t mode, at:
   if (accumulate && !no_splitk) ensure_splitk_workspace(a.device());
   if (gemm_use_pair()) {
     check(b200_gemm2_bf16((int)mode, a.data_ptr(), b.data_ptr(), out.data_ptr(), nullptr, (int)M, (int)N, (int)K,
-                          (int)a.stride(0), (int)b.stride(0), (int)out.stride(0), 1.f, 0.f, out_f32, accumulate, num_sms(),
+                          (int)a.stride(0), (int)b.stride(0), (int)out.stride(0), 0, 1.f, 0.f, out_f32, accumulate, num_sms(),
                           status_ptr(a.device()), cur_stream()), "gemm2_bf16");
     return out;
   }
   check(b200_gemm_bf16((int)mode, a.data_ptr(), b.data_ptr(), out.data_ptr(), nullptr, (int)M, (int)N, (int)K,
-                       (int)a.stride(0), (int)b.stride(0), (int)out.stride(0), 1.f, 0.f, out_f32, accumulate, num_sms(),
+                       (int)a.stride(0), (int)b.stride(0), (int)out.stride(0), 0, 1.f, 0.f, out_f32, accumulate, num_sms(),
                        status_ptr(a.device()), cur_stream()), "gemm_bf16");
   return out;
 }
@@ -95,8 +95,23 @@ at::Tensor gemm_bf16_epi(const at::Tensor& a, const at::Tensor& b, int64_t mode,
   at::Tensor out = at::empty({M, N}, a.options());
   if (c.has_value()) TORCH_CHECK(c->is_contiguous() && c->scalar_type() == at::kBFloat16 && c->size(0) == M && c->size(1) == N);
   check((gemm_use_pair() ? b200_gemm2_bf16 : b200_gemm_bf16)((int)mode, a.data_ptr(), b.data_ptr(), out.data_ptr(), ptr_opt(c), (int)M, (int)N,
-                       (int)K, (int)a.stride(0), (int)b.stride(0), (int)N, (float)alpha, (float)beta, 0, 0, num_sms(),
+                       (int)K, (int)a.stride(0), (int)b.stride(0), (int)N, (int)N, (float)alpha, (float)beta, 0, 0, num_sms(),
                        status_ptr(a.device()), cur_stream()), "gemm_bf16_epi");
+  return out;
+}
+
+// out(bf16) = a[M,K]·b[N,K]ᵀ + bias[N], the bias added to the fp32 sums before the one rounding
+at::Tensor gemm_bf16_bias(const at::Tensor& a, const at::Tensor& b, const at::Tensor& bias) {
+  TORCH_CHECK(a.is_cuda() && b.is_cuda() && a.scalar_type() == at::kBFloat16 && b.scalar_type() == at::kBFloat16);
+  TORCH_CHECK(a.dim() == 2 && b.dim() == 2 && a.stride(1) == 1 && b.stride(1) == 1 && b.size(1) == a.size(1));
+  const int64_t M = a.size(0), K = a.size(1), N = b.size(0);
+  TORCH_CHECK(bias.is_cuda() && bias.scalar_type() == at::kBFloat16 && bias.dim() == 1 && bias.size(0) == N && bias.is_contiguous() &&
+              N % 8 == 0 && reinterpret_cast<uintptr_t>(bias.data_ptr()) % 16 == 0, "gemm_bf16_bias: bias");
+  c10::cuda::CUDAGuard guard(a.device());
+  at::Tensor out = at::empty({M, N}, a.options());
+  check((gemm_use_pair() ? b200_gemm2_bf16 : b200_gemm_bf16)(0, a.data_ptr(), b.data_ptr(), out.data_ptr(), bias.data_ptr(), (int)M, (int)N,
+                       (int)K, (int)a.stride(0), (int)b.stride(0), (int)N, 0, 1.f, 1.f, 0, 0, num_sms(), status_ptr(a.device()),
+                       cur_stream()), "gemm_bf16_bias");
   return out;
 }
 
@@ -228,6 +243,7 @@ std::tuple<at::Tensor, at::Tensor, at::Tensor, at::Tensor> qknorm_rope_bwd(
 PYBIND11_MODULE(TORCH_EXTENSION_NAME, m) {
   m.def("gemm_bf16", &gemm_bf16, "bf16 tcgen05 GEMM", py::arg("a"), py::arg("b"), py::arg("mode"), py::arg("out_dtype"),
         py::arg("acc") = py::none());
+  m.def("gemm_bf16_bias", &gemm_bf16_bias);
   m.def("gemm_bf16_epi", &gemm_bf16_epi);
   m.def("set_gemm_pair", &set_gemm_pair);
   m.def("gemm_pair", &gemm_use_pair);

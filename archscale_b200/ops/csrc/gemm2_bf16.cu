@@ -51,6 +51,7 @@ struct Gemm2Params {
   const void* cin;
   int M, N, K;
   int ldc;
+  int ldci;                // row stride of cin: ldc, or 0 for one row that is added to all (a bias)
   float alpha, beta;
   int accumulate;
   int* status;
@@ -359,7 +360,7 @@ gemm2_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_const
             store_row32(o, r, alpha, acc_flag, p.N - col, wide);
           } else {
             __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + tl.out_off + static_cast<size_t>(row) * p.ldc + col;
-            const __nv_bfloat16* ci = p.cin ? reinterpret_cast<const __nv_bfloat16*>(p.cin) + tl.out_off + static_cast<size_t>(row) * p.ldc + col : nullptr;
+            const __nv_bfloat16* ci = p.cin ? reinterpret_cast<const __nv_bfloat16*>(p.cin) + tl.out_off + static_cast<size_t>(row) * p.ldci + col : nullptr;
             if (wide && col + 32 <= p.N) {
               uint32_t cw[2][8];
               if (ci) { load_32b(ci, cw[0]); load_32b(ci + 16, cw[1]); }
@@ -477,9 +478,10 @@ static int launch2_grouped(const CUtensorMap& ta, const CUtensorMap& tb, const G
 
 }  // namespace b200
 
-// Same contract as b200_gemm_bf16 (modes 0 NT, 1 NN, 2 TN; bf16 or fp32 output, optional α·AB + β·C or accumulate).
+// Same contract as b200_gemm_bf16 (modes 0 NT, 1 NN, 2 TN; bf16 or fp32 output, optional α·AB + β·C or accumulate; C with rows ldci
+// apart, 0 for a bias).
 extern "C" int b200_gemm2_bf16(int mode, const void* A, const void* B, void* out, const void* cin, int M, int N, int K,
-                               int lda, int ldb, int ldc, float alpha, float beta, int out_f32, int accumulate,
+                               int lda, int ldb, int ldc, int ldci, float alpha, float beta, int out_f32, int accumulate,
                                int num_sms, int* status, cudaStream_t stream) {
   using namespace b200;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
@@ -497,7 +499,7 @@ extern "C" int b200_gemm2_bf16(int mode, const void* A, const void* B, void* out
   if (mode == 0) rc = make_tmap_2d_bf16(&tb, B, K, N, ldb, T2_BK, T2_HALF);   // stored [N, K]
   else           rc = make_tmap_2d_bf16(&tb, B, N, K, ldb, 64, T2_BK);        // stored [K, N]
   if (rc) return rc;
-  Gemm2Params p{out, cin, M, N, K, ldc, alpha, beta, accumulate, status, 1, nullptr};
+  Gemm2Params p{out, cin, M, N, K, ldc, ldci, alpha, beta, accumulate, status, 1, nullptr};
   if (mode == 0) return out_f32 ? launch2<0, 0, 1>(ta, tb, p, num_sms, stream) : launch2<0, 0, 0>(ta, tb, p, num_sms, stream);
   if (mode == 1) return out_f32 ? launch2<0, 1, 1>(ta, tb, p, num_sms, stream) : launch2<0, 1, 0>(ta, tb, p, num_sms, stream);
   if (mode == 2) return out_f32 ? launch2<1, 1, 1>(ta, tb, p, num_sms, stream) : launch2<1, 1, 0>(ta, tb, p, num_sms, stream);
@@ -522,7 +524,7 @@ extern "C" int b200_gemm2_swiglu_bf16(const void* A, const void* B, void* h, voi
   if (rc) return rc;
   rc = make_tmap_2d_bf16(&tb, B, K, 2 * static_cast<uint64_t>(I), ldb, T2_BK, T2_HALF);
   if (rc) return rc;
-  Gemm2Params p{h, nullptr, M, 2 * I, K, 2 * I, 1.f, 0.f, 0, status, 1, nullptr, I, act, I};
+  Gemm2Params p{h, nullptr, M, 2 * I, K, 2 * I, 0, 1.f, 0.f, 0, status, 1, nullptr, I, act, I};
   auto kern = gemm2_bf16_kernel<0, 0, 0>;
   static bool configured = false;
   if (!configured) {
@@ -553,7 +555,7 @@ extern "C" int b200_grouped_gemm2_swiglu_bf16(const void* A, const void* B, void
   rc = make_tmap_2d_bf16(&tb, B, K, static_cast<uint64_t>(E) * 2 * I, K, T2_BK, T2_HALF);
   if (rc) return rc;
   Group2Params gp{offsets, E, 2 * I, nullptr, nullptr, 0};
-  Gemm2Params p{h, nullptr, capacity, 2 * I, K, 2 * I, 1.f, 0.f, 0, status, 1, nullptr, I, act, I};
+  Gemm2Params p{h, nullptr, capacity, 2 * I, K, 2 * I, 0, 1.f, 0.f, 0, status, 1, nullptr, I, act, I};
   const int max_tiles = (capacity / T2_BM) * ((I + T2_HALF - 1) / T2_HALF);
   return launch2_grouped<0, 0, 0, 1>(ta, tb, p, gp, max_tiles, num_sms, stream);
 }
@@ -581,7 +583,7 @@ extern "C" int b200_grouped_gemm2_bf16(int kind, const void* A, const void* B, v
     if (kind == 0) { rc = make_tmap_2d_bf16(&tb, B, K, static_cast<uint64_t>(E) * N, K, T2_BK, T2_HALF); gp.b_rows = N; }
     else           { rc = make_tmap_2d_bf16(&tb, B, N, static_cast<uint64_t>(E) * K, N, 64, T2_BK); gp.b_rows = K; }
     if (rc) return rc;
-    Gemm2Params p{out, nullptr, capacity, N, K, N, 1.f, 0.f, 0, status, 1, nullptr};
+    Gemm2Params p{out, nullptr, capacity, N, K, N, 0, 1.f, 0.f, 0, status, 1, nullptr};
     const int max_tiles = (capacity / T2_BM) * (N / T2_BN);
     return kind == 0 ? launch2_grouped<0, 0, 0, 1>(ta, tb, p, gp, max_tiles, num_sms, stream)
                      : launch2_grouped<0, 1, 0, 1>(ta, tb, p, gp, max_tiles, num_sms, stream);
@@ -591,7 +593,7 @@ extern "C" int b200_grouped_gemm2_bf16(int kind, const void* A, const void* B, v
     if (rc) return rc;
     rc = make_tmap_2d_bf16(&tb, B, N, capacity, N, 64, T2_BK);
     if (rc) return rc;
-    Gemm2Params p{out, nullptr, M, N, capacity, N, 1.f, 0.f, accumulate, status, 1, nullptr};
+    Gemm2Params p{out, nullptr, M, N, capacity, N, 0, 1.f, 0.f, accumulate, status, 1, nullptr};
     const int tiles = E * ((M + T2_BM - 1) / T2_BM) * ((N + T2_BN - 1) / T2_BN);
     return out_f32 ? launch2_grouped<1, 1, 1, 2>(ta, tb, p, gp, tiles, num_sms, stream)
                    : launch2_grouped<1, 1, 0, 2>(ta, tb, p, gp, tiles, num_sms, stream);
@@ -622,7 +624,7 @@ extern "C" int b200_gemm2_bf16_batched(int mode, const void* A, const void* B, v
   if (mode == 0) rc = make_tmap_3d_bf16(&tb, B, K, N, batch, K, static_cast<uint64_t>(N) * K, T2_BK, T2_HALF);
   else           rc = make_tmap_3d_bf16(&tb, B, N, K, batch, N, static_cast<uint64_t>(K) * N, 64, T2_BK);
   if (rc) return rc;
-  Gemm2Params p{out, cin, M, N, K, N, alpha, beta, 0, status, 1, nullptr};
+  Gemm2Params p{out, cin, M, N, K, N, N, alpha, beta, 0, status, 1, nullptr};
   if (symmetric && M != N) return -1;
   Group2Params gp{nullptr, batch, 0, alpha_vec, beta_vec, symmetric};
   const int nm = (M + T2_BM - 1) / T2_BM;

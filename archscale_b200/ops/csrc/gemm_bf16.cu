@@ -77,7 +77,8 @@ struct GemmParams {
   void* out;
   const void* cin;
   int M, N, K;
-  int ldc;          // row stride of out / cin in elements
+  int ldc;          // row stride of out in elements
+  int ldci;         // row stride of cin: ldc, or 0 for one row that is added to all (a bias)
   float alpha, beta;
   int accumulate;   // fp32 output: out += result
   int* status;
@@ -467,7 +468,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tmap_a, const __grid_consta
             __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(p.out) + tl.out_off + static_cast<size_t>(row) * p.ldc + col;
             if (FUSED_AG == 2 && own_tile)
               o = rs.out_local + static_cast<size_t>(row - rs.rank * (num_m / rs.world) * BM) * p.N + col;
-            const __nv_bfloat16* ci = p.cin ? reinterpret_cast<const __nv_bfloat16*>(p.cin) + tl.out_off + static_cast<size_t>(row) * p.ldc + col : nullptr;
+            const __nv_bfloat16* ci = p.cin ? reinterpret_cast<const __nv_bfloat16*>(p.cin) + tl.out_off + static_cast<size_t>(row) * p.ldci + col : nullptr;
 #pragma unroll
             for (int j = 0; j < 32; j += 8) {
               if (col + j < p.N) {
@@ -650,7 +651,7 @@ extern "C" void b200_gemm_set_splitk_workspace(uint32_t* sem, int n) {
 }
 
 extern "C" int b200_gemm_bf16(int mode, const void* A, const void* B, void* out, const void* cin, int M, int N, int K,
-                              int lda, int ldb, int ldc, float alpha, float beta, int out_f32, int accumulate,
+                              int lda, int ldb, int ldc, int ldci, float alpha, float beta, int out_f32, int accumulate,
                               int num_sms, int* status, cudaStream_t stream) {
   using namespace b200;
   if (M <= 0 || N <= 0 || K <= 0) return 0;
@@ -672,17 +673,17 @@ extern "C" int b200_gemm_bf16(int mode, const void* A, const void* B, void* out,
   if (mode == 0) rc = make_tmap_2d_bf16(&tb, B, K, N, ldb, BK, BN);      // stored [N, K]
   else           rc = make_tmap_2d_bf16(&tb, B, N, K, ldb, 64, BK);      // stored [K, N]
   if (rc) return rc;
-  GemmParams p{out, cin, M, N, K, ldc, alpha, beta, accumulate, status};
+  GemmParams p{out, cin, M, N, K, ldc, ldci, alpha, beta, accumulate, status};
   if (mode == 0) return out_f32 ? launch_variant<0, 0, 1>(ta, tb, p, num_sms, stream) : launch_variant<0, 0, 0>(ta, tb, p, num_sms, stream);
   if (mode == 1) return out_f32 ? launch_variant<0, 1, 1>(ta, tb, p, num_sms, stream) : launch_variant<0, 1, 0>(ta, tb, p, num_sms, stream);
   if (mode == 2) return out_f32 ? launch_variant<1, 1, 1>(ta, tb, p, num_sms, stream) : launch_variant<1, 1, 0>(ta, tb, p, num_sms, stream);
   return -4;
 }
 
-// out[M,N] (bf16) = A[M,K] · Bᵀ where B[N,K] sits at byte offset b_off of the gathered buffer `dst` that this
+// out[M,N] (bf16) = A[M,K] · Bᵀ (+ bias[N], null or 16-byte aligned) where B[N,K] sits at byte offset b_off of the gathered buffer `dst` that this
 // same launch fills from all ranks' shards (see AgParams).  `flags` needs one uint32 per 256 KiB of dst
 // and must never hold `epoch` from an earlier launch (use a fresh epoch per call).
-extern "C" int b200_ag_gemm_bf16(const void* A, void* out, int M, int N, int K, int lda, int ldc,
+extern "C" int b200_ag_gemm_bf16(const void* A, void* out, const void* bias, int M, int N, int K, int lda, int ldc,
                                  const void* const* bases, size_t src_off, void* dst, size_t shard_bytes, size_t b_off,
                                  uint32_t* flags, uint32_t epoch, int rank, int world, int n_copy, int num_sms,
                                  int* status, cudaStream_t stream) {
@@ -699,7 +700,7 @@ extern "C" int b200_ag_gemm_bf16(const void* A, void* out, int M, int N, int K, 
   if (rc) return rc;
   rc = make_tmap_2d_bf16(&tb, static_cast<const char*>(dst) + b_off, K, N, K, BK, BN);
   if (rc) return rc;
-  GemmParams p{out, nullptr, M, N, K, ldc, 1.f, 0.f, 0, status};
+  GemmParams p{out, bias, M, N, K, ldc, 0, 1.f, 1.f, 0, status};
   AgParams ag{};
   for (int i = 0; i < 8; ++i) ag.peer[i] = i < world ? bases[i] : nullptr;
   ag.src_off = src_off; ag.dst = static_cast<char*>(dst); ag.shard_bytes = shard_bytes; ag.b_off = b_off;
@@ -738,7 +739,7 @@ extern "C" int b200_ag_a_gemm_bf16(const void* const* bases, size_t src_off, voi
   if (rc) return rc;
   rc = make_tmap_2d_bf16(&tb, B, K, N, ldb, BK, BN);
   if (rc) return rc;
-  GemmParams p{out, nullptr, M, N, K, ldc, 1.f, 0.f, 0, status};
+  GemmParams p{out, nullptr, M, N, K, ldc, 0, 1.f, 0.f, 0, status};
   AgParams ag{};
   for (int i = 0; i < 8; ++i) ag.peer[i] = i < world ? bases[i] : nullptr;
   ag.src_off = src_off; ag.dst = static_cast<char*>(dst); ag.shard_bytes = shard_bytes; ag.b_off = 0;
@@ -780,7 +781,7 @@ extern "C" int b200_gemm_rs_bf16(const void* A, const void* B, int M, int N, int
   rc = make_tmap_2d_bf16(&tb, B, K, N, ldb, BK, BN);
   if (rc) return rc;
   void* part = const_cast<char*>(static_cast<const char*>(bases[rank])) + part_off;
-  GemmParams p{part, nullptr, M, N, K, N, 1.f, 0.f, 0, status};
+  GemmParams p{part, nullptr, M, N, K, N, 0, 1.f, 0.f, 0, status};
   RsParams rs{};
   for (int i = 0; i < 8; ++i) rs.peer[i] = i < world ? bases[i] : nullptr;
   rs.part_off = part_off; rs.cnt_off = cnt_off; rs.expect = expect; rs.rank = rank; rs.world = world;
@@ -826,7 +827,7 @@ extern "C" int b200_grouped_gemm_bf16(int kind, const void* A, const void* B, vo
     if (kind == 0) { rc = make_tmap_2d_bf16(&tb, B, K, static_cast<uint64_t>(E) * N, K, BK, BN); gp.b_rows = N; }
     else           { rc = make_tmap_2d_bf16(&tb, B, N, static_cast<uint64_t>(E) * K, N, 64, BK); gp.b_rows = K; }
     if (rc) return rc;
-    GemmParams p{out, nullptr, capacity, N, K, N, 1.f, 0.f, 0, status};
+    GemmParams p{out, nullptr, capacity, N, K, N, 0, 1.f, 0.f, 0, status};
     const int max_tiles = (capacity / BM) * ((N + BN - 1) / BN);
     const int grid = max_tiles < num_sms ? (max_tiles > 0 ? max_tiles : 1) : num_sms;
     if (kind == 0) {
@@ -846,7 +847,7 @@ extern "C" int b200_grouped_gemm_bf16(int kind, const void* A, const void* B, vo
     if (rc) return rc;
     rc = make_tmap_2d_bf16(&tb, B, N, capacity, N, 64, BK);
     if (rc) return rc;
-    GemmParams p{out, nullptr, M, N, capacity, N, 1.f, 0.f, accumulate, status};
+    GemmParams p{out, nullptr, M, N, capacity, N, 0, 1.f, 0.f, accumulate, status};
     const int tiles = E * ((M + BM - 1) / BM) * ((N + BN - 1) / BN);
     const int grid = tiles < num_sms ? tiles : num_sms;
     if (out_f32) {
@@ -885,7 +886,7 @@ extern "C" int b200_gemm_bf16_batched(int mode, const void* A, const void* B, vo
   if (mode == 0) rc = make_tmap_3d_bf16(&tb, B, K, N, batch, K, static_cast<uint64_t>(N) * K, BK, BN);
   else           rc = make_tmap_3d_bf16(&tb, B, N, K, batch, N, static_cast<uint64_t>(K) * N, 64, BK);
   if (rc) return rc;
-  GemmParams p{out, cin, M, N, K, N, alpha, beta, 0, status};
+  GemmParams p{out, cin, M, N, K, N, N, alpha, beta, 0, status};
   AgParams none{};
   GroupParams gp{nullptr, batch, 0};
   const int tiles = batch * ((M + BM - 1) / BM) * ((N + BN - 1) / BN);

@@ -47,10 +47,21 @@ def _cuda_ok_tn(a: torch.Tensor, b: torch.Tensor, M: int, N: int, K: int) -> boo
     return M % 8 == 0 and N % 8 == 0 and K >= 64 and M >= 1 and _operands_ok(a, b)
 
 
-def matmul_nt(a: torch.Tensor, b: torch.Tensor, out_dtype: Optional[torch.dtype] = None) -> torch.Tensor:
-    """a:(M,K) b:(N,K) → a @ bᵀ : (M,N)."""
+def bias_row(bias: torch.Tensor) -> torch.Tensor:
+    """``bias`` as the GEMM epilogue reads it: dense bf16 on a 16-byte boundary."""
+    bias = bias.to(torch.bfloat16).contiguous()
+    return bias if bias.data_ptr() % 16 == 0 else bias.clone()
+
+
+def matmul_nt(a: torch.Tensor, b: torch.Tensor, out_dtype: Optional[torch.dtype] = None, bias: Optional[torch.Tensor] = None) -> torch.Tensor:
+    """a:(M,K) b:(N,K) → a @ bᵀ : (M,N); ``bias`` (N,) (bf16 result) is added to the sums before they are rounded."""
     M, K = a.shape
     N = b.shape[0]
+    if bias is not None:
+        if _cuda_ok(a, b, M, N, K) and backend.use_cuda_kernel("gemm", a, b, bias):
+            backend.count_launch()
+            return backend.require_extension().gemm_bf16_bias(a, b, bias_row(bias))
+        return torch.nn.functional.linear(a, b, bias.to(a.dtype))
     if _cuda_ok(a, b, M, N, K) and backend.use_cuda_kernel("gemm", a, b):
         backend.count_launch()
         return backend.require_extension().gemm_bf16(a, b, 0, out_dtype or torch.bfloat16, None)
@@ -108,14 +119,12 @@ class _LinearFn(torch.autograd.Function):
             if weight._fsdp_first and x2.shape[0] % 8 == 0 and _cuda_ok(x2, weight, x2.shape[0], weight.shape[0], x2.shape[1]):
                 # FSDP forward: this GEMM also gathers the unit's matrix parameters from all ranks
                 g.ag_pending = False
-                y = eng.symm.ag_gemm(x2, g, weight.shape[0])
+                y = eng.symm.ag_gemm(x2, g, weight.shape[0], bias=None if bias is None else bias_row(bias))
             else:
                 eng.finish_pending_gather(g)
-                y = matmul_nt(x2, weight)
+                y = matmul_nt(x2, weight, bias=bias)
         else:
-            y = matmul_nt(x2, weight)
-        if bias is not None:
-            y = y + bias.to(y.dtype)
+            y = matmul_nt(x2, weight, bias=bias)
         return y.view(*x.shape[:-1], weight.shape[0])
 
     @staticmethod
@@ -237,15 +246,13 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     16383 26.0 / 28.5; 5632x1024 at 257 6.8 / 11.2, 1001 12.6 / 16.2, 4001 37.1 / 34.9, 8191 69.5 / 68.8; 2048x2048 at 1001 9.3 / 15.7, 16383
     91.7 / 96.0; host 11 / 15.
 
-    With a bias they stay there with gradients too: the library adds it before the one rounding to bf16.
-    ``_LinearFn`` adds it to the rounded product, where a bias below half a unit in the last place is lost: with biases of
-    some 1e-4 the second training step's loss moved by 4e-4 to 8e-4 of its value at 1001 to 9001 tokens (now by 2e-4 at most).
-    Eight-layer hybrid steps, library everywhere / only here, ms: 1001 tokens 77.0 / 72.3, 4001 100.0 / 98.5, 9001 152.0 / 143.4."""
+    A bias is added to the fp32 sums, before the one rounding to bf16, on either route: added to a rounded product, a bias below half a
+    unit in the last place is lost."""
     if bias is None and _skinny_ok(x, (weight,)):
         return _skinny(x, [weight], False)
     if (x.is_cuda and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16
             and x.shape[-1] % 8 == 0 and weight.shape[0] % 8 == 0 and x.shape[-1] >= 64 and x.numel() > 0
-            and ((x.numel() // x.shape[-1]) % 8 == 0 or (bias is None and not backend.plain_call()))
+            and ((x.numel() // x.shape[-1]) % 8 == 0 or not backend.plain_call())
             and backend.use_cuda_kernel("gemm", x, weight)):
         if not x.is_contiguous():
             x = x.contiguous()

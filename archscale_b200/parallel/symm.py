@@ -143,8 +143,8 @@ class SymmetricContext:
                                 self.heap.rank, self.comm_ctas)
         backend.count_launch()
 
-    def ag_gemm(self, x2: torch.Tensor, g, n_out: int, n_copy: int = 16) -> torch.Tensor:
-        """``x2 @ Wᵀ`` for the first weight ``W (n_out × K)`` of group ``g`` with the all-gather of the whole
+    def ag_gemm(self, x2: torch.Tensor, g, n_out: int, n_copy: int = 16, bias=None) -> torch.Tensor:
+        """``x2 @ Wᵀ`` (+ bias) for the first weight ``W (n_out × K)`` of group ``g`` with the all-gather of the whole
         group fused into the same kernel launch."""
         m = self.meta[id(g)]
         if "ag_flags" not in m:
@@ -153,7 +153,7 @@ class SymmetricContext:
             m["ag_epoch"] = 0
         m["ag_epoch"] += 1
         out = self.ext.ag_gemm(x2, self.heap.bases, m["lp_off"], g.full, g.shard_numel * g.full.element_size(), 0,
-                               n_out, m["ag_flags"], m["ag_epoch"], self.heap.rank, n_copy)
+                               n_out, m["ag_flags"], m["ag_epoch"], self.heap.rank, n_copy, bias)
         backend.count_launch()
         return out
 

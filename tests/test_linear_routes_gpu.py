@@ -60,3 +60,28 @@ def test_odd_token_counts_without_gradients_run_the_library(T):
     with torch.no_grad():
         gemm.linear(x[:T // 8 * 8], w)
         assert backend.launches() == n0 + 2
+
+
+@pytest.mark.parametrize("one_cta", [False, True])
+@pytest.mark.parametrize("T,N,off", [(1, 512, 0), (8, 512, 0), (64, 520, 0), (67, 512, 4), (1000, 512, 8), (1001, 264, 0), (1024, 512, 0)])
+def test_a_bias_is_rounded_once_on_the_own_kernel(T, N, off, one_cta):
+    """`off`: elements between a 32-byte boundary and the bias (no 16-byte boundary: copied; no 32-byte one: the narrow epilogue)."""
+    torch.manual_seed(3)
+    x, w = (torch.randn(T, 256, device="cuda") * 0.5).bfloat16(), (torch.randn(N, 256, device="cuda") * 0.5).bfloat16()
+    b = (torch.randn(N + 16, device="cuda") * 2.0 ** -8).bfloat16()[off:off + N].requires_grad_()
+    ext = backend.require_extension()
+    was = ext.set_gemm_pair(not one_cta)
+    try:
+        n0 = backend.launches()
+        y = gemm.linear(x, w, b)
+        assert backend.launches() == n0 + 1
+    finally:
+        ext.set_gemm_pair(was)
+    ref = x.double() @ w.double().t() + b.double()
+    # half an ulp (at most 2^-8 of the value), and fp32 sums of 256 products of magnitude below 8
+    assert bool(((y.double() - ref).abs() <= ref.abs() * 2.0 ** -8 + 256 * 8 * 2.0 ** -24).all())
+    # two roundings leave errors of up to a whole ulp: with one, no element is further off than the library's by more than the sums' error
+    lib = F.linear(x, w, b)
+    assert bool(((y.double() - ref).abs() <= (lib.double() - ref).abs() + 2 * 256 * 8 * 2.0 ** -24).all())
+    db, = torch.autograd.grad(y, b, torch.ones_like(y))
+    assert torch.equal(db, torch.full_like(db, T))
