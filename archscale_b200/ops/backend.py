@@ -89,12 +89,17 @@ def use_cuda_kernel(op: str, *tensors: torch.Tensor) -> bool:
     return True
 
 
+def transformed() -> bool:
+    """True while a functorch transform, a forward-mode level or a ``torch.jit`` trace is active."""
+    return (torch._C._are_functorch_transforms_active() or forward_ad._current_level >= 0
+            or torch._C._get_tracing_state() is not None)
+
+
 def plain_call() -> bool:
-    """True when no autograd machinery can see a call: gradients are off, and no functorch transform, forward-mode level or
-    ``torch.jit`` trace is active.  An op then runs its kernel directly instead of through ``autograd.Function.apply`` (8 µs per
-    call, which is what a forward pass over a few dozen tokens spends most of its time on)."""
-    return (not torch.is_grad_enabled() and not torch._C._are_functorch_transforms_active() and forward_ad._current_level < 0
-            and torch._C._get_tracing_state() is None)
+    """True when no autograd machinery can see a call: gradients are off and nothing is :func:`transformed`.  An op then runs its
+    kernel directly instead of through ``autograd.Function.apply`` (8 µs per call, which is what a forward pass over a few
+    dozen tokens spends most of its time on)."""
+    return not torch.is_grad_enabled() and not transformed()
 
 
 class NoCtx:

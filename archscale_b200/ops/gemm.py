@@ -131,6 +131,7 @@ class _LinearFn(torch.autograd.Function):
     def backward(ctx, dy):
         x, weight = ctx.saved_tensors
         dy2 = dy.reshape(-1, dy.shape[-1])
+        main_grad = getattr(ctx.weight_ref, "main_grad", None)
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
         x2 = x.reshape(-1, x.shape[-1])
@@ -138,7 +139,6 @@ class _LinearFn(torch.autograd.Function):
         if ctx.needs_input_grad[0]:
             dx = matmul_nn(dy2, weight).view(x.shape)
         if ctx.needs_input_grad[1]:
-            main_grad = getattr(ctx.weight_ref, "main_grad", None)
             if main_grad is not None:
                 matmul_tn_acc_(main_grad, dy2, x2)      # wgrad accumulates straight into fp32
             else:
@@ -196,8 +196,8 @@ def _skinny_ok(x: torch.Tensor, ws) -> bool:
     """Whether the kernel for few rows (``csrc/gemm_skinny.cu``) takes ``x @ [w₀; w₁; …]ᵀ``: no gradients, at most 64 rows (one
     block of its tokens), dense bf16 rows that the TMA can read (16-byte base, widths that are multiples of 8)."""
     K = x.shape[-1]
-    if not (x.is_cuda and x.dtype == torch.bfloat16 and 0 < x.numel() <= SKINNY_ROWS * K and K % 8 == 0 and x.is_contiguous()
-            and x.data_ptr() % 16 == 0 and backend.plain_call() and backend.has("gemm_skinny")):
+    if not (x.is_cuda and x.dtype == torch.bfloat16 and 0 < x.numel() <= SKINNY_ROWS * K and K % 8 == 0 and backend.plain_call()
+            and x.is_contiguous() and x.data_ptr() % 16 == 0 and backend.has("gemm_skinny")):
         return False
     for w in ws:
         if not (w.is_cuda and w.dtype == torch.bfloat16 and w.dim() == 2 and w.shape[0] % 8 == 0 and w.shape[0] > 0 and w.stride(1) == 1
@@ -228,7 +228,7 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor) -> Optional[torch.Tenso
     if not (x.is_cuda and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and weight.dim() == 2
             and weight.shape[0] % 16 == 0 and x.shape[-1] % 8 == 0 and x.shape[-1] >= 64 and x.numel() > 0
             and weight.stride(-1) == 1 and weight.stride(0) % 8 == 0
-            and weight.data_ptr() % 16 == 0 and fused_swiglu_enabled() and backend.use_cuda_kernel("gemm", x, weight)):
+            and not backend.transformed() and weight.data_ptr() % 16 == 0 and fused_swiglu_enabled() and backend.use_cuda_kernel("gemm", x, weight)):
         return None
     g = getattr(weight, "_fsdp_group", None)
     if g is not None and getattr(g, "ag_pending", False):
@@ -246,13 +246,15 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     16383 26.0 / 28.5; 5632x1024 at 257 6.8 / 11.2, 1001 12.6 / 16.2, 4001 37.1 / 34.9, 8191 69.5 / 68.8; 2048x2048 at 1001 9.3 / 15.7, 16383
     91.7 / 96.0; host 11 / 15.
 
+    Functorch transforms, forward-mode differentiation and traces see the library's operator at every token count.
+
     A bias is added to the fp32 sums, before the one rounding to bf16, on either route: added to a rounded product, a bias below half a
     unit in the last place is lost."""
     if bias is None and _skinny_ok(x, (weight,)):
         return _skinny(x, [weight], False)
     if (x.is_cuda and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16
             and x.shape[-1] % 8 == 0 and weight.shape[0] % 8 == 0 and x.shape[-1] >= 64 and x.numel() > 0
-            and ((x.numel() // x.shape[-1]) % 8 == 0 or not backend.plain_call())
+            and ((x.numel() // x.shape[-1]) % 8 == 0 or not backend.plain_call()) and not backend.transformed()
             and backend.use_cuda_kernel("gemm", x, weight)):
         if not x.is_contiguous():
             x = x.contiguous()
@@ -324,18 +326,18 @@ class _MultiLinearFn(torch.autograd.Function):
                 y = matmul_nt(x2, w_cat)
         else:
             y = matmul_nt(x2, w_cat)
-        ctx.save_for_backward(x2, w_cat)
+        ctx.save_for_backward(x, w_cat)
         ctx.weights = weights
         return y.view(*x.shape[:-1], w_cat.shape[0])
 
     @staticmethod
     def backward(ctx, dy):
-        x2, w_cat = ctx.saved_tensors
-        dy2 = dy.reshape(-1, dy.shape[-1])
+        x, w_cat = ctx.saved_tensors
+        x2, dy2 = x.reshape(-1, x.shape[-1]), dy.reshape(-1, dy.shape[-1])
+        mgs = [getattr(w, "main_grad", None) for w in ctx.weights]
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
         dx = matmul_nn(dy2, w_cat).view(*dy.shape[:-1], x2.shape[1]) if ctx.needs_input_grad[0] else None
-        mgs = [getattr(w, "main_grad", None) for w in ctx.weights]
         if all(m is not None for m in mgs) and _adjacent(mgs):
             matmul_tn_acc_(_cat_view(mgs), dy2, x2)
             return (dx,) + (None,) * len(ctx.weights)
@@ -373,8 +375,8 @@ def linear_multi(x: torch.Tensor, layers, keep_fused: bool = False):
     if len(ws) <= 3 and _skinny_ok(x, ws):
         y = _skinny(x, ws, False)                       # the weights need not be neighbours here
         return y if keep_fused else list(y.split([w.shape[0] for w in ws], dim=-1))
-    fusable = (x.is_cuda and x.dtype == torch.bfloat16 and all(w.dtype == torch.bfloat16 for w in ws) and _adjacent(ws)
-               and x.numel() > 0 and x.shape[-1] % 8 == 0 and x.shape[-1] >= 64
+    fusable = (x.is_cuda and x.dtype == torch.bfloat16 and not backend.transformed() and all(w.dtype == torch.bfloat16 for w in ws)
+               and _adjacent(ws) and x.numel() > 0 and x.shape[-1] % 8 == 0 and x.shape[-1] >= 64
                and backend.use_cuda_kernel("gemm", x, ws[0]))
     if not fusable:
         return [l(x) for l in layers]

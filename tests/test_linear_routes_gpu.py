@@ -85,3 +85,16 @@ def test_a_bias_is_rounded_once_on_the_own_kernel(T, N, off, one_cta):
     assert bool(((y.double() - ref).abs() <= (lib.double() - ref).abs() + 2 * 256 * 8 * 2.0 ** -24).all())
     db, = torch.autograd.grad(y, b, torch.ones_like(y))
     assert torch.equal(db, torch.full_like(db, T))
+
+
+@pytest.mark.parametrize("T", [41, 67, 72])
+def test_transforms_and_traces_of_linear_layers(T):
+    torch.manual_seed(5)
+    x, w = (torch.randn(T, 128, device="cuda") / 8).bfloat16(), (torch.randn(64, 128, device="cuda") / 8).bfloat16()
+    want = F.linear(x, w)
+    for grad in (False, True):
+        with torch.set_grad_enabled(grad):
+            torch.testing.assert_close(torch.vmap(lambda r: gemm.linear(r, w))(x[:, None])[:, 0], want, rtol=2.0 ** -7, atol=2.0 ** -9)
+            y, t = torch.func.jvp(lambda x: gemm.linear(x, w), (x,), (x,))
+            torch.testing.assert_close(t, want, rtol=2.0 ** -7, atol=2.0 ** -9)
+    assert not torch.jit.trace(lambda x: gemm.linear(x, w), x, check_trace=False).graph.findNode("prim::PythonOp")
