@@ -132,6 +132,8 @@ class _LinearFn(torch.autograd.Function):
         x, weight = ctx.saved_tensors
         dy2 = dy.reshape(-1, dy.shape[-1])
         main_grad = getattr(ctx.weight_ref, "main_grad", None)
+        if torch.is_grad_enabled() and main_grad is None:                    # create_graph: the kernels have no backward of their own
+            return (dy @ weight, dy2.t() @ x.reshape(-1, x.shape[-1]), dy2.float().sum(0).to(dy.dtype) if ctx.has_bias else None)
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
         x2 = x.reshape(-1, x.shape[-1])
@@ -246,7 +248,8 @@ def linear(x: torch.Tensor, weight: torch.Tensor, bias: Optional[torch.Tensor] =
     16383 26.0 / 28.5; 5632x1024 at 257 6.8 / 11.2, 1001 12.6 / 16.2, 4001 37.1 / 34.9, 8191 69.5 / 68.8; 2048x2048 at 1001 9.3 / 15.7, 16383
     91.7 / 96.0; host 11 / 15.
 
-    Functorch transforms, forward-mode differentiation and traces see the library's operator at every token count.
+    Functorch transforms, forward-mode differentiation and traces see the library's operator at every token count, and a backward pass
+    that is itself recorded (``create_graph``) is made of differentiable operators.
 
     A bias is added to the fp32 sums, before the one rounding to bf16, on either route: added to a rounded product, a bias below half a
     unit in the last place is lost."""
@@ -335,6 +338,8 @@ class _MultiLinearFn(torch.autograd.Function):
         x, w_cat = ctx.saved_tensors
         x2, dy2 = x.reshape(-1, x.shape[-1]), dy.reshape(-1, dy.shape[-1])
         mgs = [getattr(w, "main_grad", None) for w in ctx.weights]
+        if torch.is_grad_enabled() and all(m is None for m in mgs):          # create_graph: see _LinearFn
+            return (dy @ torch.cat(ctx.weights), *(dy2.t() @ x2).split([w.shape[0] for w in ctx.weights]))
         if not dy2.is_contiguous():
             dy2 = dy2.contiguous()
         dx = matmul_nn(dy2, w_cat).view(*dy.shape[:-1], x2.shape[1]) if ctx.needs_input_grad[0] else None

@@ -98,3 +98,33 @@ def test_transforms_and_traces_of_linear_layers(T):
             y, t = torch.func.jvp(lambda x: gemm.linear(x, w), (x,), (x,))
             torch.testing.assert_close(t, want, rtol=2.0 ** -7, atol=2.0 ** -9)
     assert not torch.jit.trace(lambda x: gemm.linear(x, w), x, check_trace=False).graph.findNode("prim::PythonOp")
+
+
+def _penalty(fn, x, ws):
+    """Gradients of the squared norm of an input gradient, as a gradient penalty takes them."""
+    x = x.clone().requires_grad_()
+    ws = [w.clone().requires_grad_() for w in ws]
+    gx, = torch.autograd.grad(fn(x, ws).float().square().sum(), x, create_graph=True)
+    return torch.autograd.grad(gx.float().square().sum(), [x, *ws])
+
+
+@pytest.mark.parametrize("T", [41, 67, 72])
+def test_second_derivatives_of_linear_layers(T):
+    torch.manual_seed(4)
+    x = (torch.randn(T, 128, device="cuda") / 8).bfloat16()
+    flat = (torch.randn(96, 128, device="cuda") / 8).bfloat16()
+    b = torch.zeros(64, device="cuda", dtype=torch.bfloat16)
+
+    def multi(x, ws):
+        layers = [Linear(128, n, bias=False, device="cuda", dtype=torch.bfloat16) for n in (64, 32)]
+        for l, w in zip(layers, ws[0].split([64, 32])):
+            del l.weight
+            l.weight = w                                       # neighbours in one buffer, with a graph behind them
+        return torch.cat(gemm.linear_multi(x, layers), -1)
+
+    lib = lambda x, ws: F.linear(x, ws[0])
+    for fn, ref, ws in ((lambda x, ws: gemm.linear(x, ws[0], b), lib, [flat[:64]]), (lambda x, ws: gemm.linear(x, ws[0]), lib, [flat[:64]]),
+                        (multi, lib, [flat])):
+        for got, want in zip(_penalty(fn, x, ws), _penalty(ref, x.float(), [w.float() for w in ws])):
+            # four products in a row, a rounding to bf16 (2^-9) after each, none amplified
+            assert float((got.float() - want).norm() / want.norm()) < 2.0 ** -6
