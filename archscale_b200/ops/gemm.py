@@ -230,7 +230,8 @@ def linear_swiglu(x: torch.Tensor, weight: torch.Tensor) -> Optional[torch.Tenso
     if not (x.is_cuda and x.dtype == torch.bfloat16 and weight.dtype == torch.bfloat16 and weight.dim() == 2
             and weight.shape[0] % 16 == 0 and x.shape[-1] % 8 == 0 and x.shape[-1] >= 64 and x.numel() > 0
             and weight.stride(-1) == 1 and weight.stride(0) % 8 == 0
-            and not backend.transformed() and weight.data_ptr() % 16 == 0 and fused_swiglu_enabled() and backend.use_cuda_kernel("gemm", x, weight)):
+            and not backend.transformed() and weight.data_ptr() % 16 == 0 and (x.data_ptr() % 16 == 0 or not x.is_contiguous())
+            and fused_swiglu_enabled() and backend.use_cuda_kernel("gemm", x, weight)):
         return None
     g = getattr(weight, "_fsdp_group", None)
     if g is not None and getattr(g, "ag_pending", False):

@@ -6,7 +6,7 @@ import torch.nn.functional as F
 from archscale_b200.config import Config
 from archscale_b200.models.gpt import LLaMAMLP
 from archscale_b200.models.layers import Linear
-from archscale_b200.ops import backend, gemm
+from archscale_b200.ops import backend, gemm, swiglu_packed
 
 pytestmark = pytest.mark.gpu
 
@@ -128,3 +128,13 @@ def test_second_derivatives_of_linear_layers(T):
         for got, want in zip(_penalty(fn, x, ws), _penalty(ref, x.float(), [w.float() for w in ws])):
             # four products in a row, a rounding to bf16 (2^-9) after each, none amplified
             assert float((got.float() - want).norm() / want.norm()) < 2.0 ** -6
+
+
+@pytest.mark.parametrize("T", [67, 72])
+def test_an_input_off_the_16_byte_grid_is_taken(T):
+    x = torch.randn(T * 256 + 4, device="cuda").bfloat16()[4:].view(T, 256)
+    w = (torch.randn(128, 256, device="cuda") / 16).bfloat16()
+    y = gemm.linear_swiglu(x, w)
+    y = y if y is not None else swiglu_packed(gemm.linear(x, w))
+    g, u = (x.double() @ w.double().t()).chunk(2, -1)
+    assert float((y.double() - F.silu(g) * u).norm() / (F.silu(g) * u).norm()) < 2.0 ** -7     # three roundings to bf16
