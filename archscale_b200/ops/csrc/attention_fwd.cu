@@ -338,7 +338,15 @@ extern "C" int b200_attn_fwd(const void* q, const void* k, const void* v, void* 
   // Two tiles per CTA where that leaves no SM without work: measured (ms, one tile / two tiles per CTA, D 128, causal)
   // B8 T4096 H16 G4 0.641 / 0.481, B3 T2731 H16 G4 0.150 / 0.108, B1 T4096 H40 G40 0.232 / 0.223, B3 T1000 H12 G4 (288 tiles)
   // 0.034 / 0.031; at 256 tiles 0.069 / 0.072 and 0.031 / 0.029, at 128 tiles 0.029 / 0.041.
-  if (static_cast<long long>(B) * H * ((T + ATT_BM - 1) / ATT_BM) > 256)
+  // Pairs of two heads (an even number of query heads per KV head) win from there on, at every T (T 64 0.0126 / 0.0095).  Pairs of
+  // two row blocks of one head waste the second tile where the number of blocks is odd, and come in waves of one per SM
+  // instead of two: below a few waves they lose unless one wave takes them all.  µs, D 128: H16 G16 T300 B6 (288 tiles, 192 pairs)
+  // 17.0 / 22.2, T1100 B3 (432, 240) 39.2 / 44.7, T3001 B1 window 512 (384, 192) 35.3 / 41.4, T384 B11 (528, 352) 32.2 / 33.9, T768 B3 (288,
+  // 144) 24.2 / 21.4, T900 B7 (896) 66.9 / 60.4; three heads per KV head share its tiles and win earlier: H12 G4 T4096 B1 window 512 (384,
+  // 192) 37.5 / 40.9, T900 B5 (480) 42.0 / 36.1.  One block of at most 64 rows: D 64 T32 B64 36.6 / 39.3.
+  const int n_qt = (T + ATT_BM - 1) / ATT_BM, group = H / G;
+  const long long tiles = static_cast<long long>(B) * H * n_qt, pairs = static_cast<long long>(B) * H * ((n_qt + 1) / 2);
+  if (tiles > 256 && (group % 2 == 0 || (T > 64 && (pairs <= 148 || tiles > (group == 1 ? 700 : 384)))))
     return b200_attn_fwd_pair(q, k, v, out, lse, row_start, B, T, H, G, D, window_left, scale, status, stream);
   CUtensorMap tq, tk, tv;
   int rc = make_tmap_2d_bf16(&tq, q, static_cast<uint64_t>(H) * D, static_cast<uint64_t>(B) * T, static_cast<uint64_t>(H) * D, 64, 128);
