@@ -18,6 +18,8 @@ different TMA boxes and UMMA descriptor major-ness.
 """
 from __future__ import annotations
 
+import functools
+import os
 from typing import Optional
 
 import torch
@@ -186,7 +188,6 @@ class _LinearSwiGLUFn(torch.autograd.Function):
 
 def fused_swiglu_enabled() -> bool:
     """SwiGLU in the epilogue of the SM-pair GEMM (off with ``ARCHSCALE_B200_FUSED_SWIGLU=0`` or the one-CTA GEMM)."""
-    import os
     return (os.environ.get("ARCHSCALE_B200_FUSED_SWIGLU", "1") != "0" and os.environ.get("ARCHSCALE_B200_GEMM", "") != "1cta"
             and backend.has("gemm_swiglu"))
 
@@ -194,12 +195,18 @@ def fused_swiglu_enabled() -> bool:
 SKINNY_ROWS = 64
 
 
+@functools.lru_cache(maxsize=None)
+def _one_cta() -> bool:
+    """``ARCHSCALE_B200_GEMM=1cta``: every product on the one-CTA GEMM, those of few rows too."""
+    return os.environ.get("ARCHSCALE_B200_GEMM", "") == "1cta"
+
+
 def _skinny_ok(x: torch.Tensor, ws) -> bool:
     """Whether the kernel for few rows (``csrc/gemm_skinny.cu``) takes ``x @ [w₀; w₁; …]ᵀ``: no gradients, at most 64 rows (one
     block of its tokens), dense bf16 rows that the TMA can read (16-byte base, widths that are multiples of 8)."""
     K = x.shape[-1]
     if not (x.is_cuda and x.dtype == torch.bfloat16 and 0 < x.numel() <= SKINNY_ROWS * K and K % 8 == 0 and backend.plain_call()
-            and x.is_contiguous() and x.data_ptr() % 16 == 0 and backend.has("gemm_skinny")):
+            and x.is_contiguous() and x.data_ptr() % 16 == 0 and not _one_cta() and backend.has("gemm_skinny")):
         return False
     for w in ws:
         if not (w.is_cuda and w.dtype == torch.bfloat16 and w.dim() == 2 and w.shape[0] % 8 == 0 and w.shape[0] > 0 and w.stride(1) == 1

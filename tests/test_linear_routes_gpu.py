@@ -138,3 +138,14 @@ def test_an_input_off_the_16_byte_grid_is_taken(T):
     y = y if y is not None else swiglu_packed(gemm.linear(x, w))
     g, u = (x.double() @ w.double().t()).chunk(2, -1)
     assert float((y.double() - F.silu(g) * u).norm() / (F.silu(g) * u).norm()) < 2.0 ** -7     # three roundings to bf16
+
+
+def test_the_one_cta_switch_steers_products_of_few_rows(monkeypatch):
+    x, w = torch.randn(16, 64, device="cuda").bfloat16(), torch.randn(64, 64, device="cuda").bfloat16()
+    with torch.no_grad():
+        assert gemm._skinny_ok(x, (w,))
+        monkeypatch.setenv("ARCHSCALE_B200_GEMM", "1cta")
+        gemm._one_cta.cache_clear()
+        assert not gemm._skinny_ok(x, (w,))
+    monkeypatch.undo()
+    gemm._one_cta.cache_clear()
