@@ -117,10 +117,7 @@ class SonicMoE(nn.Module):
             mixed = self.share_expert
         with torch.no_grad():
             if indices.is_cuda:
-                # one row of counts per token, then their sum: bincount reads its largest value back to size the result, a wait
-                # for the device in every layer, and one shared row would queue all tokens on a few addresses
-                rows = torch.zeros(indices.shape[0], self.n_mods, dtype=torch.int32, device=indices.device)
-                counts = rows.scatter_add_(1, indices.long(), torch.ones_like(indices, dtype=torch.int32)).sum(0).to(torch.float32)
+                counts = ops.moe.expert_counts(indices, self.n_mods)
             else:
                 counts = torch.bincount(indices.reshape(-1).long(), minlength=self.n_mods).to(torch.float32)
             if self.collect_stats:
