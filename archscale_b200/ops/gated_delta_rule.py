@@ -218,7 +218,8 @@ class _BmmNTf32(torch.autograd.Function):
 
 class _MaskFn(torch.autograd.Function):
     """Gram blocks ``Gk = k̂·k̂ᵀ``, ``Gq = q̂·k̂ᵀ`` (fp32) → the strictly lower ``A = Gk ∘ decay ∘ β`` (fp32) and the lower ``Gq ∘ decay``
-    (bf16), ``decay[i, j] = exp(gc_i − gc_j)``; one pass each way (``csrc/gdn_pieces.cu``)."""
+    (bf16), ``decay[i, j] = exp(gc_i − gc_j)``; one pass each way (``csrc/gdn_pieces.cu``).  The Gram gradients leave in bf16, as the
+    products behind them take them; in between autograd casts them to the fp32 of its inputs and ``_BmmNTf32`` back."""
 
     @staticmethod
     def forward(ctx, Gk, Gq, gc, beta):
@@ -230,9 +231,7 @@ class _MaskFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dA, dqk):
         Gk, Gq, gc, beta = ctx.saved_tensors
-        dA = torch.zeros_like(Gk) if dA is None else dA.contiguous()
-        dqk = torch.zeros(Gk.shape, dtype=torch.bfloat16, device=Gk.device) if dqk is None else dqk.contiguous()
-        dGk, dGq, dgc, dbeta = backend.require_extension().gdn_mask_bwd(dA, dqk, Gk, Gq, gc, beta)
+        dGk, dGq, dgc, dbeta = backend.require_extension().gdn_mask_bwd(dA.contiguous(), dqk.contiguous(), Gk, Gq, gc, beta)
         backend.count_launch()
         return dGk, dGq, dgc, dbeta
 
@@ -250,8 +249,7 @@ class _ColsFn(torch.autograd.Function):
     @staticmethod
     def backward(ctx, dTu, dTw):
         Tm, gc, beta = ctx.saved_tensors
-        z = lambda t: torch.zeros(Tm.shape, dtype=torch.bfloat16, device=Tm.device) if t is None else t.contiguous()
-        dT, dgc, dbeta = backend.require_extension().gdn_cols_bwd(z(dTu), z(dTw), Tm, gc, beta)
+        dT, dgc, dbeta = backend.require_extension().gdn_cols_bwd(dTu.contiguous(), dTw.contiguous(), Tm, gc, beta)
         backend.count_launch()
         return dT, dgc, dbeta
 
