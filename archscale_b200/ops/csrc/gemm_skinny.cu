@@ -11,9 +11,9 @@
 // takes up to three weight matrices that share X (the query / key / value projections, written as column blocks of one
 // output) or a SwiGLU pair (gate rows first).
 // At 41 tokens, µs in a graph (weights not in the L2), with one rank's load after the other and one CTA per SM / now / library:
-// 1024x1024 6.9 / 5.6 / 4.2, 5632x1024 9.2 / 7.7 / 5.4, 1024x2816 8.2 / 7.0 / 6.4, 2048x2048 14.2 / 7.5 / 5.8, 32000x1024 24.4 / 16.9 /
+// 1024x1024 6.9 / 5.6 / 4.2, 5632x1024 9.2 / 8.1 / 5.4, 1024x2816 8.2 / 7.0 / 6.4, 2048x2048 14.2 / 7.5 / 5.8, 32000x1024 24.4 / 16.9 /
 // 16.2; query, key and value of 1024, 256, 256 x 1024 7.0 / 5.8 / 12.1 (three launches); SwiGLU of 2 x 2816 x 1024 9.3 / 7.9 / 7.4 (with the
-// activation's launch), 2 x 5632 x 2048 17.2 / 13.9 / 14.3.  A layer of a 41-token pass takes 26 µs in these four products, the
+// activation's launch), 2 x 5632 x 2048 17.2 / 15.2 / 14.3.  A layer of a 41-token pass takes 26 µs in these four products, the
 // library's seven launches 30.
 //
 // 192 threads: warp 0 TMA, warp 1 MMA, warps 2..5 tensor memory → shared memory (thread = weight row); all of them add.
@@ -80,8 +80,8 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
   const int wi = (p.n[2] > 0 && tile >= p.tile0[2]) ? 2 : (p.n[1] > 0 && tile >= p.tile0[1]) ? 1 : 0;
   const int rows = p.swiglu ? SKY_BN / 2 : SKY_BN;      // output columns of this tile
   const int n0 = (tile - (wi == 2 ? p.tile0[2] : wi == 1 ? p.tile0[1] : p.tile0[0])) * rows;
-  const int num_kb = (p.K + SKY_BK - 1) / SKY_BK;       // ≥ S: every rank has a share
-  const int kb0 = rank * num_kb / S, kb1 = (rank + 1) * num_kb / S;
+  const int num_kb = (p.K + SKY_BK - 1) / SKY_BK, per = (num_kb + S - 1) / S;
+  const int kb0 = min(rank * per, num_kb), kb1 = min(kb0 + per, num_kb);      // the last ranks may have no share
   const CUtensorMap* tw = wi == 0 ? &tmap_w0 : wi == 1 ? &tmap_w1 : &tmap_w2;
 
   auto load = [&](int kb, int st) {
@@ -127,19 +127,24 @@ gemm_skinny_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_cons
         umma_bf16_warp(tmem_base, make_smem_desc(sa + k * 32, 16, 1024), make_smem_desc(sa + SKY_A + k * 32, 16, 1024), idesc, (i | k) != 0);
       umma_commit_warp(&empty_bar[st]);
     }
-    if (ok) umma_commit_warp(done_bar);
+    if (ok && kb1 > kb0) umma_commit_warp(done_bar);
   } else {
     const int q = warp & 3;
     const int row = q * 32 + lane;
     // every product has been read from the stages when this barrier flips (all loads have landed before that)
-    const bool ok = mbar_wait_warp(done_bar, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL);
+    const bool share = kb1 > kb0 && mbar_wait_warp(done_bar, 0, abort_flag, p.status, STATUS_TIMEOUT_TMEM_FULL);
     tc_fence_after();
 #pragma unroll
     for (int c = 0; c < SKY_BT / 32; ++c) {
-      if (ok && c * 32 < p.M) {
+      if (c * 32 < p.M) {
         uint32_t r[32];
-        tmem_ld_32x32(tmem_base + c * 32 + (static_cast<uint32_t>(q * 32) << 16), r);
-        tmem_ld_wait();
+        if (share) {
+          tmem_ld_32x32(tmem_base + c * 32 + (static_cast<uint32_t>(q * 32) << 16), r);
+          tmem_ld_wait();
+        } else {
+#pragma unroll
+          for (int e = 0; e < 32; ++e) r[e] = 0u;
+        }
 #pragma unroll
         for (int e = 0; e < 32; ++e) part[(c * 32 + e) * SKY_BN + row] = __uint_as_float(r[e]);
       }
@@ -231,10 +236,10 @@ extern "C" int b200_gemm_skinny(const void* X, const void* const* W, const int* 
     col += n;
   }
   const int num_kb = (K + SKY_BK - 1) / SKY_BK;
-  // up to 5/4 CTAs per SM: at 41 tokens 176 CTAs beat 88 (5632x1024 7.7 against 8.1 µs, SwiGLU 2 x 5632 x 2048 13.9 against 15.2), 192
-  // in clusters of eight lose to 96 in clusters of four (3072x2048 8.3 against 8.1)
+  // (More CTAs than SMs, two of them on some: 5632x1024 7.7 against 8.1 µs, SwiGLU 2 x 5632 x 2048 13.9 against 15.2, but 3072x2048 8.3 against
+  // 8.1, and another order of the sums.)
   int S = 1;
-  while (S < 8 && tiles * S * 2 * 4 <= num_sms * 5 && S * 2 <= num_kb) S *= 2;
+  while (S < 8 && tiles * S * 2 <= num_sms && S * 2 <= num_kb) S *= 2;
   switch (S) {
     case 8: return launch_skinny<8>(tx, tw, p, tiles, stream);
     case 4: return launch_skinny<4>(tx, tw, p, tiles, stream);
