@@ -197,13 +197,17 @@ __device__ __forceinline__ void bwd_heads(const __nv_bfloat16* gsrc, const __nv_
     float rsv[ROPE_U];
 #pragma unroll
     for (int u = 0; u < ROPE_U; ++u) {
-      const int h = min(h0 + 2 * u + sub, per - 1);            // past the last head: loaded again, counted and stored nowhere
-      ld_raw(gsrc + h * D, rgl[u]);
-      ld_raw(gsrc + h * D + D / 2, rgh[u]);
-      if (has_w) {
-        ld_raw(xsrc + h * hstride, rxl[u]);
-        ld_raw(xsrc + h * hstride + D / 2, rxh[u]);
-        rsv[u] = rstd[h];
+      const int h = h0 + 2 * u + sub;
+      rgl[u] = rgh[u] = rxl[u] = rxh[u] = Raw<EPL>{};            // past the last head: zeros, which add nothing to the gain gradient
+      rsv[u] = 0.f;
+      if (h < per) {
+        ld_raw(gsrc + h * D, rgl[u]);
+        ld_raw(gsrc + h * D + D / 2, rgh[u]);
+        if (has_w) {
+          ld_raw(xsrc + h * hstride, rxl[u]);
+          ld_raw(xsrc + h * hstride + D / 2, rxh[u]);
+          rsv[u] = rstd[h];
+        }
       }
     }
 #pragma unroll
@@ -224,11 +228,11 @@ __device__ __forceinline__ void bwd_heads(const __nv_bfloat16* gsrc, const __nv_
         float xlo[EPL], xhi[EPL], dot = 0.f;
         expand<EPL>(rxl[u], xlo);
         expand<EPL>(rxh[u], xhi);
-        const float rs = rsv[u], rs_dw = h < per ? rs : 0.f;
+        const float rs = rsv[u];
 #pragma unroll
         for (int e = 0; e < EPL; ++e) {
-          dw[e] += glo[e] * xlo[e] * rs_dw;
-          dw[EPL + e] += ghi[e] * xhi[e] * rs_dw;
+          dw[e] += glo[e] * xlo[e] * rs;
+          dw[EPL + e] += ghi[e] * xhi[e] * rs;
           glo[e] *= w[e];
           ghi[e] *= w[EPL + e];
           dot += glo[e] * xlo[e] + ghi[e] * xhi[e];

@@ -149,3 +149,25 @@ def test_the_one_cta_switch_steers_products_of_few_rows(monkeypatch):
         assert not gemm._skinny_ok(x, (w,))
     monkeypatch.undo()
     gemm._one_cta.cache_clear()
+
+
+@pytest.mark.parametrize("one_cta", [False, True])
+@pytest.mark.parametrize("T", [65, 257, 4099])
+def test_odd_token_counts_run_one_own_launch_per_product(T, one_cta):
+    torch.manual_seed(6)
+    x, w, dy = ((torch.randn(*s, device="cuda") * 0.5).bfloat16() for s in ((T, 136), (264, 136), (T, 264)))
+    ext, acc = backend.require_extension(), torch.full((264, 136), 0.25, device="cuda")
+    ref = dy.double().t() @ x.double()
+    was = ext.set_gemm_pair(not one_cta)
+    try:
+        for fn, want, tol in ((lambda: gemm.matmul_nt(x, w), x.double() @ w.double().t(), 2.0 ** -8),
+                              (lambda: gemm.matmul_nn(dy, w), dy.double() @ w.double(), 2.0 ** -8),
+                              (lambda: gemm.matmul_tn(dy, x), ref, 2.0 ** -8),
+                              (lambda: gemm.matmul_tn_acc_(acc, dy, x), ref + 0.25, 1e-5)):        # fp32 sums of bf16 products
+            n0 = backend.launches()
+            got = fn()
+            assert backend.launches() == n0 + 1
+            assert float((got.double() - want).norm() / want.norm()) < tol
+    finally:
+        ext.set_gemm_pair(was)
+    assert ext.device_status() == 0

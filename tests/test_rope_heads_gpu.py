@@ -46,3 +46,17 @@ def test_qkv_norm_rope_matches_reference(B, T, H, G, D, norm, rot, grouped):
     assert rel(grads[0], ref[0]) < 2.0 ** -8
     for a, b in zip(grads[1:], ref[1:]):
         assert rel(a, b) < 1e-4
+
+
+@pytest.mark.parametrize("H,D", [(3, 128), (5, 64)])
+def test_an_infinite_gradient_in_the_last_head_stays_infinite(H, D):
+    """The steps over heads go past the last one where four do not divide their number: that adds nothing, not 0 · inf."""
+    torch.manual_seed(1)
+    x = torch.randn(1, 6, (H + 2) * D, device="cuda").bfloat16().requires_grad_()
+    w = [(torch.rand(D, device="cuda") + 0.5).requires_grad_() for _ in range(2)]
+    ang = torch.rand(6, D // 2, device="cuda") + 0.2
+    q, k, v = qkv_norm_rope(x, H, 1, False, w[0], w[1], ang.cos().bfloat16(), ang.sin().bfloat16(), 1e-5)
+    g = torch.randn_like(q)
+    g[0, 4, H - 1, 5] = float("inf")
+    dw, = torch.autograd.grad(q, w[0], g)
+    assert not dw.isnan().any() and dw.isinf().nonzero().flatten().tolist() == [5, 5 + D // 2]
