@@ -237,7 +237,8 @@ def bench_gdn(res: list) -> None:
         g = (-torch.rand(B, T, H, device="cuda") * 0.3).requires_grad_()
         beta = (torch.rand(B, T, H, device="cuda") * 2).requires_grad_()
         row = {"kernel": "gated_delta_rule", "shape": [B, T, H, Dk, Dv]}
-        for name, core in (("kernel", G._chunk_core), ("torch_loop", G._chunk_core_ref)):
+        loop = lambda *a: G._chunk_core_ref(*(t.float() for t in a))         # (the loop keeps its operands' type; its state is fp32)
+        for name, core in (("kernel", G._chunk_core), ("torch_loop", loop)):
             if name == "torch_loop" and B > 1:
                 continue
             saved, G._chunk_core = G._chunk_core, core
