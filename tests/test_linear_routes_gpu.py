@@ -171,3 +171,19 @@ def test_odd_token_counts_run_one_own_launch_per_product(T, one_cta):
     finally:
         ext.set_gemm_pair(was)
     assert ext.device_status() == 0
+
+
+def test_the_gathering_gemm_adds_the_bias():
+    """Both ranks' shards on one device, as the launch pulls them; the copying CTAs and the product are one kernel."""
+    torch.manual_seed(7)
+    ext, (M, N, K) = backend.require_extension(), (264, 512, 256)
+    shards = [(0.05 * torch.randn(N * K // 2, device="cuda")).bfloat16() for _ in range(2)]
+    a, b = torch.randn(M, K, device="cuda").bfloat16(), torch.randn(N, device="cuda").bfloat16()
+    dst = torch.zeros(N * K, device="cuda", dtype=torch.bfloat16)
+    flags = torch.zeros((dst.numel() * 2 + 256 * 1024 - 1) // (256 * 1024), dtype=torch.int32, device="cuda")
+    args = (a, [t.data_ptr() for t in shards], 0, dst, N * K, 0, N, flags)
+    y = ext.ag_gemm(*args, 1, 0, 16, gemm.bias_row(b))
+    ref = a.double() @ torch.cat(shards).view(N, K).double().t()
+    assert float((y.double() - ref - b.double()).norm() / ref.norm()) < 2.0 ** -8          # one rounding to bf16
+    assert float((ext.ag_gemm(*args, 2, 0, 16).double() - ref).norm() / ref.norm()) < 2.0 ** -8
+    assert ext.device_status() == 0
