@@ -7,7 +7,7 @@
 // and their backward with the row and column sums that go to gc and beta.  As element-wise PyTorch ops these were about 14 launches
 // forward and 35 backward per layer over [blocks, 64, 64] fp32 tensors; here each is one pass that reads and writes every
 // block once (16 KB per fp32 block; memory-bound).  Whole op, forward / forward + backward, ms, before (with the recurrence kernel as it was
-// then) and now: B8 T4096 H6 Dk256 Dv512 1.90 / 6.48 -> 1.49 / 5.27, B3 T2731 1.02 / 2.59 -> 0.66 / 2.06.
+// then) and now: B8 T4096 H6 Dk256 Dv512 1.90 / 6.48 -> 1.42 / 5.01, B3 T2731 1.02 / 2.59 -> 0.66 / 2.06.
 // 256 threads per block: thread t does row t / 4, columns 16·(t % 4) .. + 15.  Sums run in a fixed order.  Built without
 // --use_fast_math, whose exponential loses bits of strongly decayed factors and flushes those below 2^-126.
 #include "sm100.cuh"
